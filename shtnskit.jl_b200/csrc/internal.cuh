@@ -43,6 +43,8 @@ cudaError_t noalloc_scratch_address(void** out);
 
 // Degrees of one FP64 analysis tile (64 of each parity).
 constexpr int kAnaTile = 128;
+// Recurrence chains start at multiples of kStartStep degrees from their order.
+constexpr int kStartStep = 8;
 // Largest checkpoint table the plan keeps (bytes); the spacing grows from 16 degrees
 // until the table fits.
 constexpr size_t kCkptBudget = size_t(2) << 30;
@@ -58,8 +60,8 @@ struct PlanDev {
   const long long* off;    // [nm+1] packed (im, l) offsets, l in [m, lrec]
   const double* alpha;     // packed: r_l = alpha_l x r_{l-1} - r_{l-2}
   const double* cfac;      // packed: P_l = c_l r_l
-  const int* l0;           // [nm*npair] first significant degree per (im, pair)
-  const double2* r01;      // [nm*npair] (r_{l0}, r_{l0+1})
+  const int* l0;           // [nm*npair] start degree of (im, pair): m + a multiple of kStartStep; zeros below
+  const double2* start;    // [nm*npair] state (r_{l0-1}, r_{l0-2}) before it
   // recurrence checkpoints every ckstep degrees: entry (ckbase[im] + k) * npair + pair holds
   // the state (r_{t-1}, r_{t-2}) before degree t = m + k * ckstep
   const double2* ckpt;

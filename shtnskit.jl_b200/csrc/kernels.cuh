@@ -51,6 +51,12 @@ int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, v
 int launch_leg_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                      const Factors& F, int zero_fill, cudaStream_t st);
 
+// The same for one or two fields, on the FP64 pipes without MMAs (simt.cu).
+int launch_simt_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end, int mlim,
+                      cudaStream_t st);
+int launch_simt_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
+                      const Factors& F, int zero_fill, cudaStream_t st);
+
 // Vector coefficient transforms around the scalar Legendre stage.
 int launch_sphtor_pre64(const shtb_plan* p, const double2* S, const double2* T, double2* U, int nf, int ltr,
                         const Factors& F, int div_ll, cudaStream_t st);

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kLegThreads, 1)
     if (pp < npair) {
       px = P.x[pp];
       pl0 = P.l0[(size_t)im * npair + pp];
-      const double2 v = P.r01[(size_t)im * npair + pp];
+      const double2 v = P.start[(size_t)im * npair + pp];
       pr0 = v.x;
       pr1 = v.y;
     }
@@ -181,9 +181,9 @@ __global__ void __launch_bounds__(kLegThreads, 1)
         rb = v.y;
       }
       for (int l = lk; l < lc; ++l) {   // only when the checkpoints are sparser than a chunk
-        double r = fma(sAl[l - m] * px, ra, -rb);
-        r = (l == pl0) ? pr0 : r;
-        r = (l == pl0 + 1) ? pr1 : r;
+        ra = (l == pl0) ? pr0 : ra;
+        rb = (l == pl0) ? pr1 : rb;
+        const double r = fma(sAl[l - m] * px, ra, -rb);
         rb = ra;
         ra = r;
       }
@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(kLegThreads, 1)
         const int l = lc + s;
         const bool in = l <= lend;
         const double a = in ? sAl[l - m] : 0.0, f = in ? sFa[l - m] : 0.0;
-        double r = fma(a * px, ra, -rb);
-        r = (l == pl0) ? pr0 : r;
-        r = (l == pl0 + 1) ? pr1 : r;
+        ra = (l == pl0) ? pr0 : ra;
+        rb = (l == pl0) ? pr1 : rb;
+        const double r = fma(a * px, ra, -rb);
         rb = ra;
         ra = r;
         Pn[((s & 1) * (kSynDeg / 2) + (s >> 1)) * kSynPS + pq] = r * f;
@@ -290,6 +290,7 @@ static int launch_syn_ncol(const shtb_plan* p, const CoefSrc& src, const Factors
 
 int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end,
                      int mlim, cudaStream_t st) {
+  if (nf <= 2) return launch_simt_syn64(p, src, F, W, nf, row_end, mlim, st);
   if (nf > 32) return launch_syn_ncol<128>(p, src, F, W, nf, row_end, mlim, st);
   if (nf > 16) return launch_syn_ncol<64>(p, src, F, W, nf, row_end, mlim, st);
   if (nf > 8) return launch_syn_ncol<32>(p, src, F, W, nf, row_end, mlim, st);
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(kLegThreads, 1)
           ra = stv.x;
           rb = stv.y;
           l0 = P.l0[(size_t)im * npair + p];
-          const double2 v = P.r01[(size_t)im * npair + p];
+          const double2 v = P.start[(size_t)im * npair + p];
           r0 = v.x;
           r1 = v.y;
         }
@@ -416,9 +417,9 @@ __global__ void __launch_bounds__(kLegThreads, 1)
 #pragma unroll 4
         for (int s = 0; s < cs; ++s) {
           const int d = d0 + s, l = t0 + d;
-          double r = fma(salph[d] * x, ra, -rb);
-          r = (l == l0) ? r0 : r;
-          r = (l == l0 + 1) ? r1 : r;
+          ra = (l == l0) ? r0 : ra;
+          rb = (l == l0) ? r1 : rb;
+          const double r = fma(salph[d] * x, ra, -rb);
           rb = ra;
           ra = r;
           Ar[((d & 1) * 64 + (d >> 1)) * kAnaAS] = r;
@@ -527,6 +528,7 @@ static int launch_ana_ncol(const shtb_plan* p, const void* W, int nf, int row_en
 
 int launch_leg_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                      const Factors& F, int zero_fill, cudaStream_t st) {
+  if (nf <= 2) return launch_simt_ana64(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
   if (nf > 32) return launch_ana_ncol<128>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
   if (nf > 16) return launch_ana_ncol<64>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
   if (nf > 8) return launch_ana_ncol<32>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);

@@ -1291,20 +1291,18 @@ __global__ void mixed_table_kernel(PlanDev P, float* __restrict__ tabS, float* _
   const long long poff = P.off[im];
   const double x = P.x[pair];
   const int l0 = P.l0[(size_t)im * P.npair + pair];
-  const double2 r01 = P.r01[(size_t)im * P.npair + pair];
+  const double2 start = P.start[(size_t)im * P.npair + pair];
   const int pt = pair / kM, pr = pair % kM;
   const float asc = (float)(1 << f16_table_exp(P.lmax));   // exact scaling
   double ra = 0.0, rb = 0.0;
   unsigned long long nzm[2] = {0ull, 0ull};   // 64-row blocks of each parity with a nonzero value
   unsigned char* nzf = nzb + (long long)(2 * im) * nrb * npb + pair / 64;
   for (int l = m; l <= P.lrec; ++l) {
-    double r;
-    if (l == l0)
-      r = r01.x;
-    else if (l == l0 + 1)
-      r = r01.y;
-    else
-      r = fma(P.alpha[poff + (l - m)] * x, ra, -rb);
+    if (l == l0) {
+      ra = start.x;
+      rb = start.y;
+    }
+    const double r = fma(P.alpha[poff + (l - m)] * x, ra, -rb);
     rb = ra;
     ra = r;
     const int par = (l - m) & 1, j = (l - m) >> 1;

@@ -43,10 +43,14 @@ __device__ inline double plm_b(int l, int m) {
 // exponent (legendre.jl:252-271), the scaled recurrence until the exponent
 // returns to zero (legendre.jl:287-322), then the c-scaled recurrence
 //   r_l = alpha_l x r_{l-1} - r_{l-2}
-// through lrec, recording the state in front of every ckstep-th degree.
-// Values whose exponent is still negative are below 2^-480 and are dropped.
+// through lrec, recording the state in front of every ckstep-th degree. Values below
+// 2^-480 are dropped, but for those after the start degree: the chain starts at the last
+// multiple of kStartStep degrees from m at or below the first degree that reaches 2^-480,
+// from the state (r_{l0-1}, r_{l0-2}) (r_m = pmm from (0, -pmm)), so that the kernels look
+// for starts once every kStartStep degrees only. A degree grows |P| by at most
+// sqrt(2 l + 1), so the start states stay above 2^-600.
 __global__ void plan_setup_kernel(PlanDev P, const double* __restrict__ seedfac, int* __restrict__ l0_out,
-                                  double2* __restrict__ r01_out, double2* __restrict__ ckpt_out) {
+                                  double2* __restrict__ start_out, double2* __restrict__ ckpt_out) {
   const int pair = blockIdx.x * blockDim.x + threadIdx.x;
   const int im = blockIdx.y;
   if (pair >= P.npair) return;
@@ -66,17 +70,20 @@ __global__ void plan_setup_kernel(PlanDev P, const double* __restrict__ seedfac,
     }
   }
   const long long base = P.off[im];
-  int l0;
-  double r0 = 0.0, r1 = 0.0;
-  if (e == 0) {
-    l0 = m;
-    r0 = pmm;
-    r1 = sqrt((double)(2 * m + 3)) * x * pmm;
-  } else {
-    double p2 = pmm, p1 = sqrt((double)(2 * m + 3)) * x * pmm;
-    int l = m + 2;
-    bool ok = false;
+  int l0 = m;
+  double sa = 0.0, sb = -pmm;
+  if (e != 0) {
+    // record: (P_{la-1}, P_{la-2}) 2^qe before degree la
+    double qa = 0.0, qb = -pmm, p2 = pmm, p1 = sqrt((double)(2 * m + 3)) * x * pmm;
+    int qe = e, la = m, l = m + 2;
+    l0 = INT_MAX / 2;
     while (l <= LR) {
+      if ((l - m) % kStartStep == 0) {
+        qa = p1;
+        qb = p2;
+        qe = e;
+        la = l;
+      }
       const double p = plm_a(l, m) * x * p1 - plm_b(l, m) * p2;
       p2 = p1;
       p1 = p;
@@ -87,7 +94,7 @@ __global__ void plan_setup_kernel(PlanDev P, const double* __restrict__ seedfac,
         p1 *= DOWN;
         e += 960;
         if (e == 0) {
-          ok = true;
+          l0 = la;
           break;
         }
       } else if (mag < TINY && mag != 0.0) {
@@ -96,29 +103,22 @@ __global__ void plan_setup_kernel(PlanDev P, const double* __restrict__ seedfac,
         e -= 960;
       }
     }
-    if (ok) {
-      l0 = l - 2;
-      r0 = p2 / P.cfac[base + (l0 - m)];
-      r1 = p1 / P.cfac[base + (l0 + 1 - m)];
-    } else {
-      l0 = INT_MAX / 2;
-    }
+    sa = (la > m) ? scalbn(qa, qe) / P.cfac[base + (la - 1 - m)] : 0.0;
+    sb = (la > m) ? scalbn(qb, qe) / P.cfac[base + (la - 2 - m)] : scalbn(qb, qe);
   }
   l0_out[(size_t)im * P.npair + pair] = l0;
-  r01_out[(size_t)im * P.npair + pair] = make_double2(r0, r1);
+  start_out[(size_t)im * P.npair + pair] = make_double2(sa, sb);
   // checkpoints: state before degrees m + ckstep * k
   const int tb = P.ckbase[im];
   double ra = 0.0, rb = 0.0;
   for (int l = m; l <= LR; ++l) {
+    if (l == l0) {
+      ra = sa;
+      rb = sb;
+    }
     if (((l - m) % P.ckstep) == 0)
       ckpt_out[(size_t)(tb + (l - m) / P.ckstep) * P.npair + pair] = make_double2(ra, rb);
-    double r;
-    if (l == l0)
-      r = r0;
-    else if (l == l0 + 1)
-      r = r1;
-    else
-      r = fma(P.alpha[base + (l - m)] * x, ra, -rb);
+    const double r = fma(P.alpha[base + (l - m)] * x, ra, -rb);
     rb = ra;
     ra = r;
   }
@@ -326,6 +326,8 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
         const double al = std::sqrt(((double)(2 * l - 1) * (double)(2 * l + 1)) / ((double)(l - m) * (double)(l + m)));
         cfac[k] = bl * cfac[k - 2];
         alpha[k] = al * cfac[k - 1] / cfac[k];
+      } else if (l == m + 1) {
+        alpha[k] = std::sqrt((double)(2 * m + 3));
       }
       dco[k] = (l == 0 || l == m) ? 0.0 : std::sqrt(std::max(0.0, (double)(l * l - m * m) / (double)(4 * l * l - 1)));
     }
@@ -365,7 +367,7 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   auto take = [&](size_t bytes) { size_t r = o; o = align_up(o + bytes, 256); return r; };
   const size_t o_x = take(nlat * 8), o_w = take(nlat * 8), o_s = take(nlat * 8);
   const size_t o_off = take((nm + 1) * 8), o_alpha = take(npk * 8), o_c = take(npk * 8), o_d = take(npk * 8);
-  const size_t o_l0 = take((size_t)nm * npair * 4), o_r01 = take((size_t)nm * npair * 16);
+  const size_t o_l0 = take((size_t)nm * npair * 4), o_start = take((size_t)nm * npair * 16);
   const size_t o_ck = take((size_t)nseg * npair * 16), o_ckbase = take((size_t)nm * 4);
   const size_t o_atiles = take((size_t)natiles * 16);
   const size_t o_scale = coeff_scale ? take((size_t)(lmax + 1) * (mmax + 1) * 8) : 0;
@@ -416,7 +418,7 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   dv.alpha = (const double*)(D + o_alpha);
   dv.cfac = (const double*)(D + o_c);
   dv.l0 = (const int*)(D + o_l0);
-  dv.r01 = (const double2*)(D + o_r01);
+  dv.start = (const double2*)(D + o_start);
   dv.ckpt = (const double2*)(D + o_ck);
   dv.ckbase = (const int*)(D + o_ckbase);
   dv.ckstep = ckstep;
@@ -434,7 +436,7 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   if (ce == cudaSuccess) ce = cudaMemset(D + o_err, 0, 16);
 
   dim3 grid((npair + 127) / 128, nm);
-  plan_setup_kernel<<<grid, 128>>>(dv, (const double*)(D + o_seed), (int*)(D + o_l0), (double2*)(D + o_r01),
+  plan_setup_kernel<<<grid, 128>>>(dv, (const double*)(D + o_seed), (int*)(D + o_l0), (double2*)(D + o_start),
                                    (double2*)(D + o_ck));
   count_launch();
   ce = cudaGetLastError();

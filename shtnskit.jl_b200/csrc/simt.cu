@@ -1,143 +1,400 @@
-// simt.cu — mixed-precision Legendre synthesis for batches of one or two fields, with the
-// recurrence regenerated on the fly on the FP64 pipes.
+// simt.cu — Legendre stage for one or two fields, with the recurrence regenerated on the fly
+// on the FP64 pipes: synthesis and analysis of the FP64 path, synthesis of the mixed path.
 //
-// The tensor-core synthesis GEMM of mixed.cu reads the plan's P table image (4 bytes per
-// value) once per transform whatever the number of fields, so with one or two fields that
-// stream, not the arithmetic, sets its time: 4 bytes of table for 2 or 4 output columns. Here
-// each thread runs the c-scaled three-term recurrence of its own latitude pair in FP64,
-//   r_l = alpha_l x r_{l-1} - r_{l-2},   P_l^m = c_l r_l,
-// from the plan's start records (values below 2^-480 are zero until the record's first
-// degree l0), so P is never read from memory: 2 FP64 operations per value plus the
-// multiply-adds of the fields. Thread = latitude pair, CTA = 128 pairs of one order; the
-// order's coefficients (times c_l and the per-(l, m) factors, in FP64) are staged in shared
-// memory and read as broadcasts; E and O sums in FP64. Output: the Fourier buffer
-// W[field][im][E|O][pair] (FP32) that the FFT synthesis reads, as the GEMM writes it.
-//
-// The analysis keeps the tensor-core GEMM: its sums run over latitude pairs, across threads,
-// and a version of this kernel that reduced them across each CTA per block of degrees ran
-// several times slower than the GEMM on one-field batches (latency-bound chains at a few
-// warps per SM).
+// With one or two fields an MMA tile is mostly padding: the FP64 MMAs take 8 columns for 2 or
+// 4, and the tensor-core GEMM of mixed.cu streams 4 bytes of P table per value for 2 or 4
+// columns. Here a value of P costs 2 FP64 operations of the c-scaled three-term recurrence
+//   r_l = alpha_l x r_{l-1} - r_{l-2},   P_l^m = c_l r_l
+// and each field 2 more (real and imaginary part), and P is never read from memory. Chains
+// start from the plan's start records (zeros below the start degree, a multiple of kStartStep
+// degrees from m, so starts are looked for once every kStartStep degrees).
+//   synthesis  lane = latitude pair; the sum over degrees stays in the lane
+//   analysis   lane = latitude pair, warp = a segment of degrees with their sums in registers;
+//              the sum over pairs crosses the lanes once, at the end
+// E and O (even and odd l - m) sums in FP64 on both paths. Measured at lmax 1023, one field
+// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 164 us against the 8-column MMA
+// kernels; the FP64 pipes alone would take about 60 us each.
 #include <climits>
 #include <cstring>
+#include <type_traits>
 
 #include "kernels.cuh"
 
 namespace shtb {
 namespace sx {
 
-constexpr int kSynThreads = 128;
+constexpr int kThreads = 128;
 
 struct Args {
   PlanDev P;
-  const double* sc;       // normalization scale table (dense) or null
-  int sc_mode;            // 0 none, 1 multiply
-  const float2* cin;      // coefficients, field stride ld_k
-  float2* Wout;           // Fourier buffer
-  long long ld_k;
-  int cpacked;            // coefficients in the packed LM layout (ld_k = nlm)
-  int nf, lend;
+  Factors F;              // per-(l, m) multipliers of the coefficients
+  const void* cin;        // synthesis: coefficients (double2 or float2); analysis: Fourier buffer
+  void* out;              // synthesis: Fourier buffer; analysis: coefficients
+  long long ld_k, ld_m;   // coefficient strides (field, order) and layout, as CoefSrc / CoefSink
+  int packed;
+  int nf, lend;           // last degree of the sums
+  int mlim, lcap, zero_fill;   // analysis: largest order, last stored degree, clear l < m and l > lcap
 };
 
-__device__ __forceinline__ double coef_factor(const Args& a, int l, int m) {
-  double s = 1.0;
-  if (a.sc_mode) {
-    const double q = a.sc[l + (long long)(a.P.lmax + 1) * m];
-    s = q;
+template <typename C> struct Real;
+template <> struct Real<double2> { using type = double; };
+template <> struct Real<float2> { using type = float; };
+
+__device__ __forceinline__ double2 wide(double2 v) { return v; }
+__device__ __forceinline__ double2 wide(float2 v) { return make_double2(v.x, v.y); }
+__device__ __forceinline__ void narrow(double2& d, double2 v) { d = v; }
+__device__ __forceinline__ void narrow(float2& d, double2 v) { d = make_float2((float)v.x, (float)v.y); }
+
+__device__ __forceinline__ double factor_at(const Args& a, long long poff, int l, int m) {
+  const Factors& F = a.F;
+  double s = (m == 0) ? F.mf0 : F.mf1;
+  if (F.fac) s *= F.fac[poff + (l - m)];
+  if (F.sc_mode) {
+    const double q = F.sc[l + (long long)(a.P.lmax + 1) * m];
+    s = (F.sc_mode == 1) ? s * q : s / q;
   }
   return s;
 }
 
-// ------------------------------------------------------------------------- synthesis
-// Order index im, pairs 128 pb .. 128 pb + 127. smem: alpha of the order's degrees, then the
-// folded coefficients [degree][field] (syn_smem_bytes of the plan's lmax). All threads of the
-// CTA call it (it synchronises them).
-__host__ __device__ inline size_t syn_smem_bytes(int lmax, int nf) {
-  return (size_t)((lmax + 2) & ~1) * 8 + (size_t)(lmax + 1) * nf * 16 + 64;
+// Offset of degree 0 of order m in one field's coefficients.
+__device__ __forceinline__ long long coef_base(const Args& a, long long poff, int m) {
+  return a.packed == 1 ? poff - m : a.packed == 2 ? lm_base(a.P.lmax, a.P.mres, m) : (long long)m * a.ld_m;
 }
 
+// ------------------------------------------------------------------------- synthesis
+// One warp per CTA: a lane carries UP latitude pairs of one order. Per degree and field one
+// broadcast 16-byte shared-memory load feeds 2 UP multiply-adds: a broadcast load still fills
+// 32 lanes' registers (24 bytes a degree with alpha: 6 cycles of the SM's 128-byte path at one
+// field) while a pair's 4 FP64 operations take 2 cycles of its 64 units, so one pair per lane
+// is bound by those loads and four per lane by the FP64 units. The order's alpha and
+// coefficients (times the factors, in FP64) are staged kChunk<NF> degrees at a time in two
+// buffers; the next chunk's values are in registers while the current one is summed. Warps
+// share nothing: the warps nearer the poles start at higher degrees, and in CTAs of four
+// warps the barrier of the shared staging made them wait for the others (148 us, 44 % of
+// the issue slots, at lmax 1023 and one field).
 template <int NF>
-__device__ __forceinline__ void syn_body(const Args& a, int im, int pb, double* smem) {
+constexpr int kChunk = 64 / NF;   // two coefficients per lane
+
+template <typename C, int NF, int UP>
+__global__ void __launch_bounds__(32) syn_kernel(const __grid_constant__ Args a) {
+  constexpr int CH = kChunk<NF>;
+  __shared__ double sAl[2][CH];
+  __shared__ __align__(16) double2 sC[2][CH * NF];
   const PlanDev& P = a.P;
-  const int m = im * P.mres;
-  const int lend = a.lend, ndeg = lend - m + 1;
+  const int im = blockIdx.y, m = im * P.mres;
+  const int lane = threadIdx.x;
+  const int npair = P.npair, ndeg = a.lend - m + 1;
   const long long poff = P.off[im];
-  double* sAl = smem;
-  double2* sC = reinterpret_cast<double2*>(smem + ((ndeg + 1) & ~1));
-  for (int d = threadIdx.x; d < ndeg; d += kSynThreads) sAl[d] = P.alpha[poff + d];
-  for (int i = threadIdx.x; i < ndeg * NF; i += kSynThreads) {
-    const int d = i / NF, k = i - d * NF, l = m + d;
-    double2 v = make_double2(0.0, 0.0);
-    if (k < a.nf) {
-      const long long col = a.cpacked ? lm_base(P.lmax, P.mres, m) : (long long)m * (P.lmax + 1);
-      const float2 c = a.cin[(long long)k * a.ld_k + col + l];
-      const double f = P.cfac[poff + d] * coef_factor(a, l, m);
-      v = make_double2(c.x * f, c.y * f);
-    }
-    sC[i] = v;
-  }
-  const int npair = P.npair, pair = pb * kSynThreads + threadIdx.x;
-  int l0 = INT_MAX / 2;
-  double x = 0.0, s0 = 0.0, s1 = 0.0;
-  if (pair < npair) {
-    x = P.x[pair];
-    l0 = P.l0[(size_t)im * npair + pair];
-    const double2 v = P.r01[(size_t)im * npair + pair];
-    s0 = v.x;
-    s1 = v.y;
-  }
-  // each warp starts at its own pairs' first significant degree (below it every value is
-  // zero) and a warp with no pair of the plan skips the degree loop
-  int mn = l0;
-  for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-  __syncthreads();   // the staged alpha and coefficients
-  const int lbeg = max(mn, m);
-  const bool warp_live = pb * kSynThreads + (threadIdx.x & ~31) < npair;
-  double2 accE[NF], accO[NF];
+  const C* cin = (const C*)a.cin + coef_base(a, poff, m) + m;
+  const int pair0 = blockIdx.x * (32 * UP) + lane;
+  __shared__ double2 sS[UP][32];   // start states
+  double x[UP], ra[UP], rb[UP];
+  int l0[UP];
+  int mn = INT_MAX / 2;   // first start of the warp's pairs, relative to m (a multiple of kStartStep)
 #pragma unroll
-  for (int k = 0; k < NF; ++k) accE[k] = accO[k] = make_double2(0.0, 0.0);
-  double ra = 0.0, rb = 0.0;
-  // one degree into acc (E for even l - m, O for odd): the parity is static in the unrolled
-  // loop below, so the accumulators stay in registers
-  auto step = [&](int l, double2 (&acc)[NF]) {
-    const int d = l - m;
-    double r = fma(sAl[d] * x, ra, -rb);
-    r = (l == l0) ? s0 : r;
-    r = (l == l0 + 1) ? s1 : r;
-    rb = ra;
-    ra = r;
+  for (int u = 0; u < UP; ++u) {
+    const int pair = pair0 + 32 * u;
+    const bool ok = pair < npair;
+    x[u] = ok ? P.x[pair] : 0.0;
+    l0[u] = ok ? P.l0[(size_t)im * npair + pair] - m : INT_MAX / 2;
+    sS[u][lane] = ok ? P.start[(size_t)im * npair + pair] : make_double2(0.0, 0.0);
+    ra[u] = rb[u] = 0.0;
+    mn = min(mn, l0[u]);
+  }
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  double2 accE[UP][NF], accO[UP][NF];
 #pragma unroll
-    for (int k = 0; k < NF; ++k) {
-      const double2 c = sC[d * NF + k];
-      acc[k].x = fma(r, c.x, acc[k].x);
-      acc[k].y = fma(r, c.y, acc[k].y);
+  for (int u = 0; u < UP; ++u)
+#pragma unroll
+    for (int k = 0; k < NF; ++k) accE[u][k] = accO[u][k] = make_double2(0.0, 0.0);
+
+  // chunk stager: lane stages degrees sd0, sd0 + 32 / NF of field sk
+  const int sk = lane / (32 / NF), sd0 = lane % (32 / NF);
+  double al[2], cf[2];
+  C cv[2];
+  auto fetch = [&](int d0) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int d = d0 + sd0 + q * (32 / NF);
+      al[q] = cf[q] = 0.0;
+      cv[q].x = cv[q].y = 0;
+      if (d < ndeg) {
+        if (sk == 0) al[q] = P.alpha[poff + d];
+        cv[q] = cin[(long long)sk * a.ld_k + d];
+        cf[q] = factor_at(a, poff, m + d, m);
+      }
     }
   };
-  if (warp_live) {
-    int l = lbeg;
-    if (((l - m) & 1) && l <= lend) step(l++, accO);
-    for (; l + 1 <= lend; l += 2) {
-      step(l, accE);
-      step(l + 1, accO);
+  auto put = [&](int b) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int sd = sd0 + q * (32 / NF);
+      if (sk == 0) sAl[b][sd] = al[q];
+      const double2 c = wide(cv[q]);
+      sC[b][sd * NF + sk] = make_double2(c.x * cf[q], c.y * cf[q]);
     }
-    if (l <= lend) step(l, accE);
+  };
+  int buf = 0;
+  if (mn < ndeg) {
+    fetch(mn);
+    put(0);
   }
-  if (pair < npair) {
+  __syncwarp();
+  for (int d0 = mn; d0 < ndeg; d0 += CH, buf ^= 1) {
+    const bool more = d0 + CH < ndeg;
+    if (more) fetch(d0 + CH);
+    const int nd = min(CH, ndeg - d0);
+    auto step = [&](int d, double2 (&acc)[UP][NF]) {
+      const double av = sAl[buf][d];
+      double2 c[NF];
+#pragma unroll
+      for (int k = 0; k < NF; ++k) c[k] = sC[buf][d * NF + k];
+#pragma unroll
+      for (int u = 0; u < UP; ++u) {
+        const double r = fma(av * x[u], ra[u], -rb[u]);
+        rb[u] = ra[u];
+        ra[u] = r;
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+          acc[u][k].x = fma(r, c[k].x, acc[u][k].x);
+          acc[u][k].y = fma(r, c[k].y, acc[u][k].y);
+        }
+      }
+    };
+    for (int g = 0; g < nd; g += kStartStep) {
+      bool st = false;
+#pragma unroll
+      for (int u = 0; u < UP; ++u) st |= l0[u] == d0 + g;
+      if (__any_sync(0xffffffffu, st)) {
+#pragma unroll
+        for (int u = 0; u < UP; ++u)
+          if (l0[u] == d0 + g) {
+            const double2 v = sS[u][lane];
+            ra[u] = v.x;
+            rb[u] = v.y;
+          }
+      }
+      // degrees past the order's last have zero alpha and coefficients
+#pragma unroll
+      for (int d = 0; d < kStartStep; d += 2) {
+        step(g + d, accE);
+        step(g + d + 1, accO);
+      }
+    }
+    if (more) {
+      put(buf ^ 1);
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UP; ++u) {
+    const int pair = pair0 + 32 * u;
+    if (pair >= npair) continue;
 #pragma unroll
     for (int k = 0; k < NF; ++k) {
-      if (k >= a.nf) break;
-      float2* w = a.Wout + (((size_t)k * P.nm + im) * 2) * npair + pair;
-      w[0] = make_float2((float)accE[k].x, (float)accE[k].y);
-      w[npair] = make_float2((float)accO[k].x, (float)accO[k].y);
+      C* w = (C*)a.out + (((size_t)k * P.nm + im) * 2) * npair + pair;
+      narrow(w[0], accE[u][k]);
+      narrow(w[npair], accO[u][k]);
     }
   }
-  __syncthreads();   // shared memory is reused by the caller's next item
 }
 
-// blockIdx.x = block of 128 pairs, blockIdx.y = order index.
+// -------------------------------------------------------------------------- analysis
+// a_l = sum over pairs of P_l(x_pair) W[pair]: a warp owns kSeg<NF> = 32 / NF consecutive degrees
+// of one order and holds their sums for every lane (kSeg x NF complex doubles = 128 registers);
+// lane = latitude pair, the warp walks the pairs 32 at a time. Per pair and segment the chain
+// starts from the plan's checkpoint and the pair's Fourier values stay in registers, so P
+// costs 2 FP64 operations and each field 2 more, with one broadcast load of alpha per degree.
+// The lanes' sums meet once, at the end, in a butterfly that halves the values each lane keeps
+// per step (62 adds for 64 sums) and leaves lane i with item i = (degree i / NF, field i % NF).
+// Pair blocks whose every pair starts above the segment are skipped while they lead.
+// Every lane copies its own operands of the next pairs into its slots of a shared-memory
+// ring (cp.async; only the lane itself reads them, so no barrier): the registers left beside
+// the sums allow two warps per scheduler, too few to cover the loads. A slot holds kPU<NF>
+// blocks of 32 pairs, summed together: one alpha load serves both, and their chains overlap.
 template <int NF>
-__global__ void __launch_bounds__(kSynThreads) syn_kernel(const __grid_constant__ Args a) {
-  extern __shared__ __align__(16) double smem[];
-  syn_body<NF>(a, blockIdx.y, blockIdx.x, smem);
+constexpr int kSeg = 32 / NF;
+template <int NF>
+constexpr int kPU = 2 / NF;
+template <int NF>
+constexpr int kRing = NF == 1 ? 3 : 4;
+
+template <typename C, int NF>
+struct Ring {   // one warp's slots
+  double2 ck[kRing<NF>][kPU<NF>][32];
+  C w[kRing<NF>][kPU<NF>][2 * NF][32];
+  double x[kRing<NF>][kPU<NF>][32];
+  int l0[kRing<NF>][kPU<NF>][32];
+};
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst), n = ok ? BYTES : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(BYTES), "r"(n) : "memory");
+}
+
+template <typename C, int NF>
+__device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, const double* sal, Ring<C, NF>& R) {
+  constexpr int SG = kSeg<NF>, PU = kPU<NF>, RG = kRing<NF>;
+  const PlanDev& P = a.P;
+  const int lane = threadIdx.x & 31, npair = P.npair, m = im * P.mres;
+  const long long poff = P.off[im];
+  const int cs = P.ckstep, ks = (lseg - m) / cs, roll = (lseg - m) - ks * cs;
+  const double2* ck = P.ckpt + (size_t)(P.ckbase[im] + ks) * npair;
+  const int* pl0 = P.l0 + (size_t)im * npair;
+  const C* W = (const C*)a.cin + (size_t)im * 2 * npair;
+  const size_t wld = (size_t)P.nm * 2 * npair;
+  double2 acc[SG][NF];
+#pragma unroll
+  for (int s = 0; s < SG; ++s)
+#pragma unroll
+    for (int k = 0; k < NF; ++k) acc[s][k] = make_double2(0.0, 0.0);
+  // pairs from the first block with a start below the segment's end
+  int p0 = 0;
+  for (; p0 < npair; p0 += 32) {
+    const int p = p0 + lane;
+    if (__any_sync(0xffffffffu, p < npair && pl0[p] < lseg + SG)) break;
+  }
+  int fp = p0 + lane, fq = 0;   // next pair and slot to copy
+  auto fetch = [&]() {
+#pragma unroll
+    for (int u = 0; u < PU; ++u) {
+      const int p = fp + 32 * u;
+      const bool ok = p < npair;
+      const int pc = ok ? p : 0;
+      cp_async<16>(&R.ck[fq][u][lane], ck + pc, ok);
+      cp_async<8>(&R.x[fq][u][lane], P.x + pc, ok);
+      cp_async<4>(&R.l0[fq][u][lane], pl0 + pc, ok);
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        cp_async<sizeof(C)>(&R.w[fq][u][2 * k][lane], W + k * wld + pc, ok);
+        cp_async<sizeof(C)>(&R.w[fq][u][2 * k + 1][lane], W + k * wld + npair + pc, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    fp += 32 * PU;
+    fq = fq + 1 == RG ? 0 : fq + 1;
+  };
+#pragma unroll
+  for (int i = 0; i < RG - 1; ++i) fetch();
+  int q = 0;
+  for (; p0 < npair; p0 += 32 * PU) {
+    fetch();
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(RG - 1) : "memory");
+    double x[PU], ra[PU], rb[PU];
+    int l0[PU];
+    double2 E[PU][NF], O[PU][NF];
+    bool st = false;
+#pragma unroll
+    for (int u = 0; u < PU; ++u) {
+      x[u] = R.x[q][u][lane];
+      const double2 v = R.ck[q][u][lane];
+      ra[u] = v.x;
+      rb[u] = v.y;
+      l0[u] = R.l0[q][u][lane];   // 0 for pairs past the end: no start to look for
+      st |= l0[u] > lseg && l0[u] < lseg + SG;
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        E[u][k] = wide(R.w[q][u][2 * k][lane]);
+        O[u][k] = wide(R.w[q][u][2 * k + 1][lane]);
+      }
+    }
+    q = q + 1 == RG ? 0 : q + 1;
+    auto step = [&](int s, double al) {
+#pragma unroll
+      for (int u = 0; u < PU; ++u) {
+        const double r = fma(al * x[u], ra[u], -rb[u]);
+        rb[u] = ra[u];
+        ra[u] = r;
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+          const double2 w = (s & 1) ? O[u][k] : E[u][k];
+          acc[s][k].x = fma(r, w.x, acc[s][k].x);
+          acc[s][k].y = fma(r, w.y, acc[s][k].y);
+        }
+      }
+    };
+    if (!roll && !__any_sync(0xffffffffu, st)) {
+#pragma unroll
+      for (int s = 0; s < SG; ++s) step(s, sal[s]);
+    } else {
+      // a pair of the warp starts inside the segment, or the checkpoint lies below it
+      double2 v[PU];
+#pragma unroll
+      for (int u = 0; u < PU; ++u) {
+        const int p = p0 + 32 * u + lane;
+        v[u] = p < npair ? P.start[(size_t)im * npair + p] : make_double2(0.0, 0.0);
+      }
+      auto begin = [&](int l) {
+#pragma unroll
+        for (int u = 0; u < PU; ++u)
+          if (l == l0[u]) {
+            ra[u] = v[u].x;
+            rb[u] = v[u].y;
+          }
+      };
+      for (int l = lseg - roll; l < lseg; ++l) {
+        begin(l);
+        const double al = P.alpha[poff + (l - m)];
+#pragma unroll
+        for (int u = 0; u < PU; ++u) {
+          const double r = fma(al * x[u], ra[u], -rb[u]);
+          rb[u] = ra[u];
+          ra[u] = r;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < SG; ++s) {
+        if (s % kStartStep == 0) begin(lseg + s);
+        step(s, sal[s]);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy in flight past the segment
+  // items i = s * NF + k; after the step with lane bit o, a lane keeps the half of its items
+  // whose index has that bit as its lane number has
+  double2 (&v)[SG * NF] = reinterpret_cast<double2 (&)[SG * NF]>(acc);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const double2 send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      v[i].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, o);
+      v[i].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, o);
+    }
+  }
+  const int l = lseg + lane / NF, k = lane % NF;
+  if (l <= a.lcap && k < a.nf) {
+    const double f = factor_at(a, poff, l, m);
+    C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
+    narrow(*dst, make_double2(v[0].x * f, v[0].y * f));
+  }
+}
+
+// CTA = four consecutive segments of one order, a warp each: blockIdx.y of NF parts of a
+// kAnaTile-degree tile.
+template <typename C, int NF>
+__global__ void __launch_bounds__(128) ana_kernel(const __grid_constant__ Args a) {
+  constexpr int ND = 4 * kSeg<NF>;
+  __shared__ double sal[ND];
+  __shared__ __align__(16) Ring<C, NF> ring[4];
+  const PlanDev& P = a.P;
+  const int4 tile = P.atiles[blockIdx.x];
+  const int im = tile.x, t0 = tile.y + ND * blockIdx.y, m = im * P.mres;
+  if (m > a.mlim || t0 > a.lend) return;
+  const long long poff = P.off[im];
+  for (int i = threadIdx.x; i < ND; i += blockDim.x) sal[i] = (t0 + i <= a.lend) ? P.alpha[poff + (t0 + i - m)] : 0.0;
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lseg = t0 + kSeg<NF> * w;
+  if (lseg <= a.lend) ana_segment<C, NF>(a, im, lseg, sal + kSeg<NF> * w, ring[w]);
+  if (a.zero_fill && t0 == m) {
+    const int nrow = m + max(P.lmax - a.lcap, 0);   // rows [0, m) and (lcap, lmax]
+    for (int idx = threadIdx.x; idx < nrow * a.nf; idx += blockDim.x) {
+      const int r = idx % nrow, k = idx / nrow, l = (r < m) ? r : a.lcap + 1 + (r - m);
+      narrow(((C*)a.out)[(long long)k * a.ld_k + (long long)m * a.ld_m + l], make_double2(0.0, 0.0));
+    }
+  }
 }
 
 // Persistent kernel over the items of many transforms (uneven batches), one item per warp:
@@ -146,8 +403,8 @@ __global__ void __launch_bounds__(kSynThreads) syn_kernel(const __grid_constant_
 // stages its order's recurrence coefficients and FP64 coefficients in its own shared-memory
 // slice, kGroupChunk degrees at a time, so warps never wait for one another (a CTA-wide item
 // ends with a barrier at which the warps nearer the poles, which start at higher degrees,
-// wait for the others). Per thread the arithmetic is that of syn_body, so the results are
-// the same bit for bit.
+// wait for the others). Per latitude pair the arithmetic is that of syn_kernel, so the results
+// are the same bit for bit.
 constexpr int kGroupChunk = 128;
 constexpr size_t kGroupWarpDoubles = kGroupChunk + kGroupChunk * 2 * 2;   // alpha, then [degree][NF <= 2] double2
 
@@ -165,15 +422,13 @@ __device__ __forceinline__ void syn_warp_item(const Args& a, int im, int pb, dou
   double x = 0.0, s0 = 0.0, s1 = 0.0;
   if (pair < npair) {
     x = P.x[pair];
-    l0 = P.l0[(size_t)im * npair + pair];
-    const double2 v = P.r01[(size_t)im * npair + pair];
+    l0 = P.l0[(size_t)im * npair + pair] - m;
+    const double2 v = P.start[(size_t)im * npair + pair];
     s0 = v.x;
     s1 = v.y;
   }
-  int mn = l0;
-  for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-  const int dbeg = max(mn, m) - m;   // first degree (relative to m) with a nonzero value
-  const long long col = a.cpacked ? lm_base(P.lmax, P.mres, m) : (long long)m * (P.lmax + 1);
+  const int dbeg = __reduce_min_sync(0xffffffffu, l0);   // first start, a multiple of kStartStep from m
+  const long long col = coef_base(a, poff, m);
   double2 accE[NF], accO[NF];
 #pragma unroll
   for (int k = 0; k < NF; ++k) accE[k] = accO[k] = make_double2(0.0, 0.0);
@@ -181,23 +436,23 @@ __device__ __forceinline__ void syn_warp_item(const Args& a, int im, int pb, dou
   for (int d0 = dbeg; d0 < ndeg; d0 += kGroupChunk) {
     const int nd = min(kGroupChunk, ndeg - d0);
     __syncwarp();   // the previous chunk's values are read
-    for (int d = lane; d < nd; d += 32) sAl[d] = P.alpha[poff + d0 + d];
-    for (int i = lane; i < nd * NF; i += 32) {
+    // up to the next multiple of kStartStep, zeros past the order's last degree
+    const int nz = (nd + kStartStep - 1) & ~(kStartStep - 1);
+    for (int d = lane; d < nz; d += 32) sAl[d] = d < nd ? P.alpha[poff + d0 + d] : 0.0;
+    for (int i = lane; i < nz * NF; i += 32) {
       const int d = i / NF, k = i - d * NF, l = m + d0 + d;
       double2 v = make_double2(0.0, 0.0);
-      if (k < a.nf) {
-        const float2 c = a.cin[(long long)k * a.ld_k + col + l];
-        const double f = P.cfac[poff + d0 + d] * coef_factor(a, l, m);
+      if (d < nd && k < a.nf) {
+        const float2 c = ((const float2*)a.cin)[(long long)k * a.ld_k + col + l];
+        double f = P.cfac[poff + d0 + d];
+        if (a.F.sc_mode) f *= a.F.sc[l + (long long)(P.lmax + 1) * m];
         v = make_double2(c.x * f, c.y * f);
       }
       sC[i] = v;
     }
     __syncwarp();
-    auto step = [&](int l, double2 (&acc)[NF]) {
-      const int d = l - m - d0;
-      double r = fma(sAl[d] * x, ra, -rb);
-      r = (l == l0) ? s0 : r;
-      r = (l == l0 + 1) ? s1 : r;
+    auto step = [&](int d, double2 (&acc)[NF]) {
+      const double r = fma(sAl[d] * x, ra, -rb);
       rb = ra;
       ra = r;
 #pragma unroll
@@ -207,27 +462,30 @@ __device__ __forceinline__ void syn_warp_item(const Args& a, int im, int pb, dou
         acc[k].y = fma(r, c.y, acc[k].y);
       }
     };
-    int l = m + d0;
-    const int le = m + d0 + nd - 1;
-    if (((l - m) & 1) && l <= le) step(l++, accO);
-    for (; l + 1 <= le; l += 2) {
-      step(l, accE);
-      step(l + 1, accO);
+    for (int g = 0; g < nd; g += kStartStep) {
+      if (l0 == d0 + g) {
+        ra = s0;
+        rb = s1;
+      }
+#pragma unroll
+      for (int d = 0; d < kStartStep; d += 2) {
+        step(g + d, accE);
+        step(g + d + 1, accO);
+      }
     }
-    if (l <= le) step(l, accE);
   }
   if (pair < npair) {
 #pragma unroll
     for (int k = 0; k < NF; ++k) {
       if (k >= a.nf) break;
-      float2* w = a.Wout + (((size_t)k * P.nm + im) * 2) * npair + pair;
+      float2* w = (float2*)a.out + (((size_t)k * P.nm + im) * 2) * npair + pair;
       w[0] = make_float2((float)accE[k].x, (float)accE[k].y);
       w[npair] = make_float2((float)accO[k].x, (float)accO[k].y);
     }
   }
 }
 
-__global__ void __launch_bounds__(kSynThreads, 8) syn_group_kernel(const Args* __restrict__ targs,
+__global__ void __launch_bounds__(kThreads, 8) syn_group_kernel(const Args* __restrict__ targs,
                                                                 const int4* __restrict__ items, int nitems,
                                                                 int* __restrict__ queue) {
   extern __shared__ __align__(16) double smem[];
@@ -250,40 +508,83 @@ __global__ void __launch_bounds__(kSynThreads, 8) syn_group_kernel(const Args* _
 }  // namespace sx
 
 // ---------------------------------------------------------------------------- host
-bool simt_applicable(const shtb_plan* p, int nf) { return nf >= 1 && nf <= 2; }
+bool simt_applicable(const shtb_plan*, int nf) { return nf >= 1 && nf <= 2; }
 
-static sx::Args simt_args(const shtb_plan* p, const void* alm, void* W, int nf, int ltr, int packed) {
-  sx::Args a;
+static sx::Args simt_args(const shtb_plan* p, const void* in, void* out, const Factors& F, int nf, int lend) {
+  sx::Args a{};
   a.P = p->dev;
-  a.sc = p->d_scale;
-  a.sc_mode = p->d_scale ? 1 : 0;
-  a.cin = (const float2*)alm;
-  a.Wout = (float2*)W;
-  a.cpacked = packed;
-  a.ld_k = packed ? lm_count(p->lmax, p->mmax, p->mres) : (long long)(p->lmax + 1) * (p->mmax + 1);
+  a.F = F;
+  a.cin = in;
+  a.out = out;
   a.nf = nf;
-  a.lend = ltr;
+  a.lend = lend;
   return a;
+}
+
+// Pairs per lane: two (94 us at lmax 1023, one field; four 96 us) where that still gives every
+// SM a dozen warps, else one.
+static int syn_pairs_per_thread(const shtb_plan* p, int nmu) {
+  const long long per32 = (long long)((p->npair + 31) / 32) * nmu;
+  return per32 / 2 >= 1776 ? 2 : 1;
+}
+
+template <typename C, int NF>
+static int launch_syn(const shtb_plan* p, const sx::Args& a, int nmu, const char* name, cudaStream_t st) {
+  const int up = syn_pairs_per_thread(p, nmu);
+  const dim3 grid((p->npair + 32 * up - 1) / (32 * up), nmu);
+  prof_begin(st);
+  if (up == 2)
+    sx::syn_kernel<C, NF, 2><<<grid, 32, 0, st>>>(a);
+  else
+    sx::syn_kernel<C, NF, 1><<<grid, 32, 0, st>>>(a);
+  SHTB_LAUNCHED(name);
+  return SHTB_OK;
+}
+
+static Factors mixed_factors(const shtb_plan* p) {
+  return Factors{p->dev.cfac, p->d_scale, p->d_scale ? 1 : 0, 1.0, 1.0};
 }
 
 // Coefficients (FP32, dense or packed LM) -> Fourier buffer W (FP32), orders 0..mlim.
 int launch_simt_syn(const shtb_plan* p, const void* alm, void* W, int nf, int ltr, int mlim, int packed,
                     cudaStream_t st) {
-  const sx::Args a = simt_args(p, alm, W, nf, ltr, packed);
+  sx::Args a = simt_args(p, alm, W, mixed_factors(p), nf, ltr);
+  a.packed = packed ? 2 : 0;
+  a.ld_k = packed ? lm_count(p->lmax, p->mmax, p->mres) : (long long)(p->lmax + 1) * (p->mmax + 1);
+  a.ld_m = p->lmax + 1;
   const int nmu = mlim / p->mres + 1;
-  const size_t smem = sx::syn_smem_bytes(p->lmax, nf);
-  dim3 grid((p->npair + sx::kSynThreads - 1) / sx::kSynThreads, nmu);
+  return nf == 1 ? launch_syn<float2, 1>(p, a, nmu, "simt legendre synthesis kernel", st)
+                 : launch_syn<float2, 2>(p, a, nmu, "simt legendre synthesis kernel", st);
+}
+
+// FP64 coefficients -> Fourier buffer for one or two fields.
+int launch_simt_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end, int mlim,
+                      cudaStream_t st) {
+  sx::Args a = simt_args(p, src.ptr, W, F, nf, std::min(row_end, p->lrec));
+  a.packed = src.packed;
+  a.ld_k = src.ld_k;
+  a.ld_m = src.ld_m;
+  const int nmu = mlim / p->mres + 1;
+  return nf == 1 ? launch_syn<double2, 1>(p, a, nmu, "legendre synthesis kernel", st)
+                 : launch_syn<double2, 2>(p, a, nmu, "legendre synthesis kernel", st);
+}
+
+// FP64 Fourier buffer -> coefficients for one or two fields.
+int launch_simt_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
+                      const Factors& F, int zero_fill, cudaStream_t st) {
+  sx::Args a = simt_args(p, W, dst.ptr, F, nf, std::min(row_end, p->lrec));
+  a.packed = dst.packed;
+  a.ld_k = dst.ld_k;
+  a.ld_m = dst.ld_m;
+  a.mlim = mlim;
+  a.lcap = dst.packed == 1 ? a.lend : std::min(a.lend, p->lmax);
+  a.zero_fill = zero_fill && !dst.packed;
   prof_begin(st);
-  if (nf == 1) {
-    SHTB_TRY_CUDA(cudaFuncSetAttribute(sx::syn_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                  "simt smem attr");
-    sx::syn_kernel<1><<<grid, sx::kSynThreads, smem, st>>>(a);
-  } else {
-    SHTB_TRY_CUDA(cudaFuncSetAttribute(sx::syn_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                  "simt smem attr");
-    sx::syn_kernel<2><<<grid, sx::kSynThreads, smem, st>>>(a);
-  }
-  SHTB_LAUNCHED("simt legendre synthesis kernel");
+  if (nf == 1)
+    sx::ana_kernel<double2, 1><<<p->dev.natiles, 128, 0, st>>>(a);
+  else
+    sx::ana_kernel<double2, 2><<<dim3(p->dev.natiles, 2), 128, 0, st>>>(a);
+  SHTB_LAUNCHED("legendre analysis kernel");
   return SHTB_OK;
 }
 
@@ -291,20 +592,22 @@ int launch_simt_syn(const shtb_plan* p, const void* alm, void* W, int nf, int lt
 size_t simt_args_bytes() { return sizeof(sx::Args); }
 
 void simt_fill_args(const shtb_plan* p, const void* alm, void* W, int nf, void* host_args) {
-  const sx::Args a = simt_args(p, alm, W, nf, p->lmax, 0);
+  sx::Args a = simt_args(p, alm, W, mixed_factors(p), nf, p->lmax);
+  a.ld_k = (long long)(p->lmax + 1) * (p->mmax + 1);
+  a.ld_m = p->lmax + 1;
   std::memcpy(host_args, &a, sizeof(a));
 }
 
 int simt_syn_pair_blocks(const shtb_plan* p) { return (p->npair + 31) / 32; }   // per-warp items of the group kernel
 
-size_t simt_group_syn_smem(const shtb_plan*) { return (sx::kSynThreads / 32) * sx::kGroupWarpDoubles * sizeof(double); }
+size_t simt_group_syn_smem(const shtb_plan*) { return (sx::kThreads / 32) * sx::kGroupWarpDoubles * sizeof(double); }
 
 int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, size_t smem, int* queue,
                       cudaStream_t st) {
   if (nitems <= 0) return SHTB_OK;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(sx::syn_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "simt group smem attr");
-  sx::syn_group_kernel<<<grid, sx::kSynThreads, smem, st>>>((const sx::Args*)targs, items, nitems, queue);
+  sx::syn_group_kernel<<<grid, sx::kThreads, smem, st>>>((const sx::Args*)targs, items, nitems, queue);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "simt group launch");
   return SHTB_OK;
