@@ -170,7 +170,7 @@ __device__ __forceinline__ void fft_syn_body(const FFTJob<T>& J, int p0, int k, 
   const int sh = fft_padsh(fd, sizeof(V)), N = fd.n, S = fft_row_stride(N, sh);
   V* Z = reinterpret_cast<V*>(smem_raw);
   V* scratch = Z + H * S;
-  T* gfac = reinterpret_cast<T*>(Z + ((GENERIC && fd.direct) ? 2 : 1) * H * S);
+  T* gfac = reinterpret_cast<T*>(Z + ((GENERIC && fd.big) ? 2 : 1) * H * S);
   const int npair = P.npair, nlat = P.nlat;
   const int hv = min(H, npair - p0);
   // Bins the order loop below does not write (|m| > mlim, or m off the mres lattice)
@@ -306,7 +306,7 @@ __device__ __forceinline__ void fft_ana_body(const FFTJob<T>& J, int p0, int k, 
   const int sh = fft_padsh(fd, sizeof(V)), N = fd.n, S = fft_row_stride(N, sh);
   V* Z = reinterpret_cast<V*>(smem_raw);
   V* scratch = Z + H * S;
-  T* wfac = reinterpret_cast<T*>(Z + ((GENERIC && fd.direct) ? 2 : 1) * H * S);
+  T* wfac = reinterpret_cast<T*>(Z + ((GENERIC && fd.big) ? 2 : 1) * H * S);
   const int npair = P.npair, nlat = P.nlat;
   const int hv = min(H, npair - p0);
   const T* in = (ncomp == 2 && (k & 1)) ? in1 : in0;
@@ -533,17 +533,17 @@ static FFTJob<T> fft_job(const shtb_plan* p, const int* perm, const typename V2<
 static int fft_pick_h(const FFTDesc& fd, size_t celem, int npair) {
   const size_t S = (size_t)fft_row_stride(fd.n, fft_padsh(fd, celem));
   int h = 16;
-  while (h > 1 && (size_t)h * S * celem * (fd.direct ? 2 : 1) + 16 * 8 > 200 * 1024) h >>= 1;
+  while (h > 1 && (size_t)h * S * celem * (fd.big ? 2 : 1) + 16 * 8 > 200 * 1024) h >>= 1;
   while (h > 1 && h / 2 >= npair) h >>= 1;
   return h;
 }
 
 static size_t fft_smem(const FFTDesc& fd, size_t celem, int h) {
-  return (size_t)h * fft_row_stride(fd.n, fft_padsh(fd, celem)) * celem * (fd.direct ? 2 : 1) + (size_t)h * 8 + 16;
+  return (size_t)h * fft_row_stride(fd.n, fft_padsh(fd, celem)) * celem * (fd.big ? 2 : 1) + (size_t)h * 8 + 16;
 }
 
 static bool fft_generic(const shtb_plan* p) {
-  bool g = p->fft.direct;
+  bool g = false;
   for (int i = 0; i < p->fft.nrad; ++i) {
     const int r = p->fft.rad[i];
     g = g || !(r == 2 || r == 3 || r == 4 || r == 5 || r == 8 || r == 16);
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(512) fft_ana_cplx_kernel(PlanDev P, FFTDesc fd
 static int fft_pick_h_cplx(const FFTDesc& fd, int npair) {
   const size_t S = (size_t)fft_row_stride(fd.n, fft_padsh(fd, sizeof(double2)));
   int h = 8;
-  while (h > 1 && (size_t)2 * h * S * sizeof(double2) * (fd.direct ? 2 : 1) > 200 * 1024) h >>= 1;
+  while (h > 1 && (size_t)2 * h * S * sizeof(double2) * (fd.big ? 2 : 1) > 200 * 1024) h >>= 1;
   while (h > 1 && h / 2 >= npair) h >>= 1;
   return h;
 }
@@ -718,7 +718,7 @@ template <int H>
 static int launch_cplx_h(const shtb_plan* p, int syn, const void* src, void* dst, int nf, int mlim, double scale,
                          cudaStream_t st) {
   const size_t smem = (size_t)2 * H * fft_row_stride(p->fft.n, fft_padsh(p->fft, sizeof(double2))) * sizeof(double2) *
-                      (p->fft.direct ? 2 : 1);
+                      (p->fft.big ? 2 : 1);
   if (smem > 227 * 1024) return set_error(SHTB_ERR_UNSUPPORTED, "nlon too large for the complex-row FFT");
   const bool gen = fft_generic(p);
   dim3 grid((p->npair + H - 1) / H, nf);

@@ -10,7 +10,8 @@
 // The transform is an in-place decimation-in-frequency mixed-radix FFT
 // (radices 16, 8, 4, 2, 3, 5 and generic odd radices up to 13): every pass updates
 // disjoint groups of r elements where they lie, so one shared buffer and one
-// barrier per pass suffice for any thread count. The result comes out in
+// barrier per pass suffice for any thread count. Prime factors above 13 are passes of
+// their own radix between two buffers (dif_pass_prime). The result comes out in
 // mixed-radix digit-reversed order; callers read bin k at position rev[k]
 // (a plan table). Indices are skewed by pad(n) = n + n/8 to spread the strided
 // accesses of the late passes over the shared-memory banks.
@@ -53,7 +54,7 @@ __host__ __device__ inline int fft_row_stride(int n, int sh) { return n + (n >> 
 __host__ __device__ inline int fft_padsh(const FFTDesc& fd, size_t celem) { return celem == 8 ? fd.padsh : 3; }
 // Radix of pass s when the grid I/O can take it over (power-of-two radices), else 0.
 __host__ __device__ inline int fft_fusable_radix(const FFTDesc& fd, int s) {
-  if (fd.direct || fd.nrad < 2) return 0;
+  if (fd.nrad < 2) return 0;
   const int r = fd.rad[s];
   return (r == 2 || r == 4 || r == 8 || r == 16) ? r : 0;
 }
@@ -232,38 +233,111 @@ __device__ __forceinline__ void dif_pass(V* X, int F, int N, int S, int Ns, int 
   __syncthreads();
 }
 
-// Full in-place FFT of F rows (natural-order input; output bin k at rev[k]), or its
-// passes s0 .. s1-1 only (s1 < 0: to the end) when the caller fuses the first or the
-// last pass with its global loads or stores. `scratch` (same size as X) is used only in
-// direct mode (a prime factor above 13).
+// One DIF pass of a prime radix r > 13, out of place: X -> Y (X is overwritten). With
+// h = (r - 1) / 2, s_j = x_j + x_{r-j} and d_j = x_j - x_{r-j} (formed in place first),
+//   X_k, X_{r-k} = A_k +- dir i B_k,  A_k = x_0 + sum_{j<=h} cos(2 pi j k / r) s_j,
+//                                     B_k = sum_{j<=h} sin(2 pi j k / r) d_j,
+// r real multiply-adds per complex output (2 r multiply-adds per output pair) where the plain
+// sum takes 4 r, and N r in all where a dense DFT of the row takes 4 N^2. A thread sums KU
+// values of k for GU groups, so that a pair of table values serves GU groups and a pair of
+// elements KU sums (one table load and one shared-memory load for every 8 multiply-adds).
+// FP64, nlon 402 = 2 3 67, 102 pairs x 3 fields: 279 -> 33 us against the dense DFT.
+template <typename T, typename V>
+__device__ __forceinline__ void dif_pass_prime(V* X, V* Y, int F, int N, int S, int Ns, int r, const V* __restrict__ tw,
+                                               const V* __restrict__ twp, unsigned mrow, unsigned mspan, int dir, int sh) {
+  constexpr int KU = 4, GU = 2;
+  const int span = Ns / r, per_row = N / r, total = F * per_row, h = (r - 1) >> 1, tws = N / r;
+  const int bd = blockDim.x;
+  auto locate = [&](int b, int& rowoff, int& base, int& j) {
+    const int f = mrow ? (int)__umulhi((unsigned)b, mrow) : b;
+    const int t = b - f * per_row;
+    const int blk = mspan ? (int)__umulhi((unsigned)t, mspan) : t;
+    j = t - blk * span;
+    base = blk * span * r + j;
+    rowoff = f * S;
+  };
+  for (int i = threadIdx.x; i < total * h; i += bd) {
+    const int q = i / total + 1;
+    int ro, ba, j;
+    locate(i - (q - 1) * total, ro, ba, j);
+    V* p = X + ro + fft_pad(ba + q * span, sh);
+    V* m = X + ro + fft_pad(ba + (r - q) * span, sh);
+    const V a = *p, b = *m;
+    *p = cadd(a, b);
+    *m = csub(a, b);
+  }
+  __syncthreads();
+  const int ngb = (total + GU - 1) / GU, nkb = h / KU + 1;
+  for (int i = threadIdx.x; i < ngb * nkb; i += bd) {
+    const int kb = i / ngb, gb = i - kb * ngb, k0 = kb * KU;
+    int ro[GU], ba[GU], jj[GU], t[KU];
+    V A[GU][KU], B[GU][KU];
+#pragma unroll
+    for (int g = 0; g < GU; ++g) {
+      locate(min(gb + g * ngb, total - 1), ro[g], ba[g], jj[g]);
+      const V x0 = X[ro[g] + fft_pad(ba[g], sh)];
+#pragma unroll
+      for (int u = 0; u < KU; ++u) {
+        A[g][u] = x0;
+        B[g][u].x = B[g][u].y = 0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < KU; ++u) t[u] = 0;
+    for (int j = 1; j <= h; ++j) {
+      V w[KU];
+#pragma unroll
+      for (int u = 0; u < KU; ++u) {
+        t[u] += min(k0 + u, h);
+        if (t[u] >= r) t[u] -= r;
+        w[u] = tw[t[u] * tws];   // (cos, -sin)
+      }
+#pragma unroll
+      for (int g = 0; g < GU; ++g) {
+        const V s = X[ro[g] + fft_pad(ba[g] + j * span, sh)], d = X[ro[g] + fft_pad(ba[g] + (r - j) * span, sh)];
+#pragma unroll
+        for (int u = 0; u < KU; ++u) {
+          A[g][u].x += w[u].x * s.x;
+          A[g][u].y += w[u].x * s.y;
+          B[g][u].x -= w[u].y * d.x;
+          B[g][u].y -= w[u].y * d.y;
+        }
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < GU; ++g) {
+      if (gb + g * ngb >= total) continue;
+#pragma unroll
+      for (int u = 0; u < KU; ++u) {
+        const int k = k0 + u;
+        if (k > h) continue;
+        const V ib = crot(B[g][u], dir);
+        V lo = cadd(A[g][u], ib), hi = csub(A[g][u], ib);
+        if (jj[g] != 0 && k != 0) {
+          V wl = twp[(k - 1) * span + jj[g]], wh = twp[(r - k - 1) * span + jj[g]];
+          if (dir > 0) {
+            wl.y = -wl.y;
+            wh.y = -wh.y;
+          }
+          lo = cmul(lo, wl);
+          hi = cmul(hi, wh);
+        }
+        Y[ro[g] + fft_pad(ba[g] + k * span, sh)] = lo;
+        if (k != 0) Y[ro[g] + fft_pad(ba[g] + (r - k) * span, sh)] = hi;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// FFT of F rows (natural-order input; output bin k at rev[k]), or its passes s0 .. s1-1
+// only (s1 < 0: to the end) when the caller fuses the first or the last pass with its
+// global loads or stores. In place but for prime radices above 13, which move the rows
+// between X and `scratch` (same size); X is left at the buffer that holds the result.
 template <typename T, typename V, bool GENERIC>
-__device__ void fft_rows(V* X, V* scratch, int F, int S, const FFTDesc& fd, const V* __restrict__ tw,
+__device__ void fft_rows(V*& X, V* scratch, int F, int S, const FFTDesc& fd, const V* __restrict__ tw,
                          const V* __restrict__ twp, int dir, int s0 = 0, int s1 = -1) {
   const int N = fd.n, sh = fft_padsh(fd, sizeof(V));
-  if (GENERIC && fd.direct) {
-    // O(N^2) DFT into scratch, written at natural positions (rev = identity in direct mode)
-    for (int idx = threadIdx.x; idx < F * N; idx += blockDim.x) {
-      const int f = idx / N, k = idx - f * N;
-      V acc;
-      acc.x = 0; acc.y = 0;
-      int t = 0;
-      for (int n = 0; n < N; ++n) {
-        V wv = tw[t];
-        if (dir > 0) wv.y = -wv.y;
-        acc = cadd(acc, cmul(X[(size_t)f * S + fft_pad(n, sh)], wv));
-        t += k;
-        if (t >= N) t -= N;
-      }
-      scratch[(size_t)f * S + fft_pad(k, sh)] = acc;
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < F * N; idx += blockDim.x) {
-      const int f = idx / N, k = idx - f * N;
-      X[(size_t)f * S + fft_pad(k, sh)] = scratch[(size_t)f * S + fft_pad(k, sh)];
-    }
-    __syncthreads();
-    return;
-  }
   int Ns = N;
   for (int s = 0; s < s0; ++s) Ns /= fd.rad[s];
   const int send = s1 < 0 ? fd.nrad : s1;
@@ -279,7 +353,16 @@ __device__ void fft_rows(V* X, V* scratch, int F, int S, const FFTDesc& fd, cons
       case 8: dif_pass<T, V, 8>(X, F, N, S, Ns, 8, tw, tp, mr, ms, dir, sh); break;
       case 16: dif_pass<T, V, 16>(X, F, N, S, Ns, 16, tw, tp, mr, ms, dir, sh); break;
       default:
-        if constexpr (GENERIC) dif_pass<T, V, 13>(X, F, N, S, Ns, r, tw, tp, mr, ms, dir, sh);
+        if constexpr (GENERIC) {
+          if (r <= 13) {
+            dif_pass<T, V, 13>(X, F, N, S, Ns, r, tw, tp, mr, ms, dir, sh);
+          } else {
+            dif_pass_prime<T, V>(X, scratch, F, N, S, Ns, r, tw, tp, mr, ms, dir, sh);
+            V* z = X;
+            X = scratch;
+            scratch = z;
+          }
+        }
         break;
     }
     Ns /= r;

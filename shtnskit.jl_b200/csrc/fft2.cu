@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(128 * HP, 4 / HP) group_kernel(const Job* __re
 // Whether the packed-pair kernels take this plan's FP32 FFTs.
 bool fft2_applicable(const shtb_plan* p) {
   const FFTDesc& fd = p->fft;
-  if (fd.direct || fd.nrad < 2 || (p->nlat & 3)) return false;   // npair even: 16-byte pair loads
+  if (fd.nrad < 2 || (p->nlat & 3)) return false;   // npair even: 16-byte pair loads
   if (fd.n < 64 || fd.n > 2048 || (fd.n & (fd.n - 1))) return false;
   for (int s = 0; s < fd.nrad; ++s)
     if (!(fd.rad[s] == 2 || fd.rad[s] == 4 || fd.rad[s] == 8 || fd.rad[s] == 16)) return false;

@@ -127,7 +127,7 @@ __global__ void plan_setup_kernel(PlanDev P, const double* __restrict__ seedfac,
 static bool factor_fft(int n, FFTDesc& d) {
   d.n = n;
   d.nrad = 0;
-  d.direct = false;
+  d.big = false;
   int k = n;
   // prefer radix 16, 8 and 4, then 2, 3, 5, 7 and small odd primes up to 16: fewer
   // passes over shared memory
@@ -138,9 +138,10 @@ static bool factor_fft(int n, FFTDesc& d) {
   const int odd[] = {3, 5, 7, 11, 13};
   for (int p : odd)
     while (k % p == 0 && d.nrad < 24) { d.rad[d.nrad++] = p; k /= p; }
-  if (k != 1) {
-    d.direct = true;
-    d.nrad = 0;
+  // larger prime factors: passes of their own radix, last (smallest span), in ascending order
+  for (int q = 17; k != 1 && d.nrad < 24; q += 2) {
+    if (q * q > k) q = k;
+    while (k % q == 0 && d.nrad < 24) { d.rad[d.nrad++] = q; k /= q; d.big = true; }
   }
   // FP32 rows: skew i + i/16 leaves every pass of a power-of-two length free of bank
   // conflicts; mixed radices (odd last passes) do better with i + i/8 (fft_padsh).
@@ -342,7 +343,6 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   }
   std::vector<int> rev(nlon);
   for (int k = 0; k < nlon; ++k) {
-    if (p->fft.direct) { rev[k] = k; continue; }
     int pos = 0, kk = k, Ns = nlon;
     for (int s = 0; s < p->fft.nrad; ++s) {
       const int r = p->fft.rad[s];
