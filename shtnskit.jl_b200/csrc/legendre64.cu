@@ -55,6 +55,265 @@ __device__ __forceinline__ void dmma_16x8x4(double (&d)[4], double a0, double a1
       : "d"(a0), "d"(a1), "d"(b0));
 }
 
+__device__ __forceinline__ void cp16(void* smem, const void* gmem, unsigned src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+               "l"(gmem), "r"(src_bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait_group() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// synthesis: CTA = (64 MT pairs, order m, 4 NT fields), four warps of 16 MT pairs
+// ---------------------------------------------------------------------------
+// P never leaves the registers. In the A fragment lane (g, t) holds rows g and g + 8 of
+// column t; with rows = latitude pairs, that lane runs the recurrence of its own pairs over
+// the t-th quarter of the order's degrees, so at step s the four columns are degrees
+// lbeg + t Q + s (Q even: one parity) and every lane's new P value is the A operand as it
+// comes. The contraction over degrees sums in the accumulators of the step's parity whatever
+// the order, so nothing is exchanged between lanes. The coefficients of the four degrees (B
+// fragment: column g, degree t) come from shared memory, kSynSteps steps per stage, filled by
+// cp.async two stages ahead; the skew 4 t doubles and the row stride = 2 mod 16 doubles keep
+// both the 16-byte writes and the fragment reads free of bank conflicts. Per step a warp
+// issues MT NT MMAs (512 FMAs each) for 3 FP64 operations per P value, 2 MT values a lane.
+constexpr int kSynSteps = 8;
+constexpr int kSynStages = 3;
+constexpr int kSynThreads = 128;
+
+template <int NT>
+struct SynSmem {
+  static constexpr int NF = 4 * NT;                          // fields per CTA
+  static constexpr int RS = 8 * NT + 2;                      // doubles per degree
+  static constexpr int STAGE = 4 * kSynSteps * RS + 16;      // doubles
+  static constexpr int TAB = kSynStages * STAGE;             // then alpha and the factor of every degree
+  static constexpr int kPad = 8;                             // steps past lend of the last quarter
+  static size_t bytes(int ndeg) { return (size_t)(TAB + 2 * (ndeg + kPad)) * 8; }
+};
+
+template <int NT, int MT>
+__global__ void __launch_bounds__(kSynThreads, NT == 4 ? 4 : 1)
+    leg_syn64_kernel(PlanDev P, CoefSrc src, Factors F, double2* __restrict__ W, int nf, int row_end) {
+  using SM = SynSmem<NT>;
+  constexpr int NF = SM::NF, RS = SM::RS, KS = kSynSteps;
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_lmin;
+  __shared__ double2 s_start[64 * MT];   // start states of the CTA's pairs
+  const int im = blockIdx.y, m = im * P.mres;
+  const int kb = blockIdx.z * NF;
+  const int npair = P.npair;
+  const long long poff = P.off[im];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int row0 = (blockIdx.x * 4 + warp) * 16 * MT + g;    // pairs row0 + 16 i + 8 h
+  const int lend = min(row_end, P.lrec), ndeg = lend - m + 1;
+  double* sAl = sm + SM::TAB;
+  double* sFa = sAl + ndeg + SM::kPad;
+  if (tid == 0) s_lmin = INT_MAX;
+  // everything the first degrees need that does not depend on where they start
+  double x[MT][2], ra[MT][2], rb[MT][2];
+  int l0[MT][2];
+  int mn = INT_MAX / 2;
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int p = row0 + 16 * i + 8 * h;
+      l0[i][h] = p < npair ? P.l0[(size_t)im * npair + p] : INT_MAX / 2;
+      x[i][h] = p < npair ? P.x[p] : 0.0;
+      ra[i][h] = rb[i][h] = 0.0;
+      mn = min(mn, l0[i][h]);
+    }
+  for (int i = tid; i < 64 * MT; i += kSynThreads) {
+    const int p = blockIdx.x * (64 * MT) + i;
+    s_start[i] = p < npair ? P.start[(size_t)im * npair + p] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  mn = __reduce_min_sync(0xffffffffu, mn);
+  if (lane == 0) atomicMin(&s_lmin, mn);
+  __syncthreads();
+  // degrees from lbeg (an even distance from m, no pair starts below it), a quarter per t
+  const int lbeg = m + ((max(s_lmin, m) - m) & ~1);
+  const int nd = lend - lbeg + 1;                            // <= 0: no pair starts in range
+  const int Q = nd > 0 ? ((nd + 3) / 4 + 1) & ~1 : 0;
+  const int nch = (Q + KS - 1) / KS;
+  const int lq = lbeg + t * Q;                               // this lane's first degree
+  const long long cbase = src.packed == 1 ? (poff - m)
+                          : src.packed == 2 ? lm_base(P.lmax, P.mres, m) : (long long)m * src.ld_m;
+  const double2* st0 = s_start + warp * 16 * MT + g;
+
+  auto stage = [&](int c, int slot) {
+    double* B = sm + slot * SM::STAGE;
+    for (int idx = tid; idx < NF * 4 * KS; idx += kSynThreads) {
+      const int s = idx % KS, q = (idx / KS) & 3, fl = idx / (4 * KS);
+      const int l = lbeg + q * Q + c * KS + s, kf = kb + fl;
+      const bool ok = c * KS + s < Q && l <= lend && kf < nf;
+      const double2* gp = ok ? src.ptr + (long long)kf * src.ld_k + cbase + l : src.ptr;
+      cp16(B + (q * KS + s) * RS + 4 * q + 2 * fl, gp, ok ? 16u : 0u);
+    }
+  };
+  for (int c = 0; c < 2; ++c) {
+    if (c < nch) stage(c, c);
+    cp_commit();
+  }
+#pragma unroll 4
+  for (int i = tid; i < ndeg + SM::kPad; i += kSynThreads) {
+    const bool in = i < ndeg;
+    sAl[i] = in ? P.alpha[poff + i] : 0.0;
+    sFa[i] = in ? factor_at(P, F, poff, m + i, m) : 0.0;
+  }
+  __syncthreads();
+  // state before degree lq: the checkpoint at or below it, rolled forward
+  {
+    const int cs = P.ckstep;
+    const bool in = nd > 0 && lq <= lend;
+    const int ks = in ? (lq - m) / cs : 0, lk = m + ks * cs, nroll = in ? lq - lk : 0;
+    const int mroll = __reduce_max_sync(0xffffffffu, nroll);
+    const double2* ck = P.ckpt + (size_t)(P.ckbase[im] + ks) * npair + row0;
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (in && row0 + 16 * i + 8 * h < npair) {
+          const double2 v = ck[16 * i + 8 * h];
+          ra[i][h] = v.x;
+          rb[i][h] = v.y;
+        }
+    for (int k = 0; k <= mroll; ++k) {
+      if (k > nroll || !in) continue;
+      const int l = lk + k;
+      const double al = sAl[l - m];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (l == l0[i][h]) {
+            ra[i][h] = st0[16 * i + 8 * h].x;
+            rb[i][h] = st0[16 * i + 8 * h].y;
+          }
+          if (k == nroll) continue;   // the state before lq, its own start included
+          const double r = fma(al * x[i][h], ra[i][h], -rb[i][h]);
+          rb[i][h] = ra[i][h];
+          ra[i][h] = r;
+        }
+    }
+  }
+
+  double acc[2][MT][NT][4];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[p][i][j][q] = 0.0;
+
+  int slot = 0;
+  for (int c = 0; c < nch; ++c) {
+    cp_wait_group<1>();
+    __syncthreads();   // stage c is filled; stage c - 1 is read by every warp
+    if (c + 2 < nch) stage(c + 2, slot == 0 ? 2 : slot - 1);
+    cp_commit();
+    const double* B = sm + slot * SM::STAGE + t * (KS * RS + 4) + g;
+    slot = slot == 2 ? 0 : slot + 1;
+    const int s0 = c * KS, ns = min(KS, Q - s0), ls = lq + s0;
+    const double* al = sAl + (ls - m);
+    const double* fa = sFa + (ls - m);
+    bool some = false, start = false;   // a pair has begun by the chunk's end; one begins inside it
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        some |= l0[i][h] < ls + ns;
+        start |= l0[i][h] >= ls + (c == 0) && l0[i][h] < ls + ns;
+      }
+    if (!__any_sync(0xffffffffu, some && ls <= lend)) continue;
+    const bool slow = __any_sync(0xffffffffu, start) || ns < KS;
+    // steps past lend (4 Q <= nd + 7) read zeros from the padding
+    auto step = [&](int s, int par, double a_l, double f_l, bool sel) {
+      double a[MT][2], b[NT];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (sel && ls + s == l0[i][h]) {
+            ra[i][h] = st0[16 * i + 8 * h].x;
+            rb[i][h] = st0[16 * i + 8 * h].y;
+          }
+          const double r = fma(a_l * x[i][h], ra[i][h], -rb[i][h]);
+          rb[i][h] = ra[i][h];
+          ra[i][h] = r;
+          a[i][h] = r * f_l;
+        }
+#pragma unroll
+      for (int j = 0; j < NT; ++j) b[j] = B[s * RS + 8 * j];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) dmma_16x8x4(acc[par][i][j], a[i][0], a[i][1], b[j]);
+    };
+    if (!slow) {
+#pragma unroll
+      for (int s = 0; s < KS; ++s) step(s, s & 1, al[s], fa[s], false);
+    } else {
+      for (int s = 0; s < ns; s += 2) {
+        step(s, 0, al[s], fa[s], true);
+        step(s + 1, 1, al[s + 1], fa[s + 1], true);
+      }
+    }
+  }
+  cp_wait_group<0>();   // no copy of this thread is in flight when the CTA exits
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int pr = row0 + 16 * i + 8 * h;
+      if (pr >= npair) continue;
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const int kf = kb + 4 * j + t;
+        if (kf >= nf) continue;
+        double2* w = W + (((size_t)kf * P.nm + im) * 2) * npair + pr;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) w[(size_t)p * npair] = make_double2(acc[p][i][j][2 * h], acc[p][i][j][2 * h + 1]);
+      }
+    }
+}
+
+template <int NT, int MT>
+static int launch_syn_tile(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end,
+                           int mlim, cudaStream_t st) {
+  auto kern = leg_syn64_kernel<NT, MT>;
+  // shared memory for the longest order (m = 0)
+  const size_t smem = SynSmem<NT>::bytes(std::min(row_end, p->lrec) + 1);
+  if (smem > 227 * 1024) return set_error(SHTB_ERR_UNSUPPORTED, "lmax too large for the FP64 synthesis kernel");
+  SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "synthesis smem attr");
+  const dim3 grid((p->npair + 64 * MT - 1) / (64 * MT), mlim / p->mres + 1, (nf + 4 * NT - 1) / (4 * NT));
+  prof_begin(st);
+  kern<<<grid, kSynThreads, smem, st>>>(p->dev, src, F, (double2*)W, nf, row_end);
+  SHTB_LAUNCHED("legendre synthesis kernel");
+  return SHTB_OK;
+}
+
+int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end,
+                     int mlim, cudaStream_t st) {
+  if (nf <= 2) return launch_simt_syn64(p, src, F, W, nf, row_end, mlim, st);
+  // 32 columns a warp leave registers for four CTAs an SM, 64 for three: 2424 against 2536 us at
+  // lmax 1023 x 64 fields, 57 against 62 at lmax 255 x 32 fields plus a wind field
+  if (nf > 8) return launch_syn_tile<4, 1>(p, src, F, W, nf, row_end, mlim, st);
+  // narrower tiles: two row tiles per warp share each B fragment where that still leaves CTAs
+  // for every SM
+  const bool two = (long long)((p->npair + 127) / 128) * (mlim / p->mres + 1) >= 592;
+  if (nf > 4)
+    return two ? launch_syn_tile<2, 2>(p, src, F, W, nf, row_end, mlim, st)
+               : launch_syn_tile<2, 1>(p, src, F, W, nf, row_end, mlim, st);
+  return two ? launch_syn_tile<1, 2>(p, src, F, W, nf, row_end, mlim, st)
+             : launch_syn_tile<1, 1>(p, src, F, W, nf, row_end, mlim, st);
+}
+
 constexpr int kConsumerWarps = 8;
 
 // Consumer warp layout shared by both directions: per parity an output tile of 64 rows
@@ -72,231 +331,6 @@ struct WarpTile {
 constexpr int kProducerWarps = 4;   // one per SM sub-partition, so the recurrence's FP64 work
                                     // spreads over all four FP64 pipes
 constexpr int kLegThreads = 32 * (kConsumerWarps + kProducerWarps);
-
-// ---------------------------------------------------------------------------
-// synthesis: CTA = (64 pairs, order m, NCOL/2 fields), K chunks of 16 degrees
-// ---------------------------------------------------------------------------
-constexpr int kSynPairs = 64;
-constexpr int kSynDeg = 16;                    // degrees per chunk (8 per parity)
-constexpr int kSynPS = kSynPairs + 4;          // P panel row stride (doubles), = 4 mod 16
-constexpr int kSynCS = 2 * (kSynDeg / 2) + 8;  // coefficient field stride (doubles), = 8 mod 16
-constexpr int kSynStages = 4;
-
-template <int NCOL>
-struct SynSmem {
-  static constexpr int NF = WarpTile<NCOL>::NF;
-  static constexpr int PBUF = 2 * (kSynDeg / 2) * kSynPS;   // [parity][8 degrees][pairs]
-  static constexpr int CBUF = 2 * NF * kSynCS;              // [parity][field][8 degrees x re|im]
-  static constexpr int STAGE = PBUF + CBUF;                 // doubles
-  static constexpr int BAR = kSynStages * STAGE;            // then full[S], empty[S], flags
-  // stages, barriers, abort flag and two pair minima, then alpha and the folded factor of
-  // every degree m..lend
-  static size_t bytes(int ndeg) { return (size_t)BAR * 8 + 2 * kSynStages * 8 + 16 + (size_t)2 * ndeg * 8; }
-};
-
-template <int NCOL>
-__global__ void __launch_bounds__(kLegThreads, 1)
-    leg_syn64_kernel(PlanDev P, CoefSrc src, Factors F, double2* __restrict__ W, int nf, int row_end, int* err) {
-  using WT = WarpTile<NCOL>;
-  using SM = SynSmem<NCOL>;
-  constexpr int NF = WT::NF, S = kSynStages;
-  extern __shared__ __align__(16) double sm[];
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + SM::BAR);
-  unsigned long long* empty = full + S;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + S);
-  int* sLmin = reinterpret_cast<int*>(empty + S) + 1;
-  double* sAl = reinterpret_cast<double*>(empty + S + 2);
-  const int im = blockIdx.y, m = im * P.mres;
-  const int p0 = blockIdx.x * kSynPairs;
-  const int kb = blockIdx.z * NF;
-  const int npair = P.npair;
-  const long long poff = P.off[im];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool producer = warp >= kConsumerWarps;
-  const int lend = min(row_end, P.lrec);
-  const int ndeg = max(lend - m + 1, 0);
-  double* sFa = sAl + ndeg;
-
-  if (tid == 0) {
-    for (int q = 0; q < S; ++q) {
-      pipe_bar_init(&full[q], 64);   // one group of two producer warps fills a stage
-      pipe_bar_init(&empty[q], kConsumerWarps);
-    }
-    *abort_flag = 0;
-    pipe_bar_init_fence();
-  }
-  for (int i = tid; i < ndeg; i += kLegThreads) {
-    sAl[i] = P.alpha[poff + i];
-    sFa[i] = factor_at(P, F, poff, m + i, m);
-  }
-  // producer state: the producer warps form two groups that fill alternate chunks; in
-  // each group, thread q = 32 (w % 2) + lane takes pair p0 + q
-  double px = 0.0, pr0 = 0.0, pr1 = 0.0;
-  int pl0 = INT_MAX / 2;
-  const int pw = warp - kConsumerWarps, pgroup = pw >> 1, pq = 32 * (pw & 1) + lane;
-  const int pp = p0 + pq;
-  if (producer) {
-    if (pp < npair) {
-      px = P.x[pp];
-      pl0 = P.l0[(size_t)im * npair + pp];
-      const double2 v = P.start[(size_t)im * npair + pp];
-      pr0 = v.x;
-      pr1 = v.y;
-    }
-    int mn = pl0;
-    for (int o = 16; o > 0; o >>= 1) mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if (lane == 0 && pw < 2) sLmin[pw] = mn;
-  }
-  __syncthreads();
-  const int lmin = max(min(sLmin[0], sLmin[1]), m);
-  // chunks start at degrees m + 16 k (even l - m first)
-  const int lbeg = m + ((lmin - m) / kSynDeg) * kSynDeg;
-  const int nchunks = (lend >= lbeg) ? (lend - lbeg) / kSynDeg + 1 : 0;
-  const long long cbase = src.packed == 1 ? (poff - m)
-                          : src.packed == 2 ? lm_base(P.lmax, P.mres, m) : (long long)m * src.ld_m;
-
-  if (producer) {
-    for (int c = pgroup; c < nchunks; c += 2) {
-      const int st = c % S;
-      if (c >= S && !pipe_wait(&empty[st], ((c / S) - 1) & 1, abort_flag, err)) break;
-      double* Pn = sm + st * SM::STAGE;
-      double* C = Pn + SM::PBUF;
-      const int lc = lbeg + c * kSynDeg;
-      // coefficients: 8 consecutive threads fill one (parity, field) row of 8 degrees
-      for (int idx = pq; idx < NF * kSynDeg; idx += 64) {
-        const int s = 2 * (idx & 7) + ((idx >> 3) & 1), fl = idx / kSynDeg;
-        const int l = lc + s, kf = kb + fl;
-        const bool ok = (l <= lend) && (kf < nf);
-        const double2* gp = ok ? src.ptr + (long long)kf * src.ld_k + cbase + l : src.ptr;
-        pipe_cp16(C + ((s & 1) * NF + fl) * kSynCS + 2 * (s >> 1), gp, ok ? 16u : 0u);
-      }
-      pipe_arrive_cp_async(&full[st]);
-      // P panel column of pair pp, the per-degree factors folded in (zero past lend): the
-      // chain starts at the checkpoint at or below lc
-      const int ks = (lc - m) / P.ckstep, lk = m + ks * P.ckstep;
-      double ra = 0.0, rb = 0.0;
-      if (pp < npair) {
-        const double2 v = P.ckpt[(size_t)(P.ckbase[im] + ks) * npair + pp];
-        ra = v.x;
-        rb = v.y;
-      }
-      for (int l = lk; l < lc; ++l) {   // only when the checkpoints are sparser than a chunk
-        ra = (l == pl0) ? pr0 : ra;
-        rb = (l == pl0) ? pr1 : rb;
-        const double r = fma(sAl[l - m] * px, ra, -rb);
-        rb = ra;
-        ra = r;
-      }
-#pragma unroll
-      for (int s = 0; s < kSynDeg; ++s) {
-        const int l = lc + s;
-        const bool in = l <= lend;
-        const double a = in ? sAl[l - m] : 0.0, f = in ? sFa[l - m] : 0.0;
-        ra = (l == pl0) ? pr0 : ra;
-        rb = (l == pl0) ? pr1 : rb;
-        const double r = fma(a * px, ra, -rb);
-        rb = ra;
-        ra = r;
-        Pn[((s & 1) * (kSynDeg / 2) + (s >> 1)) * kSynPS + pq] = r * f;
-      }
-      pipe_arrive(&full[st]);
-    }
-    pipe_cp_wait_all();   // no copy of this thread is in flight when the CTA exits
-    return;
-  }
-
-  // consumer warp geometry
-  const int par = warp / WT::WPP, rg = (warp % WT::WPP) / WT::CG, cg = warp % WT::CG;
-  const int rowbase = rg * (64 / WT::RG), colbase = cg * (NCOL / WT::CG);
-  const int g = lane >> 2, t = lane & 3;
-  // first degree any pair of this warp's rows needs
-  int wlmin = INT_MAX / 2;
-  {
-    const int pr = p0 + rowbase + lane;
-    if (lane < 64 / WT::RG && pr < npair) wlmin = P.l0[(size_t)im * npair + pr];
-    for (int o = 16; o > 0; o >>= 1) wlmin = min(wlmin, __shfl_xor_sync(0xffffffffu, wlmin, o));
-  }
-  double acc[WT::MT][WT::NT][4];
-#pragma unroll
-  for (int i = 0; i < WT::MT; ++i)
-#pragma unroll
-    for (int j = 0; j < WT::NT; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
-
-  for (int c = 0; c < nchunks; ++c) {
-    const int st = c % S;
-    if (!pipe_wait(&full[st], (c / S) & 1, abort_flag, err)) break;
-    const int lc = lbeg + c * kSynDeg;
-    if (lc + kSynDeg - 1 >= wlmin) {
-      const double* Pn = sm + st * SM::STAGE + par * (kSynDeg / 2) * kSynPS;
-      const double* C = sm + st * SM::STAGE + SM::PBUF + par * NF * kSynCS;
-#pragma unroll
-      for (int ks = 0; ks < kSynDeg / 8; ++ks) {
-        double a[WT::MT][2], b[WT::NT];
-#pragma unroll
-        for (int i = 0; i < WT::MT; ++i) {
-          const double* pa = Pn + (ks * 4 + t) * kSynPS + rowbase + i * 16 + g;
-          a[i][0] = pa[0];
-          a[i][1] = pa[8];
-        }
-#pragma unroll
-        for (int j = 0; j < WT::NT; ++j) {
-          const int col = colbase + j * 8 + g;
-          b[j] = C[(col >> 1) * kSynCS + 2 * (ks * 4 + t) + (col & 1)];
-        }
-#pragma unroll
-        for (int i = 0; i < WT::MT; ++i)
-#pragma unroll
-          for (int j = 0; j < WT::NT; ++j) dmma_16x8x4(acc[i][j], a[i][0], a[i][1], b[j]);
-      }
-    }
-    __syncwarp();
-    if (lane == 0) pipe_arrive(&empty[st]);
-  }
-  if (*abort_flag) return;
-#pragma unroll
-  for (int i = 0; i < WT::MT; ++i)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int pr = p0 + rowbase + i * 16 + g + 8 * h;
-      if (pr >= npair) continue;
-#pragma unroll
-      for (int j = 0; j < WT::NT; ++j) {
-        const int kf = kb + (colbase + j * 8) / 2 + t;
-        if (kf >= nf) continue;
-        W[(((size_t)kf * P.nm + im) * 2 + par) * npair + pr] = make_double2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
-      }
-    }
-}
-
-template <int NCOL>
-static int launch_syn_ncol(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end,
-                           int mlim, cudaStream_t st) {
-  auto kern = leg_syn64_kernel<NCOL>;
-  // shared memory for the longest order (m = 0)
-  const int ndeg = std::min(row_end, p->lrec) + 1;
-  const size_t smem = SynSmem<NCOL>::bytes(ndeg);
-  if (smem > 227 * 1024) return set_error(SHTB_ERR_UNSUPPORTED, "lmax too large for the FP64 synthesis kernel");
-  SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "synthesis smem attr");
-  constexpr int NF = WarpTile<NCOL>::NF;
-  dim3 grid((p->npair + kSynPairs - 1) / kSynPairs, mlim / p->mres + 1, (nf + NF - 1) / NF);
-  prof_begin(st);
-  kern<<<grid, kLegThreads, smem, st>>>(p->dev, src, F, (double2*)W, nf, row_end, p->d_err);
-  SHTB_LAUNCHED("legendre synthesis kernel");
-  return SHTB_OK;
-}
-
-int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, void* W, int nf, int row_end,
-                     int mlim, cudaStream_t st) {
-  if (nf <= 2) return launch_simt_syn64(p, src, F, W, nf, row_end, mlim, st);
-  if (nf > 32) return launch_syn_ncol<128>(p, src, F, W, nf, row_end, mlim, st);
-  if (nf > 16) return launch_syn_ncol<64>(p, src, F, W, nf, row_end, mlim, st);
-  if (nf > 8) return launch_syn_ncol<32>(p, src, F, W, nf, row_end, mlim, st);
-  if (nf > 4) return launch_syn_ncol<16>(p, src, F, W, nf, row_end, mlim, st);
-  return launch_syn_ncol<8>(p, src, F, W, nf, row_end, mlim, st);
-}
 
 // ---------------------------------------------------------------------------
 // analysis: CTA = (128 degrees of order m, NCOL/2 fields), K chunks of kAnaPairs pairs
