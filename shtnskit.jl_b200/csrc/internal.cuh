@@ -41,12 +41,12 @@ cudaError_t noalloc_scratch_address(void** out);
     if (_rc != SHTB_OK) return _rc;                                 \
   } while (0)
 
-// Degrees of one FP64 analysis tile (64 of each parity).
+// Degrees of one tile of the few-field FP64 analysis.
 constexpr int kAnaTile = 128;
 // Recurrence chains start at multiples of kStartStep degrees from their order.
 constexpr int kStartStep = 8;
-// Largest checkpoint table the plan keeps (bytes); the spacing grows from 16 degrees
-// until the table fits.
+// Largest checkpoint table the plan keeps (bytes); the spacing grows from 8 degrees (the
+// chains of the FP64 analysis GEMM) until the table fits.
 constexpr size_t kCkptBudget = size_t(2) << 30;
 
 // ---------------------------------------------------------------------------
@@ -66,10 +66,11 @@ struct PlanDev {
   // the state (r_{t-1}, r_{t-2}) before degree t = m + k * ckstep
   const double2* ckpt;
   const int* ckbase;       // [nm]
-  int ckstep;              // 16, 32, 64 or 128 (a divisor of kAnaTile)
-  // FP64 analysis tiles of kAnaTile degrees: (im, t0, checkpoint index of t0, 0)
+  int ckstep;              // 8, 16, 32, 64 or 128 (a divisor of kAnaTile)
+  // FP64 analysis tiles (im, t0, 0, 0) of kAnaTile and of 64 degrees
   const int4* atiles;
-  int natiles;
+  const int4* atiles64;
+  int natiles, natiles64;
 };
 
 // FFT description for nlon

@@ -1,38 +1,23 @@
-// legendre64.cu — FP64 associated-Legendre contraction kernels on the FP64 tensor cores.
+// legendre64.cu — FP64 associated-Legendre contraction kernels on the FP64 tensor cores
+// (three or more fields; simt.cu takes one and two).
 //
 // Both directions work per order m on latitude PAIRS (i, nlat-1-i) folded by
 // equatorial symmetry: P_l^m(-x) = (-1)^(l-m) P_l^m(x), so every contraction is
-// split into degrees of even (E) and odd (O) parity l-m. Per order and parity each
-// direction is a dense GEMM whose P operand is regenerated on the fly:
-//   synthesis  W[pair, col] = sum_l P_l(x_pair) a[l, col]     (K = degrees)
-//   analysis   a[l, col]    = sum_pair P_l(x_pair) W[pair, col] (K = latitude pairs)
-// with col = (field, re|im).
+// split into degrees of even (E) and odd (O) parity l-m:
+//   synthesis  W[pair, col] = sum_l P_l(x_pair) a[l, col]
+//   analysis   a[l, col]    = sum_pair P_l(x_pair) W[pair, col]
+// with col = (field, re|im), on mma.sync m16n8k4 .f64 (512 FMAs in 32 cycles of an SM
+// sub-partition, the FP64 units' full rate).
 //
-// P_l^m is never stored in global memory: four producer warps per CTA regenerate the
-// panels of the coming K chunks into a ring of shared-memory stages with the c-scaled
-// three-term recurrence
+// P is regenerated where it is used: the c-scaled recurrence
 //   r_l = alpha_l x r_{l-1} - r_{l-2},   P_l^m = c_l r_l
-// (one DMUL + one DFMA per value), started from per-(m, pair) records that carry the
-// reference's extended-range sectoral seed (values below 2^-480 are zero until the
-// record's first degree l0) and, inside the degree range, from the plan's recurrence
-// checkpoints (every ckstep degrees), so the panel of a chunk is many short independent
-// chains rather than one long one; they fill the same stage with the chunk's coefficient
-// or Fourier panel by cp.async. Eight consumer warps multiply each stage with FP64 MMAs
-// (mma.sync m16n8k4 .f64: 512 FMAs per instruction, the DFMA units' full rate at an
-// eighth of the issue slots of DFMA code), operands from shared memory, accumulators in
-// registers. Stages are handed over on mbarriers (full: panels written and copies landed;
-// empty: every consumer warp done), so the producers run up to a ring's depth ahead and
-// their latency-bound recurrence, which shares the FP64 pipe with the MMAs, never holds
-// the consumers at a CTA-wide barrier. Every wait is bounded (pipe.cuh).
-//
-// Per-(l, m) multipliers (c_l, normalization, phi scales) are folded into the P panel
-// (synthesis) or applied at the store (analysis). Chunks whose P values are all zero
-// (every pair of the chunk still below its record's first degree, near the poles at
-// high m) are skipped: adding their zeros changes nothing.
+// (one DMUL + one DFMA per value) runs in the lanes whose MMA fragment needs the value, so it
+// passes through neither global nor shared memory. Each lane's chain starts from the plan's
+// recurrence checkpoints (every ckstep degrees), which carry the reference's extended-range
+// sectoral seed (values below 2^-480 are zero before the pair's start degree).
 #include <climits>
 
 #include "kernels.cuh"
-#include "pipe.cuh"
 
 namespace shtb {
 
@@ -57,6 +42,11 @@ __device__ __forceinline__ void dmma_16x8x4(double (&d)[4], double a0, double a1
 
 __device__ __forceinline__ void cp16(void* smem, const void* gmem, unsigned src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+               "l"(gmem), "r"(src_bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp8(void* smem, const void* gmem, unsigned src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
                "l"(gmem), "r"(src_bytes)
                : "memory");
 }
@@ -314,248 +304,201 @@ int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, v
              : launch_syn_tile<1, 1>(p, src, F, W, nf, row_end, mlim, st);
 }
 
-constexpr int kConsumerWarps = 8;
-
-// Consumer warp layout shared by both directions: per parity an output tile of 64 rows
-// by NCOL columns, split over kConsumerWarps / 2 warps as RG row groups x CG column
-// groups; a warp holds MT x NT fragments of 16 x 8.
-template <int NCOL>
-struct WarpTile {
-  static constexpr int WPP = kConsumerWarps / 2;   // warps per parity
-  static constexpr int RG = NCOL >= 64 ? 2 : 4, CG = WPP / RG;
-  static constexpr int MT = 64 / RG / 16, NT = NCOL / CG / 8;
-  static constexpr int NF = NCOL / 2;   // fields per CTA
-  static_assert(MT >= 1 && NT >= 1 && RG * CG == WPP, "warp tile");
-};
-
-constexpr int kProducerWarps = 4;   // one per SM sub-partition, so the recurrence's FP64 work
-                                    // spreads over all four FP64 pipes
-constexpr int kLegThreads = 32 * (kConsumerWarps + kProducerWarps);
-
 // ---------------------------------------------------------------------------
-// analysis: CTA = (128 degrees of order m, NCOL/2 fields), K chunks of kAnaPairs pairs
+// analysis: CTA = 64 degrees of one order, 8 MT CG fields; four warps = CG column groups
+// x 4 / CG parts of the latitude sum
 // ---------------------------------------------------------------------------
-constexpr int kAnaPairs = 16;                    // latitude pairs per chunk
-constexpr int kAnaAS = kAnaPairs + 4;            // P panel row stride (doubles), = 4 mod 16
-constexpr int kAnaBS = 2 * kAnaPairs + 8;        // Fourier panel field stride (doubles), = 8 mod 16
-constexpr int kAnaMaxChunks = 512;               // npair <= 8192
-constexpr int kAnaStages = 3;
+// The transposed product a[l, col]^T = sum_pair W[pair, col] P_l(x_pair): A (16 x 4) holds 8
+// fields (rows g real, g + 8 imaginary: one 16-byte load of W gives a lane both) at 4 pairs,
+// B (4 x 8) the P values of pair t at the degrees t0 + 8 g + s. Lane (g, t) therefore runs one
+// recurrence chain of 8 degrees from the plan's checkpoint at t0 + 8 g, and each new value is
+// the B operand of step s as it comes, for MT tiles of 8 fields: no P panel, no shared memory
+// and no barrier in the loop. Each step has its own accumulators (8 steps x MT x 4 doubles).
+// Four pairs take 8 chain steps (2 FP64 operations a lane) and 8 MT MMAs; the operands of
+// the next four (MT x 32 bytes of W, a checkpoint, x, the pair's first degree) load meanwhile.
+constexpr int kAnaThreads = 128;
+constexpr int kAnaSteps = 8;             // degrees per chain; 8 chains per tile
+constexpr int kAnaDeg = 8 * kAnaSteps;   // degrees per tile
+constexpr int kAnaRing = 4;              // operand ring: steps of four pairs in flight, plus one
 
-template <int NCOL>
-struct AnaSmem {
-  static constexpr int NF = WarpTile<NCOL>::NF;
-  static constexpr int ABUF = 2 * 64 * kAnaAS;   // [parity][64 rows][pairs]
-  static constexpr int BBUF = 2 * NF * kAnaBS;   // [parity][field][pairs x re|im]
-  static constexpr int STAGE = ABUF + BBUF;
-  static constexpr int ALPH = kAnaStages * STAGE;          // alpha of the tile's 128 degrees
-  static constexpr int BAR = ALPH + kAnaTile;              // then full[S], empty[S], flags, chunk list
-  static size_t bytes() { return (size_t)BAR * 8 + 2 * kAnaStages * 8 + 16 + (kAnaMaxChunks + 8) * 4; }
-};
-
-template <int NCOL>
-__global__ void __launch_bounds__(kLegThreads, 1)
+template <int MT, int CG>
+__global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
     leg_ana64_kernel(PlanDev P, const double2* __restrict__ W, int nf, int row_end, int mlim, CoefSink dst, Factors F,
-                     int zero_fill, int* err) {
-  using WT = WarpTile<NCOL>;
-  using SM = AnaSmem<NCOL>;
-  constexpr int NF = WT::NF, S = kAnaStages;
-  extern __shared__ __align__(16) double sm[];
-  double* salph = sm + SM::ALPH;
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(sm + SM::BAR);
-  unsigned long long* empty = full + S;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + S);
-  int* slist = reinterpret_cast<int*>(empty + S) + 4;   // nonzero chunks, then their count
-  const int4 tile = P.atiles[blockIdx.x];
-  const int im = tile.x, t0 = tile.y, ck0 = tile.z, m = im * P.mres;
+                     int zero_fill) {
+  constexpr int SL = kAnaSteps, KS = 4 / CG;
+  __shared__ __align__(16) unsigned char buf[4 * kAnaRing * ((2 * MT + 1) * 512 + 256)];
+  static_assert((KS - 1) * CG * SL * 4 * 32 * 8 <= sizeof(buf), "partial sums");
+  const int4 tile = P.atiles64[blockIdx.x];
+  const int im = tile.x, t0 = tile.y, m = im * P.mres;
   const int lend = min(row_end, P.lrec);
   if (m > mlim || t0 > lend) return;
-  const int kb = blockIdx.y * NF;
   const int npair = P.npair;
   const long long poff = P.off[im];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool producer = warp >= kConsumerWarps;
-  const int tlast = min(t0 + kAnaTile - 1, lend);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int cg = warp % CG, kw = warp / CG;
+  const int kb = blockIdx.y * (8 * MT * CG);            // the CTA's first field
+  const int kf0 = kb + 8 * MT * cg + g;                 // this lane's field of tile 0
+  const int lg = t0 + SL * g;                           // first degree of this lane's chain
+  const int tlast = min(t0 + kAnaDeg - 1, lend);
+  // this lane's chain: checkpoint, degrees from it to lg, alpha of its steps
+  const int cs = P.ckstep;
+  const int ks = (min(lg, P.lrec) - m) / cs, nroll = lg <= P.lrec ? lg - m - ks * cs : 0;
+  const int mroll = __reduce_max_sync(0xffffffffu, nroll);
+  const double2* ck = P.ckpt + (size_t)(P.ckbase[im] + ks) * npair;
+  const int* pl0 = P.l0 + (size_t)im * npair;
+  double al[SL];
+#pragma unroll
+  for (int s = 0; s < SL; ++s) al[s] = (lg + s <= lend) ? P.alpha[poff + (lg + s - m)] : 0.0;
+  const size_t wld = (size_t)P.nm * 2 * npair;
 
-  if (tid == 0) {
-    for (int q = 0; q < S; ++q) {
-      pipe_bar_init(&full[q], 32 * kProducerWarps);
-      pipe_bar_init(&empty[q], kConsumerWarps);
+  double acc[SL][MT][4];
+#pragma unroll
+  for (int s = 0; s < SL; ++s)
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[s][i][q] = 0.0;
+
+  // leading groups of 32 pairs that all start above the tile hold only zeros
+  const int nk = (npair + 3) / 4;
+  int k0 = 0;
+  for (; k0 < nk; k0 += 8) {
+    const int p = 4 * k0 + lane;
+    if (__any_sync(0xffffffffu, p < npair && pl0[p] <= tlast)) break;
+  }
+  // operand ring: each lane copies its own operands of the next RG - 1 steps (a checkpoint, x,
+  // W of MT fields, E and O) and reads them back itself, so no barrier is needed
+  constexpr int RG = kAnaRing, NS = 2 * MT + 1;
+  double2* ring = reinterpret_cast<double2*>(buf) + (warp * RG * NS) * 32 + lane;
+  double* xring = reinterpret_cast<double*>(buf + 4 * RG * NS * 512) + warp * RG * 32 + lane;
+  // fields and chains past the end read valid operands, nothing is stored for them; pairs
+  // past the end read zeros
+  const double2* Wi[MT];
+#pragma unroll
+  for (int i = 0; i < MT; ++i) Wi[i] = W + (size_t)min(kf0 + 8 * i, nf - 1) * wld + (size_t)im * 2 * npair;
+  auto fetch = [&](int k, int st) {
+    const int p = 4 * k + t;
+    const unsigned n = p < npair ? 16u : 0u;
+    const int pc = p < npair ? p : 0;
+    double2* r = ring + st * (NS * 32);
+    cp16(r, ck + pc, n);
+    cp8(xring + st * 32, P.x + pc, n >> 1);
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      cp16(r + (1 + 2 * i) * 32, Wi[i] + pc, n);
+      cp16(r + (2 + 2 * i) * 32, Wi[i] + npair + pc, n);
     }
-    *abort_flag = 0;
-    pipe_bar_init_fence();
+  };
+#pragma unroll
+  for (int i = 0; i < RG - 1; ++i) {
+    fetch(k0 + kw + i * KS, i);
+    cp_commit();
   }
-  for (int i = tid; i < kAnaTile; i += kLegThreads) {
-    const int l = t0 + i;
-    salph[i] = (l <= lend) ? P.alpha[poff + (l - m)] : 0.0;
-  }
-  // chunks with a nonzero P value: some pair's first significant degree is <= tlast
-  const int nch = (npair + kAnaPairs - 1) / kAnaPairs;
-  if (warp == 0) {
-    int cnt = 0;
-    for (int c0 = 0; c0 < nch; c0 += 32) {
-      const int c = c0 + lane;
-      bool nz = false;
-      if (c < nch) {
-        int mn = INT_MAX;
-        for (int q = 0; q < kAnaPairs; ++q) {
-          const int p = c * kAnaPairs + q;
-          if (p < npair) mn = min(mn, P.l0[(size_t)im * npair + p]);
-        }
-        nz = mn <= tlast;
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, nz);
-      if (nz) slist[cnt + __popc(bal & ((1u << lane) - 1u))] = c;
-      cnt += __popc(bal);
+  int st = 0;
+  for (int k = k0 + kw; k < nk; k += KS) {
+    fetch(k + (RG - 1) * KS, st == 0 ? RG - 1 : st - 1);
+    cp_commit();
+    cp_wait_group<RG - 1>();
+    const double2* r = ring + st * (NS * 32);
+    const double x = xring[st * 32];
+    double ra = r[0].x, rb = r[0].y;
+    double2 e[MT], o[MT];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+      e[i] = r[(1 + 2 * i) * 32];
+      o[i] = r[(2 + 2 * i) * 32];
     }
-    if (lane == 0) slist[kAnaMaxChunks] = cnt;
-  }
-  __syncthreads();
-  const int nz = slist[kAnaMaxChunks];
-
-  if (producer) {
-    // every producer thread takes part in every chunk: thread q = 32 w + lane runs the chain
-    // of pair q % 16 over the tile's checkpoint segment q / 16 (ckstep degrees)
-    const int ptid = tid - 32 * kConsumerWarps, pq = ptid % kAnaPairs, seg = ptid / kAnaPairs;
-    const int cs = P.ckstep, nseg = kAnaTile / cs;
-    const bool chain = seg < nseg && t0 + seg * cs <= P.lrec;
-    for (int ci = 0; ci < nz; ++ci) {
-      const int st = ci % S;
-      if (ci >= S && !pipe_wait(&empty[st], ((ci / S) - 1) & 1, abort_flag, err)) break;
-      const int c = slist[ci];
-      double* A = sm + st * SM::STAGE;
-      double* B = A + SM::ABUF;
-      for (int idx = ptid; idx < 2 * NF * kAnaPairs; idx += 32 * kProducerWarps) {
-        const int q = idx % kAnaPairs, rest = idx / kAnaPairs, fl = rest % NF, pr = rest / NF;
-        const int pair = c * kAnaPairs + q, kf = kb + fl;
-        const bool ok = pair < npair && kf < nf;
-        const double2* gp = ok ? W + (((size_t)kf * P.nm + im) * 2 + pr) * npair + pair : W;
-        pipe_cp16(B + (pr * NF + fl) * kAnaBS + 2 * q, gp, ok ? 16u : 0u);
+    st = st == RG - 1 ? 0 : st + 1;
+    if (mroll) {
+      // checkpoints sparser than the chains: roll forward, past the pair's start if it lies between
+      double2 s0 = make_double2(0.0, 0.0);
+      int l0 = INT_MAX;
+      if (4 * k + t < npair) {
+        s0 = P.start[(size_t)im * npair + 4 * k + t];
+        l0 = pl0[4 * k + t];
       }
-      pipe_arrive_cp_async(&full[st]);
-      if (seg < nseg) {
-        const int p = c * kAnaPairs + pq;
-        double x = 0.0, ra = 0.0, rb = 0.0, r0 = 0.0, r1 = 0.0;
-        int l0 = INT_MAX / 2;
-        if (p < npair && chain) {
-          x = P.x[p];
-          const double2 stv = P.ckpt[(size_t)(ck0 + seg) * npair + p];
-          ra = stv.x;
-          rb = stv.y;
-          l0 = P.l0[(size_t)im * npair + p];
-          const double2 v = P.start[(size_t)im * npair + p];
-          r0 = v.x;
-          r1 = v.y;
+      for (int i = 0; i <= mroll; ++i) {
+        const int l = lg - nroll + i;
+        if (i > nroll) continue;
+        if (l == l0) {
+          ra = s0.x;
+          rb = s0.y;
         }
-        const int d0 = seg * cs;
-        double* Ar = A + pq;
-#pragma unroll 4
-        for (int s = 0; s < cs; ++s) {
-          const int d = d0 + s, l = t0 + d;
-          ra = (l == l0) ? r0 : ra;
-          rb = (l == l0) ? r1 : rb;
-          const double r = fma(salph[d] * x, ra, -rb);
-          rb = ra;
-          ra = r;
-          Ar[((d & 1) * 64 + (d >> 1)) * kAnaAS] = r;
-        }
+        if (i == nroll) continue;   // the state before lg
+        const double q = fma(P.alpha[poff + (l - m)] * x, ra, -rb);
+        rb = ra;
+        ra = q;
       }
-      pipe_arrive(&full[st]);
     }
-    pipe_cp_wait_all();   // no copy of this thread is in flight when the CTA exits
-    return;
+#pragma unroll
+    for (int s = 0; s < SL; ++s) {
+      const double q = fma(al[s] * x, ra, -rb);
+      rb = ra;
+      ra = q;
+#pragma unroll
+      for (int i = 0; i < MT; ++i) dmma_16x8x4(acc[s][i], (s & 1) ? o[i].x : e[i].x, (s & 1) ? o[i].y : e[i].y, q);
+    }
   }
-
-  const int par = warp / WT::WPP, rg = (warp % WT::WPP) / WT::CG, cg = warp % WT::CG;
-  const int rowbase = rg * (64 / WT::RG), colbase = cg * (NCOL / WT::CG);
-  const int g = lane >> 2, t = lane & 3;
-  double acc[WT::MT][WT::NT][4];
+  cp_wait_group<0>();   // no copy of this thread is in flight when the CTA exits
+  if constexpr (KS > 1) {
+    // add the parts of the latitude sum: warps kw > 0 hand theirs over in the ring's memory
+    double* part = reinterpret_cast<double*>(buf);
+    __syncthreads();
 #pragma unroll
-  for (int i = 0; i < WT::MT; ++i)
+    for (int i = 0; i < MT; ++i) {
+      if (i > 0) __syncthreads();
+      if (kw > 0) {
+        double* d = part + ((kw - 1) * CG + cg) * SL * 4 * 32 + lane;
 #pragma unroll
-    for (int j = 0; j < WT::NT; ++j)
+        for (int s = 0; s < SL; ++s)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.0;
-
-  // 16-row fragments whose first degree lies past lend hold no output: no MMAs for them
-  // (m-tiles are in increasing degree order, so live[0] false means none is live)
-  bool live[WT::MT];
-#pragma unroll
-  for (int i = 0; i < WT::MT; ++i) live[i] = t0 + 2 * (rowbase + i * 16) + par <= lend;
-
-  for (int ci = 0; ci < nz; ++ci) {
-    const int st = ci % S;
-    if (!pipe_wait(&full[st], (ci / S) & 1, abort_flag, err)) break;
-    const double* A = sm + st * SM::STAGE + par * 64 * kAnaAS;
-    const double* B = sm + st * SM::STAGE + SM::ABUF + par * NF * kAnaBS;
-#pragma unroll
-    for (int ks = 0; ks < kAnaPairs / 4 && live[0]; ++ks) {
-      double a[WT::MT][2], b[WT::NT];
-#pragma unroll
-      for (int i = 0; i < WT::MT; ++i) {
-        const double* pa = A + (rowbase + i * 16 + g) * kAnaAS + ks * 4 + t;
-        a[i][0] = pa[0];
-        a[i][1] = pa[8 * kAnaAS];
+          for (int q = 0; q < 4; ++q) d[(s * 4 + q) * 32] = acc[s][i][q];
       }
+      __syncthreads();
+      if (kw == 0)
+        for (int w = 0; w < KS - 1; ++w) {
+          const double* d = part + (w * CG + cg) * SL * 4 * 32 + lane;
 #pragma unroll
-      for (int j = 0; j < WT::NT; ++j) {
-        const int col = colbase + j * 8 + g;
-        b[j] = B[(col >> 1) * kAnaBS + 2 * (ks * 4 + t) + (col & 1)];
-      }
+          for (int s = 0; s < SL; ++s)
 #pragma unroll
-      for (int i = 0; i < WT::MT; ++i)
-        if (live[i]) {
-#pragma unroll
-          for (int j = 0; j < WT::NT; ++j) dmma_16x8x4(acc[i][j], a[i][0], a[i][1], b[j]);
+            for (int q = 0; q < 4; ++q) acc[s][i][q] += d[(s * 4 + q) * 32];
         }
     }
-    __syncwarp();
-    if (lane == 0) pipe_arrive(&empty[st]);
   }
-  if (*abort_flag) return;
-
-  const long long dbase = dst.packed == 1 ? (poff - m)
-                          : dst.packed == 2 ? lm_base(P.lmax, P.mres, m) : (long long)m * dst.ld_m;
   const int lcap = dst.packed == 1 ? lend : min(lend, P.lmax);
+  if (kw == 0) {
+    const long long dbase = dst.packed == 1 ? (poff - m)
+                            : dst.packed == 2 ? lm_base(P.lmax, P.mres, m) : (long long)m * dst.ld_m;
+    // accumulator columns 2t and 2t + 1 are the chains 2t, 2t + 1
 #pragma unroll
-  for (int i = 0; i < WT::MT; ++i)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int row = rowbase + i * 16 + g + 8 * h;
-      const int l = t0 + 2 * row + par;
-      if (l > lcap) continue;
-      const double s = factor_at(P, F, poff, l, m);
+      for (int s = 0; s < SL; ++s) {
+        const int l = t0 + SL * (2 * t + c) + s;
+        if (l > lcap) continue;
+        const double f = factor_at(P, F, poff, l, m);
 #pragma unroll
-      for (int j = 0; j < WT::NT; ++j) {
-        const int kf = kb + (colbase + j * 8) / 2 + t;
-        if (kf >= nf) continue;
-        dst.ptr[(long long)kf * dst.ld_k + dbase + l] = make_double2(acc[i][j][2 * h] * s, acc[i][j][2 * h + 1] * s);
+        for (int i = 0; i < MT; ++i)
+          if (kf0 + 8 * i < nf)
+            dst.ptr[(long long)(kf0 + 8 * i) * dst.ld_k + dbase + l] = make_double2(acc[s][i][c] * f, acc[s][i][2 + c] * f);
       }
-    }
+  }
   if (zero_fill && !dst.packed && t0 == m) {
-    const int nz_lo = m, nz_hi = P.lmax - lcap;  // rows [0, m) and (lcap, lmax]
-    const int nrow = nz_lo + max(nz_hi, 0);
-    for (int idx = tid; idx < nrow * NF; idx += 32 * kConsumerWarps) {
-      const int r = idx % nrow, fl = idx / nrow, kf = kb + fl;
-      if (kf >= nf) continue;
-      const int l = (r < nz_lo) ? r : lcap + 1 + (r - nz_lo);
-      dst.ptr[(long long)kf * dst.ld_k + (long long)m * dst.ld_m + l] = make_double2(0.0, 0.0);
+    const int nrow = m + max(P.lmax - lcap, 0);  // rows [0, m) and (lcap, lmax]
+    const int nfl = min(8 * MT * CG, nf - kb);
+    for (int f = warp; f < nfl; f += 4) {
+      double2* col = dst.ptr + (long long)(kb + f) * dst.ld_k + (long long)m * dst.ld_m;
+      for (int r = lane; r < nrow; r += 32) col[(r < m) ? r : lcap + 1 + (r - m)] = make_double2(0.0, 0.0);
     }
   }
 }
 
-template <int NCOL>
-static int launch_ana_ncol(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
+template <int MT, int CG>
+static int launch_ana_tile(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                            const Factors& F, int zero_fill, cudaStream_t st) {
-  if ((p->npair + kAnaPairs - 1) / kAnaPairs > kAnaMaxChunks)
-    return set_error(SHTB_ERR_UNSUPPORTED, "nlat too large for the FP64 analysis kernel");
-  auto kern = leg_ana64_kernel<NCOL>;
-  const size_t smem = AnaSmem<NCOL>::bytes();
-  SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "analysis smem attr");
-  constexpr int NF = WarpTile<NCOL>::NF;
-  dim3 grid(p->dev.natiles, (nf + NF - 1) / NF);
+  const dim3 grid(p->dev.natiles64, (nf + 8 * MT * CG - 1) / (8 * MT * CG));
   prof_begin(st);
-  kern<<<grid, kLegThreads, smem, st>>>(p->dev, (const double2*)W, nf, row_end, mlim, dst, F, zero_fill, p->d_err);
+  leg_ana64_kernel<MT, CG><<<grid, kAnaThreads, 0, st>>>(p->dev, (const double2*)W, nf, row_end, mlim, dst, F, zero_fill);
   SHTB_LAUNCHED("legendre analysis kernel");
   return SHTB_OK;
 }
@@ -563,11 +506,10 @@ static int launch_ana_ncol(const shtb_plan* p, const void* W, int nf, int row_en
 int launch_leg_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                      const Factors& F, int zero_fill, cudaStream_t st) {
   if (nf <= 2) return launch_simt_ana64(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 32) return launch_ana_ncol<128>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 16) return launch_ana_ncol<64>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 8) return launch_ana_ncol<32>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 4) return launch_ana_ncol<16>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  return launch_ana_ncol<8>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (nf > 32) return launch_ana_tile<2, 4>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (nf > 16) return launch_ana_tile<2, 2>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (nf > 8) return launch_ana_tile<2, 1>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  return launch_ana_tile<1, 1>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
 }
 
 }  // namespace shtb
