@@ -106,6 +106,8 @@ _lock = threading.Lock()
 def load(path: str | os.PathLike | None = None) -> ctypes.CDLL:
     """Load the library once; raise BackendUnavailableError when it is not built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

@@ -89,7 +89,8 @@ class SHTConfig:
     # --- derived quantities -------------------------------------------------
     @property
     def nlm(self) -> int:
-        return sum(self.lmax - m + 1 for m in range(0, self.mmax + 1, self.mres))
+        n = self.mmax // self.mres + 1                  # orders 0, mres, ..., each lmax - m + 1 degrees
+        return n * (self.lmax + 1) - self.mres * (n * (n - 1) // 2)
 
     @property
     def canonical(self) -> bool:
@@ -168,9 +169,14 @@ class Plan:
         _lib.check(rc, "plan_create")
         self.handle = handle.value
         self._alive = True
+        self._ws_bytes: dict = {}                       # workspace_bytes of the calls made so far
 
     def workspace_bytes(self, op: int, nfields: int, dtype: int, precision: int) -> int:
-        return int(_lib.load().shtb_workspace_bytes(self.handle, op, nfields, dtype, precision))
+        key = (op, nfields, dtype, precision)
+        n = self._ws_bytes.get(key)
+        if n is None:
+            n = self._ws_bytes[key] = int(_lib.load().shtb_workspace_bytes(self.handle, op, nfields, dtype, precision))
+        return n
 
     def table_bytes(self) -> int:
         return int(_lib.load().shtb_plan_table_bytes(self.handle))

@@ -19,6 +19,8 @@ reference's rrules use) is provided by the library's adjoint kernels.
 """
 from __future__ import annotations
 
+import contextlib
+
 import numpy as np
 import torch
 
@@ -63,13 +65,32 @@ def julia_strides(shape) -> tuple:
 def julia_empty(shape, dtype, device) -> torch.Tensor:
     """Uninitialised tensor of ``shape`` with column-major (Julia) memory order."""
     shape = tuple(shape)
-    rev = torch.empty(shape[::-1], dtype=dtype, device=device)
-    return rev.permute(*reversed(range(len(shape))))
+    return torch.empty_strided(shape, julia_strides(shape), dtype=dtype, device=device)
 
 
 def is_julia_dense(t: torch.Tensor) -> bool:
-    exp = julia_strides(t.shape)
-    return all(t.shape[i] == 1 or t.stride(i) == exp[i] for i in range(t.dim()))
+    acc = 1
+    for n, s in zip(t.shape, t.stride()):
+        if n != 1 and s != acc:
+            return False
+        acc *= n
+    return True
+
+
+_cuda_devices: dict = {}
+_no_guard = contextlib.nullcontext()
+
+
+def _cuda_device(index: int) -> torch.device:
+    d = _cuda_devices.get(index)
+    if d is None:
+        d = _cuda_devices[index] = torch.device("cuda", index)
+    return d
+
+
+def _device_guard(index: int):
+    """Context in which ``index`` is the current CUDA device."""
+    return _no_guard if torch.cuda.current_device() == index else torch.cuda.device(index)
 
 
 def _device_index(*vals) -> int:
@@ -83,7 +104,7 @@ def _device_index(*vals) -> int:
 
 def to_device(x, dtype, device_index: int) -> torch.Tensor:
     """Place ``x`` (NumPy array or tensor) on the device, column-major, with ``dtype``."""
-    dev = torch.device("cuda", device_index)
+    dev = _cuda_device(device_index)
     if isinstance(x, np.ndarray):
         x = torch.from_numpy(np.asfortranarray(x))
     if not isinstance(x, torch.Tensor):
@@ -106,18 +127,27 @@ def _ptr(t: torch.Tensor) -> int:
 
 
 def _stream(device_index: int) -> int:
-    return torch.cuda.current_stream(device_index).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device_index)
 
 
 def _workspace(plan, op, nf, dtype_code, prec, device_index) -> tuple[torch.Tensor, int]:
     nb = plan.workspace_bytes(op, nf, dtype_code, prec)
-    ws = torch.empty(max(nb, 256), dtype=torch.uint8, device=torch.device("cuda", device_index))
+    ws = torch.empty(max(nb, 256), dtype=torch.uint8, device=_cuda_device(device_index))
     return ws, nb
 
 
 # ---------------------------------------------------------------------------
-# raw device calls (column-major tensors, batched with a trailing field index)
+# raw device calls (column-major tensors; a trailing field index when batched)
 # ---------------------------------------------------------------------------
+
+def _nfields(t: torch.Tensor) -> int:
+    return t.shape[2] if t.dim() == 3 else 1
+
+
+def _fields_shape(rows: int, cols: int, like: torch.Tensor) -> tuple:
+    """(rows, cols) with the field axis of ``like`` if it has one."""
+    return (rows, cols, like.shape[2]) if like.dim() == 3 else (rows, cols)
+
 
 def _prec_code(precision: str) -> int:
     try:
@@ -143,10 +173,10 @@ def _lcap(cfg: SHTConfig, lcap) -> int:
 def synthesis_device(cfg: SHTConfig, alm: torch.Tensor, f_out: torch.Tensor, ltr: int, prec: int) -> torch.Tensor:
     dev = alm.device.index
     plan = cfg.plan(dev)
-    nf = alm.shape[2]
+    nf = _nfields(alm)
     _, _, dcode = _types(prec)
     ws, nb = _workspace(plan, _lib.SHTB_OP_SYNTHESIS, nf, dcode, prec, dev)
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = _lib.load().shtb_synthesis(plan.handle, _ptr(alm), _ptr(f_out), nf, ltr, dcode, prec, _ptr(ws), nb,
                                         _stream(dev))
     _lib.check(rc, "synthesis")
@@ -156,10 +186,10 @@ def synthesis_device(cfg: SHTConfig, alm: torch.Tensor, f_out: torch.Tensor, ltr
 def analysis_device(cfg: SHTConfig, f: torch.Tensor, alm_out: torch.Tensor, ltr: int, prec: int) -> torch.Tensor:
     dev = f.device.index
     plan = cfg.plan(dev)
-    nf = f.shape[2]
+    nf = _nfields(f)
     _, _, dcode = _types(prec)
     ws, nb = _workspace(plan, _lib.SHTB_OP_ANALYSIS, nf, dcode, prec, dev)
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = _lib.load().shtb_analysis(plan.handle, _ptr(f), _ptr(alm_out), nf, ltr, dcode, prec, _ptr(ws), nb,
                                        _stream(dev))
     _lib.check(rc, "analysis")
@@ -169,9 +199,9 @@ def analysis_device(cfg: SHTConfig, f: torch.Tensor, alm_out: torch.Tensor, ltr:
 def synthesis_sphtor_device(cfg, S, T, Vt, Vp, ltr: int):
     dev = S.device.index
     plan = cfg.plan(dev)
-    nf = S.shape[2]
+    nf = _nfields(S)
     ws, nb = _workspace(plan, _lib.SHTB_OP_SYNTHESIS_SPHTOR, nf, _lib.SHTB_F64, _lib.SHTB_PREC_FP64, dev)
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = _lib.load().shtb_synthesis_sphtor(plan.handle, _ptr(S), _ptr(T), _ptr(Vt), _ptr(Vp), nf, ltr,
                                                _lib.SHTB_F64, _lib.SHTB_PREC_FP64, _ptr(ws), nb, _stream(dev))
     _lib.check(rc, "synthesis_sphtor")
@@ -181,9 +211,9 @@ def synthesis_sphtor_device(cfg, S, T, Vt, Vp, ltr: int):
 def analysis_sphtor_device(cfg, Vt, Vp, S, T, ltr: int):
     dev = Vt.device.index
     plan = cfg.plan(dev)
-    nf = Vt.shape[2]
+    nf = _nfields(Vt)
     ws, nb = _workspace(plan, _lib.SHTB_OP_ANALYSIS_SPHTOR, nf, _lib.SHTB_F64, _lib.SHTB_PREC_FP64, dev)
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = _lib.load().shtb_analysis_sphtor(plan.handle, _ptr(Vt), _ptr(Vp), _ptr(S), _ptr(T), nf, ltr,
                                               _lib.SHTB_F64, _lib.SHTB_PREC_FP64, _ptr(ws), nb, _stream(dev))
     _lib.check(rc, "analysis_sphtor")
@@ -195,7 +225,7 @@ def _adjoint_call(name, op, cfg, ins, outs, nf):
     plan = cfg.plan(dev)
     ws, nb = _workspace(plan, op, nf, _lib.SHTB_F64, _lib.SHTB_PREC_FP64, dev)
     fn = getattr(_lib.load(), name)
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = fn(plan.handle, *[_ptr(t) for t in ins], *[_ptr(t) for t in outs], nf, _ptr(ws), nb, _stream(dev))
     _lib.check(rc, name)
 
@@ -353,7 +383,7 @@ def _cplx_call(name, op, cfg, src, dst, ltr):
     plan = cfg.plan(dev)
     nf = src.shape[2]
     ws, nb = _workspace(plan, op, nf, _lib.SHTB_F64, _lib.SHTB_PREC_FP64, dev)
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = getattr(_lib.load(), name)(plan.handle, _ptr(src), _ptr(dst), nf, ltr, _ptr(ws), nb, _stream(dev))
     _lib.check(rc, name)
     return dst
@@ -393,22 +423,18 @@ def _synthesis_impl(cfg, alm, batched, real_output, use_rfft, fft_scratch, lcap,
     rt, ct, _ = _types(prec)
     dev = _device_index(alm, out)
     a = to_device(a if a.is_complex() else a.to(ct), ct, dev)
-    a3 = a if batched else a.unsqueeze(2)
-    nf = a3.shape[2]
-    if prec == _lib.SHTB_PREC_FP64 and a3.requires_grad and torch.is_grad_enabled() and out is None:
-        f = _Synthesis.apply(a3, cfg, ltr)
-    else:
-        f = out if out is not None else julia_empty((cfg.nlat, cfg.nlon, nf), rt, a3.device)
-        if out is not None and (out.dtype != rt or not is_julia_dense(out) or out.device != a3.device):
-            tmp = julia_empty((cfg.nlat, cfg.nlon, nf), rt, a3.device)
-            synthesis_device(cfg, a3.detach(), tmp, ltr, prec)
-            out.copy_(tmp.reshape(out.shape))
-            return out
-        if out is not None:
-            synthesis_device(cfg, a3.detach(), out.reshape(cfg.nlat, cfg.nlon, nf), ltr, prec)
-            return out
-        synthesis_device(cfg, a3.detach(), f, ltr, prec)
-    return f if batched else f[:, :, 0]
+    if prec == _lib.SHTB_PREC_FP64 and a.requires_grad and torch.is_grad_enabled() and out is None:
+        f = _Synthesis.apply(a if batched else a.unsqueeze(2), cfg, ltr)
+        return f if batched else f[:, :, 0]
+    if out is None or out.dtype != rt or not is_julia_dense(out) or out.device != a.device:
+        f = julia_empty(_fields_shape(cfg.nlat, cfg.nlon, a), rt, a.device)
+        synthesis_device(cfg, a, f, ltr, prec)
+        if out is None:
+            return f
+        out.copy_(f.reshape(out.shape))
+        return out
+    synthesis_device(cfg, a, out.reshape(_fields_shape(cfg.nlat, cfg.nlon, a)), ltr, prec)
+    return out
 
 
 def _analysis_impl(cfg, f, batched, use_rfft, fft_scratch, lcap, precision, out=None):
@@ -436,17 +462,15 @@ def _analysis_impl(cfg, f, batched, use_rfft, fft_scratch, lcap, precision, out=
     rt, ct, _ = _types(prec)
     dev = _device_index(f, out)
     t = to_device(t, rt, dev)
-    t3 = t if batched else t.unsqueeze(2)
-    nf = t3.shape[2]
-    if prec == _lib.SHTB_PREC_FP64 and t3.requires_grad and torch.is_grad_enabled() and out is None:
-        a = _Analysis.apply(t3, cfg, ltr)
-    else:
-        a = julia_empty((cfg.lmax + 1, cfg.mmax + 1, nf), ct, t3.device)
-        analysis_device(cfg, t3.detach(), a, ltr, prec)
-        if out is not None:
-            out.copy_(a.reshape(out.shape))
-            return out
-    return a if batched else a[:, :, 0]
+    if prec == _lib.SHTB_PREC_FP64 and t.requires_grad and torch.is_grad_enabled() and out is None:
+        a = _Analysis.apply(t if batched else t.unsqueeze(2), cfg, ltr)
+        return a if batched else a[:, :, 0]
+    a = julia_empty(_fields_shape(cfg.lmax + 1, cfg.mmax + 1, t), ct, t.device)
+    analysis_device(cfg, t, a, ltr, prec)
+    if out is not None:
+        out.copy_(a.reshape(out.shape))
+        return out
+    return a
 
 
 def synthesis(cfg: SHTConfig, alm, *, real_output: bool = True, use_rfft: bool = False, fft_scratch=None,
@@ -499,16 +523,14 @@ def _sphtor_synth(cfg, S, T, batched, real_output, use_rfft, lcap):
     dev = _device_index(S, T)
     s = to_device(s if s.is_complex() else s.to(torch.complex128), torch.complex128, dev)
     t = to_device(t if t.is_complex() else t.to(torch.complex128), torch.complex128, dev)
-    s3 = s if batched else s.unsqueeze(2)
-    t3 = t if batched else t.unsqueeze(2)
-    if (s3.requires_grad or t3.requires_grad) and torch.is_grad_enabled():
-        vt, vp = _SynthesisSphtor.apply(s3, t3, cfg, ltr)
-    else:
-        nf = s3.shape[2]
-        vt = julia_empty((cfg.nlat, cfg.nlon, nf), torch.float64, s3.device)
-        vp = julia_empty((cfg.nlat, cfg.nlon, nf), torch.float64, s3.device)
-        synthesis_sphtor_device(cfg, s3.detach(), t3.detach(), vt, vp, ltr)
-    return (vt, vp) if batched else (vt[:, :, 0], vp[:, :, 0])
+    if (s.requires_grad or t.requires_grad) and torch.is_grad_enabled():
+        vt, vp = _SynthesisSphtor.apply(s if batched else s.unsqueeze(2), t if batched else t.unsqueeze(2), cfg, ltr)
+        return (vt, vp) if batched else (vt[:, :, 0], vp[:, :, 0])
+    shape = _fields_shape(cfg.nlat, cfg.nlon, s)
+    vt = julia_empty(shape, torch.float64, s.device)
+    vp = julia_empty(shape, torch.float64, s.device)
+    synthesis_sphtor_device(cfg, s, t, vt, vp, ltr)
+    return vt, vp
 
 
 def _sphtor_anal(cfg, Vt, Vp, batched, use_rfft, lcap):
@@ -524,16 +546,14 @@ def _sphtor_anal(cfg, Vt, Vp, batched, use_rfft, lcap):
     dev = _device_index(Vt, Vp)
     a = to_device(a, torch.float64, dev)
     b = to_device(b, torch.float64, dev)
-    a3 = a if batched else a.unsqueeze(2)
-    b3 = b if batched else b.unsqueeze(2)
-    if (a3.requires_grad or b3.requires_grad) and torch.is_grad_enabled():
-        S, T = _AnalysisSphtor.apply(a3, b3, cfg, ltr)
-    else:
-        nf = a3.shape[2]
-        S = julia_empty((cfg.lmax + 1, cfg.mmax + 1, nf), torch.complex128, a3.device)
-        T = julia_empty((cfg.lmax + 1, cfg.mmax + 1, nf), torch.complex128, a3.device)
-        analysis_sphtor_device(cfg, a3.detach(), b3.detach(), S, T, ltr)
-    return (S, T) if batched else (S[:, :, 0], T[:, :, 0])
+    if (a.requires_grad or b.requires_grad) and torch.is_grad_enabled():
+        S, T = _AnalysisSphtor.apply(a if batched else a.unsqueeze(2), b if batched else b.unsqueeze(2), cfg, ltr)
+        return (S, T) if batched else (S[:, :, 0], T[:, :, 0])
+    shape = _fields_shape(cfg.lmax + 1, cfg.mmax + 1, a)
+    S = julia_empty(shape, torch.complex128, a.device)
+    T = julia_empty(shape, torch.complex128, a.device)
+    analysis_sphtor_device(cfg, a, b, S, T, ltr)
+    return S, T
 
 
 def synthesis_sphtor(cfg: SHTConfig, Slm, Tlm, *, real_output: bool = True, use_rfft: bool = False,
@@ -623,17 +643,16 @@ def _packed_synth(cfg, Qlm, batched, lcap, precision):
     rt, ct, dcode = _types(prec)
     dev = _device_index(Qlm)
     q = to_device(q if q.is_complex() else q.to(ct), ct, dev)
-    q2 = q if batched else q.unsqueeze(1)
-    nf = q2.shape[1]
-    f = julia_empty((cfg.nlat, cfg.nlon, nf), rt, q2.device)
+    nf = q.shape[1] if batched else 1
+    # vec(f) per field: the column-major grid itself
+    f = julia_empty((cfg.nlat * cfg.nlon, nf) if batched else (cfg.nlat * cfg.nlon,), rt, q.device)
     plan = cfg.plan(dev)
     ws, nb = _workspace(plan, _lib.SHTB_OP_SYNTHESIS, nf, dcode, prec, dev)
-    with torch.cuda.device(dev):
-        rc = _lib.load().shtb_synthesis_packed(plan.handle, _ptr(q2), _ptr(f), nf, ltr, dcode, prec, _ptr(ws), nb,
+    with _device_guard(dev):
+        rc = _lib.load().shtb_synthesis_packed(plan.handle, _ptr(q), _ptr(f), nf, ltr, dcode, prec, _ptr(ws), nb,
                                                _stream(dev))
     _lib.check(rc, "synthesis_packed")
-    flat = f.permute(2, 1, 0).reshape(nf, cfg.nlat * cfg.nlon).permute(1, 0)   # vec(f) per field
-    return flat if batched else flat[:, 0]
+    return f
 
 
 def _packed_anal(cfg, Vr, batched, lcap, precision):
@@ -644,22 +663,16 @@ def _packed_anal(cfg, Vr, batched, lcap, precision):
     prec = _prec_code(precision)
     rt, ct, dcode = _types(prec)
     dev = _device_index(Vr)
-    v = to_device(v, rt, dev)
-    v2 = v if batched else v.unsqueeze(1)
-    nf = v2.shape[1]
-    grid = v2.permute(1, 0).reshape(nf, cfg.nlon, cfg.nlat).permute(2, 1, 0)   # (nlat, nlon, nf), column-major
-    if not is_julia_dense(grid):
-        g = julia_empty((cfg.nlat, cfg.nlon, nf), rt, v2.device)
-        g.copy_(grid)
-        grid = g
-    q = julia_empty((cfg.nlm, nf), ct, v2.device)
+    v = to_device(v, rt, dev)   # column-major: the grids themselves
+    nf = v.shape[1] if batched else 1
+    q = julia_empty((cfg.nlm, nf) if batched else (cfg.nlm,), ct, v.device)
     plan = cfg.plan(dev)
     ws, nb = _workspace(plan, _lib.SHTB_OP_ANALYSIS, nf, dcode, prec, dev)
-    with torch.cuda.device(dev):
-        rc = _lib.load().shtb_analysis_packed(plan.handle, _ptr(grid), _ptr(q), nf, ltr, dcode, prec, _ptr(ws), nb,
+    with _device_guard(dev):
+        rc = _lib.load().shtb_analysis_packed(plan.handle, _ptr(v), _ptr(q), nf, ltr, dcode, prec, _ptr(ws), nb,
                                               _stream(dev))
     _lib.check(rc, "analysis_packed")
-    return q if batched else q[:, 0]
+    return q
 
 
 def synthesis_packed(cfg: SHTConfig, Qlm, *, precision: str = "fp64"):
@@ -719,7 +732,7 @@ def _spectral_op(name, op, cfg, src, out):
     nf = a.shape[2] if a.dim() == 3 else 1
     plan = cfg.plan(dev)
     dcode = _lib.SHTB_F64 if a.dtype == torch.complex128 else _lib.SHTB_F32
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         rc = _lib.load().shtb_spectral_op(plan.handle, op, _ptr(a), _ptr(o), nf, dcode, _stream(dev))
     _lib.check(rc, name)
     return o
@@ -784,18 +797,17 @@ def _divvort_synth(cfg, D, Z, batched, lcap):
     dev = _device_index(D, Z)
     d = to_device(d if d.is_complex() else d.to(torch.complex128), torch.complex128, dev)
     z = to_device(z if z.is_complex() else z.to(torch.complex128), torch.complex128, dev)
-    d3 = d if batched else d.unsqueeze(2)
-    z3 = z if batched else z.unsqueeze(2)
-    nf = d3.shape[2]
-    vt = julia_empty((cfg.nlat, cfg.nlon, nf), torch.float64, d3.device)
-    vp = julia_empty((cfg.nlat, cfg.nlon, nf), torch.float64, d3.device)
+    nf = _nfields(d)
+    shape = _fields_shape(cfg.nlat, cfg.nlon, d)
+    vt = julia_empty(shape, torch.float64, d.device)
+    vp = julia_empty(shape, torch.float64, d.device)
     plan = cfg.plan(dev)
     ws, nb = _workspace(plan, _lib.SHTB_OP_SYNTHESIS_SPHTOR, nf, _lib.SHTB_F64, _lib.SHTB_PREC_FP64, dev)
-    with torch.cuda.device(dev):
-        rc = _lib.load().shtb_synthesis_divvort(plan.handle, _ptr(d3), _ptr(z3), _ptr(vt), _ptr(vp), nf, ltr,
+    with _device_guard(dev):
+        rc = _lib.load().shtb_synthesis_divvort(plan.handle, _ptr(d), _ptr(z), _ptr(vt), _ptr(vp), nf, ltr,
                                                 _lib.SHTB_F64, _lib.SHTB_PREC_FP64, _ptr(ws), nb, _stream(dev))
     _lib.check(rc, "synthesis_divvort")
-    return (vt, vp) if batched else (vt[:, :, 0], vp[:, :, 0])
+    return vt, vp
 
 
 def _divvort_anal(cfg, Vt, Vp, batched, lcap):
@@ -805,20 +817,19 @@ def _divvort_anal(cfg, Vt, Vp, batched, lcap):
             raise DimensionMismatch(f"{nm} dims")
     ltr = _lcap(cfg, lcap)
     dev = _device_index(Vt, Vp)
-    a3 = to_device(a, torch.float64, dev)
-    b3 = to_device(b, torch.float64, dev)
-    a3 = a3 if batched else a3.unsqueeze(2)
-    b3 = b3 if batched else b3.unsqueeze(2)
-    nf = a3.shape[2]
-    D = julia_empty((cfg.lmax + 1, cfg.mmax + 1, nf), torch.complex128, a3.device)
-    Z = julia_empty((cfg.lmax + 1, cfg.mmax + 1, nf), torch.complex128, a3.device)
+    a = to_device(a, torch.float64, dev)
+    b = to_device(b, torch.float64, dev)
+    nf = _nfields(a)
+    shape = _fields_shape(cfg.lmax + 1, cfg.mmax + 1, a)
+    D = julia_empty(shape, torch.complex128, a.device)
+    Z = julia_empty(shape, torch.complex128, a.device)
     plan = cfg.plan(dev)
     ws, nb = _workspace(plan, _lib.SHTB_OP_ANALYSIS_SPHTOR, nf, _lib.SHTB_F64, _lib.SHTB_PREC_FP64, dev)
-    with torch.cuda.device(dev):
-        rc = _lib.load().shtb_analysis_divvort(plan.handle, _ptr(a3), _ptr(b3), _ptr(D), _ptr(Z), nf, ltr,
+    with _device_guard(dev):
+        rc = _lib.load().shtb_analysis_divvort(plan.handle, _ptr(a), _ptr(b), _ptr(D), _ptr(Z), nf, ltr,
                                                _lib.SHTB_F64, _lib.SHTB_PREC_FP64, _ptr(ws), nb, _stream(dev))
     _lib.check(rc, "analysis_divvort")
-    return (D, Z) if batched else (D[:, :, 0], Z[:, :, 0])
+    return D, Z
 
 
 def synthesis_divvort(cfg: SHTConfig, div, vort, *, lcap: int | None = None):
