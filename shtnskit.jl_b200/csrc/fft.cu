@@ -607,8 +607,8 @@ int launch_fft_ana(const shtb_plan* p, const GT* in0, const GT* in1, int ncomp, 
                    double wscale, int use_w, int spow, cudaStream_t st, int wtile) {
   static_assert(std::is_same<T, GT>::value, "grid and compute types match");
   if constexpr (std::is_same<T, float>::value) {
-    if (ncomp == 1 && use_w && !spow && wtile && fft2_applicable(p))
-      return launch_fft2_ana(p, (const float*)in0, W, nfw, mlim, wscale, st);
+    if (ncomp == 1 && use_w && !spow && fft2_applicable(p))
+      return launch_fft2_ana(p, (const float*)in0, W, nfw, mlim, wscale, wtile, st);
   }
   switch (fft_pick_h(p->fft, sizeof(typename V2<T>::type), p->npair)) {
     case 16: return launch_ana_h<T, 16>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, st);
@@ -759,7 +759,7 @@ void fft_fill_job_f32(const shtb_plan* p, int syn, const void* W, void* grid, in
   FFTJob<float> J = syn ? fft_job<float>(p, p->d_rinv, (const float2*)W, nullptr, (float*)grid, nullptr, 1, mlim,
                                          p->phi_inv_scale / p->nlon, 0, 0)
                         : fft_job<float>(p, p->d_rev, nullptr, (float2*)const_cast<void*>(W), (float*)grid, nullptr, 1,
-                                         mlim, p->ana_scale, 1, 0, 1, nf);
+                                         mlim, p->ana_scale, 1, 0, simt_applicable(p, nf) ? 0 : 1, nf);
   std::memcpy(host_job, &J, sizeof(J));
 }
 

@@ -219,7 +219,8 @@ struct Job {
   const int* perm;          // rev (analysis) or rinv (synthesis)
   const float2* tw;         // per-pass twiddles (c, s), layout of FFTDesc::twoff
   const float2* Win;        // synthesis: Fourier buffer
-  float* Wout;              // analysis: B tile images of the mixed analysis GEMM
+  float* Wout;              // analysis: B tile images of the mixed analysis GEMM (wtile), or the
+  int wtile;                //   Fourier buffer [field][order][E|O][pair]
   float* grid;
   int nf, mlim;
   double scale;             // synthesis: grid factor; analysis: weight factor
@@ -321,6 +322,15 @@ __device__ __forceinline__ void ana_body(const Job& J, int k, int p0, float4* X,
     const u64 hw = pk(make_float2(0.5f * wfac[2 * hp], 0.5f * wfac[2 * hp + 1]));
     const u64 Ere = mul2(hw, add2(sre, dim)), Eim = mul2(hw, sub2(sim, dre));
     const u64 Ore = mul2(hw, sub2(sre, dim)), Oim = mul2(hw, add2(sim, dre));
+    if (!J.wtile) {   // two adjacent pairs of one order: 16 bytes of the Fourier buffer
+      if (valid && pa < npair) {
+        const float2 er = up(Ere), ei = up(Eim), qr = up(Ore), qi = up(Oim);
+        float4* w = reinterpret_cast<float4*>(J.Wout + 2 * (((size_t)k * P.nm + im) * 2 * npair + pa));
+        w[0] = make_float4(er.x, ei.x, er.y, ei.y);
+        w[npair / 2] = make_float4(qr.x, qi.x, qr.y, qi.y);
+      }
+      continue;
+    }
     // the even lane keeps its real parts and takes its partner's; the odd lane the reverse
     const u64 eo = __shfl_xor_sync(0xffffffffu, odd ? Ere : Eim, 1);
     const u64 oo = __shfl_xor_sync(0xffffffffu, odd ? Ore : Oim, 1);
@@ -332,7 +342,7 @@ __device__ __forceinline__ void ana_body(const Job& J, int k, int p0, float4* X,
     *reinterpret_cast<float4*>(J.Wout + f2_btile_base(im, 0, pe, k, npair, J.nf) + off) = make_float4(e0.x, e0.y, e1.x, e1.y);
     *reinterpret_cast<float4*>(J.Wout + f2_btile_base(im, 1, pe, k, npair, J.nf) + off) = make_float4(o0.x, o0.y, o1.x, o1.y);
   }
-  if (p0 <= npair - 1 && npair - 1 < p0 + 2 * HP) {
+  if (J.wtile && p0 <= npair - 1 && npair - 1 < p0 + 2 * HP) {
     // the CTA holding the last pair also zeroes the padding pairs npair .. npair8-1
     const int pad = ((npair + 7) & ~7) - npair;
     for (int idx = threadIdx.x; idx < nmu * pad; idx += blockDim.x) {
@@ -517,6 +527,7 @@ static f2::Job fft2_job(const shtb_plan* p, const int* perm, double scale, int n
   J.tw = p->d_twp32;
   J.Win = nullptr;
   J.Wout = nullptr;
+  J.wtile = 0;
   J.grid = nullptr;
   J.nf = nf;
   J.mlim = mlim;
@@ -529,7 +540,8 @@ static f2::Job fft2_job(const shtb_plan* p, const int* perm, double scale, int n
 // at nlon 2048, 64 fields).
 constexpr int kFft2HP = 4;
 
-int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int mlim, double wscale, cudaStream_t st) {
+int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int mlim, double wscale, int wtile,
+                    cudaStream_t st) {
   constexpr int HP = kFft2HP;
   const size_t smem = (size_t)f2::smem_elems_ana<HP>(p->fft.n) * 16;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(f2::ana_kernel<HP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -537,6 +549,7 @@ int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int 
   f2::Job J = fft2_job(p, p->d_rev, wscale, nf, mlim);
   J.grid = const_cast<float*>(grid);
   J.Wout = (float*)W;
+  J.wtile = wtile;
   // blockIdx.x = field, blockIdx.y = block of 2 HP pairs: the fields' CTAs that fill one B
   // tile region run together
   dim3 grd(nf, (p->npair + 2 * HP - 1) / (2 * HP));
@@ -561,7 +574,7 @@ void fft2_fill_job(const shtb_plan* p, int syn, const void* W, void* grid, int n
   if (syn)
     J.Win = (const float2*)W;
   else
-    J.Wout = (float*)const_cast<void*>(W);
+    J.Wout = (float*)const_cast<void*>(W), J.wtile = simt_applicable(p, nf) ? 0 : 1;
   std::memcpy(host_job, &J, sizeof(J));
 }
 

@@ -1,26 +1,26 @@
 // group.cu — uneven batches: many independent mixed-precision scalar transforms, each
 // with its own plan (lmax, Gauss grid, nlon) and 1..8 fields, run as persistent stage
 // launches: B packing and order-GEMM synthesis for members with three or more fields, the
-// FP64-pipe synthesis (simt.cu) for members with one or two, FFT synthesis, FFT analysis and
-// order-GEMM analysis.
+// FP64-pipe synthesis (simt.cu) for members with one or two, FFT synthesis, FFT analysis, and
+// the order-GEMM or FP64-pipe analysis.
 //
 // Every stage owns a list of work items over all members — GEMM tiles (member, order,
 // first latitude pair or degree, parity, with the tile's live-chunk mask: chunks whose P
 // image is all zero are skipped), FP64-pipe items (member, order, block of 32 latitude
-// pairs, one per warp) and FFT tiles (member, first latitude pair, field) — sorted by
+// pairs or segment of degrees, one per warp) and FFT tiles (member, first latitude pair, field) — sorted by
 // decreasing cost, and a device work counter (zeroed by a memset at the start of every
 // roundtrip). A stage launches min(items, SMs x CTAs per SM) persistent CTAs; each claims
 // the next item with an atomicAdd on the counter whenever it has room for one, so the
 // longest tiles start first and the short ones fill in behind whichever CTA frees up first,
 // and a batch of mixed sizes keeps every SM busy without one launch per member. Members
 // whose FFTs the packed-pair kernels take (fft2_applicable) run them in a second persistent
-// FFT kernel per direction, forked beside the general one, and the FP64-pipe synthesis is
-// forked beside the packing and GEMM synthesis, so every member's results equal its
-// single-plan calls bit for bit. The memset and the launches of a roundtrip (a start marker
-// plus the stages) are captured once into a CUDA graph and replayed.
+// FFT kernel per direction, forked beside the general one, and the FP64-pipe synthesis
+// and analysis are forked beside the packing and GEMMs, so every member's results equal its
+// single-plan calls bit for bit. The memset and the launches of a roundtrip are captured once
+// into a CUDA graph and replayed.
 //
-// Per-member latency: the start marker records %globaltimer; the analysis GEMM stores,
-// per member, the time its last tile finished.
+// Per-member latency: the first synthesis kernels record %globaltimer as they start; the
+// analysis kernels store, per member, the time its last tile or item finished.
 //
 // Launch-shape autotuning times, on the bound buffers, every FFT shape (latitude pairs per
 // CTA; 1, 2 or 4 CTAs per SM, the extra CTAs queueing behind the resident ones), then one
@@ -34,19 +34,11 @@
 
 namespace shtb {
 
-__global__ void group_start_kernel(unsigned long long* done, int n, unsigned long long* t0) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) done[i] = 0;
-  if (threadIdx.x == 0) {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    *t0 = t;
-  }
-}
-
 static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
-// work counters: pack, GEMM syn, FFT syn, FFT ana, GEMM ana, fft2 syn, fft2 ana, FP64-pipe syn
-constexpr int kGroupQueues = 8;
+// work counters: pack, GEMM syn, FFT syn, FFT ana, GEMM ana, fft2 syn, fft2 ana, FP64-pipe syn,
+// FP64-pipe ana
+constexpr int kGroupQueues = 9;
 
 }  // namespace shtb
 
@@ -60,9 +52,9 @@ struct shtb_group {
   std::vector<char> f2;                 // member runs the packed-pair FFTs (fft2_applicable)
   std::vector<char> simt;               // member's Legendre synthesis runs on the FP64 pipes (simt_applicable)
   size_t sargsz = 0;
-  unsigned char* d_sargs = nullptr;
-  int4* d_items_ssyn = nullptr;
-  int n_ssyn = 0, ssyn_ctas = 148;
+  unsigned char *d_sargs = nullptr, *d_sargs_ana = nullptr;
+  int4 *d_items_ssyn = nullptr, *d_items_sana = nullptr;
+  int n_ssyn = 0, ssyn_ctas = 148, n_sana = 0, sana_ctas = 148;
   size_t ssyn_smem = 0;
   size_t argsz = 0, jobsz = 0, job2sz = 0;
   // device memory: [args syn | args ana | jobs syn | jobs ana | done | t0 | gemm items | W]
@@ -189,11 +181,31 @@ static int group_synthesis_stage(shtb_group* g, int* q, cudaStream_t st) {
     SHTB_TRY_CUDA(cudaStreamWaitEvent(g->aux, g->ev_fork, 0), "group fork");
   }
   if ((rc = launch_simt_group(g->d_sargs, g->d_items_ssyn, g->n_ssyn, g->ssyn_ctas, g->ssyn_smem, q + 7,
-                              fork ? g->aux : st)))
+                              g->d_t0, fork ? g->aux : st)))
     return rc;
-  if ((rc = launch_pack_group(g->d_args_syn, g->d_items_pack, g->n_pack, std::min(g->n_pack, 24 * g->nsm), q, st)))
+  if ((rc = launch_pack_group(g->d_args_syn, g->d_items_pack, g->n_pack, std::min(g->n_pack, 24 * g->nsm), q, g->d_t0, st)))
     return rc;
   if ((rc = launch_gemm_group(0, g->d_args_syn, g->d_items_syn, g->d_masks_syn, g->n_syn, g->gemm_ctas_syn, nullptr, q + 1, st)))
+    return rc;
+  if (fork) {
+    SHTB_TRY_CUDA(cudaEventRecord(g->ev_join, g->aux), "group join");
+    SHTB_TRY_CUDA(cudaStreamWaitEvent(st, g->ev_join, 0), "group join");
+  }
+  return SHTB_OK;
+}
+
+// The Legendre analysis stage, forked the same way.
+static int group_analysis_stage(shtb_group* g, int* q, cudaStream_t st) {
+  int rc;
+  const bool fork = g->n_sana > 0 && g->n_ana > 0;
+  if (fork) {
+    SHTB_TRY_CUDA(cudaEventRecord(g->ev_fork, st), "group fork");
+    SHTB_TRY_CUDA(cudaStreamWaitEvent(g->aux, g->ev_fork, 0), "group fork");
+  }
+  if ((rc = launch_simt_ana_group(g->d_sargs_ana, g->d_items_sana, g->n_sana, g->sana_ctas, q + 8, g->d_done,
+                                  fork ? g->aux : st)))
+    return rc;
+  if ((rc = launch_gemm_group(1, g->d_args_ana, g->d_items_ana, g->d_masks_ana, g->n_ana, g->gemm_ctas_ana, g->d_done, q + 4, st)))
     return rc;
   if (fork) {
     SHTB_TRY_CUDA(cudaEventRecord(g->ev_join, g->aux), "group join");
@@ -205,18 +217,16 @@ static int group_synthesis_stage(shtb_group* g, int* q, cudaStream_t st) {
 static int group_launch_stages(shtb_group* g, int op, cudaStream_t st) {
   int rc;
   int* q = g->d_queue;
-  SHTB_TRY_CUDA(cudaMemsetAsync(q, 0, kGroupQueues * sizeof(int), st), "group work counters");
+  // the work counters, and with a synthesis the completion times and the start time before them
+  char* z0 = (char*)(op != SHTB_OP_ANALYSIS ? (void*)g->d_done : (void*)q);
+  SHTB_TRY_CUDA(cudaMemsetAsync(z0, 0, (char*)(q + kGroupQueues) - z0, st), "group work counters");
   if (op != SHTB_OP_ANALYSIS) {
-    group_start_kernel<<<1, 256, 0, st>>>(g->d_done, g->n, g->d_t0);
-    count_launch();
-    SHTB_TRY_CUDA(cudaGetLastError(), "group start marker");
     if ((rc = group_synthesis_stage(g, q, st))) return rc;
     if ((rc = group_fft_stage(g, 1, q + 2, q + 5, st))) return rc;
   }
   if (op != SHTB_OP_SYNTHESIS) {
     if ((rc = group_fft_stage(g, 0, q + 3, q + 6, st))) return rc;
-    if ((rc = launch_gemm_group(1, g->d_args_ana, g->d_items_ana, g->d_masks_ana, g->n_ana, g->gemm_ctas_ana, g->d_done, q + 4, st)))
-      return rc;
+    if ((rc = group_analysis_stage(g, q, st))) return rc;
   }
   return SHTB_OK;
 }
@@ -257,7 +267,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   g->simt.resize(n);
   for (int t = 0; t < n; ++t) {
     g->simt[t] = simt_applicable(plans[t], nfields[t]) ? 1 : 0;
-    int rc = mixed_prepare(plans[t], 0);   // the analysis GEMM reads the plan's P table
+    int rc = g->simt[t] ? SHTB_OK : mixed_prepare(plans[t], 0);   // the GEMMs read the plan's P table
     if (rc) return fail(rc);
     g->f2[t] = fft2_applicable(plans[t]) ? 1 : 0;
     if (!g->f2[t]) g->generic = g->generic || fft_plan_generic(plans[t]);
@@ -291,8 +301,8 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   std::vector<unsigned long long> msyn, mana;
   std::vector<int> csyn, cana;
   // FP64-pipe synthesis items of the one- and two-field members, most work first
-  std::vector<int4> ssyn;
-  std::vector<int> cssyn;
+  std::vector<int4> ssyn, sana;
+  std::vector<int> cssyn, csana;
   for (int t = 0; t < n; ++t) {
     if (!g->simt[t]) continue;
     const shtb_plan* p = plans[t];
@@ -302,6 +312,12 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
       for (int pb = 0; pb < simt_syn_pair_blocks(p); ++pb) {
         ssyn.push_back(make_int4(t, im, pb, 0));
         cssyn.push_back(p->lmax - im + 1);
+      }
+    const int sg = simt_ana_segment(nfields[t]);
+    for (int im = 0; im <= mlim; ++im)
+      for (int s = 0; im + s * sg <= p->lmax; ++s) {
+        sana.push_back(make_int4(t, im, s, 0));
+        csana.push_back(p->npair * sg * (2 + 2 * nfields[t]));
       }
   }
   for (int t = 0; t < n; ++t) {
@@ -316,7 +332,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
           csyn.push_back(c);
         }
         const int JE = (p->lmax - im) / 2 + 1;
-        for (int j0 = 0; j0 < JE; j0 += TM) {
+        for (int j0 = 0; !g->simt[t] && j0 < JE; j0 += TM) {
           int c = 0;
           mana.push_back(mixed_group_tile(p, 1, im, j0, par, &c));
           ana.push_back(make_int4(t, im, j0, par));
@@ -349,6 +365,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   sort_masked(syn, msyn, csyn);
   sort_masked(ana, mana, cana);
   sort_items(ssyn, cssyn);
+  sort_items(sana, csana);
   std::vector<int2> pack;   // (member, order) for the synthesis B packing, most degrees first
   {
     std::vector<int4> tmp;
@@ -369,6 +386,8 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   g->gemm_ctas_ana = std::max(1, std::min(2 * g->nsm, g->n_ana));
   g->n_ssyn = (int)ssyn.size();
   g->ssyn_ctas = std::max(1, std::min(8 * g->nsm, g->n_ssyn));   // 128-thread CTAs, several per SM
+  g->n_sana = (int)sana.size();
+  g->sana_ctas = std::max(1, std::min(2 * g->nsm, g->n_sana));   // 128-thread CTAs, two per SM
   g->sargsz = simt_args_bytes();
   // one device allocation
   g->argsz = mixed_args_bytes();
@@ -384,6 +403,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
                o_ia = take(ana.size() * sizeof(int4)), o_ip = take(pack.size() * sizeof(int2)),
                o_ms = take(msyn.size() * 8), o_ma = take(mana.size() * 8);
   const size_t o_sas = take(n * g->sargsz), o_iss = take(ssyn.size() * sizeof(int4));
+  const size_t o_saa = take(n * g->sargsz), o_isa = take(sana.size() * sizeof(int4));
   g->woff.resize(n);
   size_t wbytes = 0;
   for (int t = 0; t < n; ++t) {
@@ -411,6 +431,8 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   g->d_items_pack = (int2*)(g->dmem + o_ip);
   g->d_sargs = g->dmem + o_sas;
   g->d_items_ssyn = (int4*)(g->dmem + o_iss);
+  g->d_sargs_ana = g->dmem + o_saa;
+  g->d_items_sana = (int4*)(g->dmem + o_isa);
   g->d_w = g->dmem + o_w;
   e = cudaMemcpy(g->d_items_syn, syn.data(), syn.size() * sizeof(int4), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(g->d_items_ana, ana.data(), ana.size() * sizeof(int4), cudaMemcpyHostToDevice);
@@ -418,9 +440,10 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   if (e == cudaSuccess && !mana.empty()) e = cudaMemcpy(g->d_masks_ana, mana.data(), mana.size() * 8, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(g->d_items_pack, pack.data(), pack.size() * sizeof(int2), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(g->d_items_ssyn, ssyn.data(), ssyn.size() * sizeof(int4), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !sana.empty()) e = cudaMemcpy(g->d_items_sana, sana.data(), sana.size() * sizeof(int4), cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !f2items.empty())
     e = cudaMemcpy(g->d_items_fft2, f2items.data(), f2items.size() * sizeof(int4), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(g->d_done, 0, n * 8);
+  if (e == cudaSuccess) e = cudaMemset(g->d_done, 0, (char*)(g->d_queue + kGroupQueues) - (char*)g->d_done);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->priv, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->aux, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ev_in, cudaEventDisableTiming);
@@ -449,7 +472,7 @@ extern "C" int shtb_group_bind(shtb_group* g, void* const* alm_in, void* const* 
   int rc = check_device(g);
   if (rc) return rc;
   std::vector<unsigned char> as(g->n * g->argsz), aa(g->n * g->argsz), js(g->n * g->jobsz), ja(g->n * g->jobsz),
-      j2s(g->n * g->job2sz), j2a(g->n * g->job2sz), sas(g->n * g->sargsz);
+      j2s(g->n * g->job2sz), j2a(g->n * g->job2sz), sas(g->n * g->sargsz), saa(g->n * g->sargsz);
   for (int t = 0; t < g->n; ++t) {
     if (!alm_in[t] || !grid[t] || !alm_out[t])
       return set_error(SHTB_ERR_BAD_ARG, "NULL buffer for member " + std::to_string(t));
@@ -465,7 +488,10 @@ extern "C" int shtb_group_bind(shtb_group* g, void* const* alm_in, void* const* 
       fft2_fill_job(p, 1, W, grid[t], g->nf[t], j2s.data() + t * g->job2sz);
       fft2_fill_job(p, 0, W, grid[t], g->nf[t], j2a.data() + t * g->job2sz);
     }
-    if (g->simt[t]) simt_fill_args(p, alm_in[t], W, g->nf[t], sas.data() + t * g->sargsz);
+    if (g->simt[t]) {
+      simt_fill_args(p, 1, alm_in[t], W, g->nf[t], sas.data() + t * g->sargsz);
+      simt_fill_args(p, 0, W, alm_out[t], g->nf[t], saa.data() + t * g->sargsz);
+    }
   }
   SHTB_TRY_CUDA(cudaMemcpy(g->d_args_syn, as.data(), as.size(), cudaMemcpyHostToDevice), "group bind");
   SHTB_TRY_CUDA(cudaMemcpy(g->d_args_ana, aa.data(), aa.size(), cudaMemcpyHostToDevice), "group bind");
@@ -474,6 +500,7 @@ extern "C" int shtb_group_bind(shtb_group* g, void* const* alm_in, void* const* 
   SHTB_TRY_CUDA(cudaMemcpy(g->d_jobs2_syn, j2s.data(), j2s.size(), cudaMemcpyHostToDevice), "group bind");
   SHTB_TRY_CUDA(cudaMemcpy(g->d_jobs2_ana, j2a.data(), j2a.size(), cudaMemcpyHostToDevice), "group bind");
   SHTB_TRY_CUDA(cudaMemcpy(g->d_sargs, sas.data(), sas.size(), cudaMemcpyHostToDevice), "group bind");
+  SHTB_TRY_CUDA(cudaMemcpy(g->d_sargs_ana, saa.data(), saa.size(), cudaMemcpyHostToDevice), "group bind");
   g->bound = true;
   drop_graph(g);
   return SHTB_OK;
@@ -517,7 +544,7 @@ extern "C" int shtb_group_roundtrip(shtb_group* g, void* stream) {
   SHTB_TRY_CUDA(cudaEventRecord(g->ev_in, st), "group event");
   SHTB_TRY_CUDA(cudaStreamWaitEvent(g->priv, g->ev_in, 0), "group wait");
   SHTB_TRY_CUDA(cudaGraphLaunch(g->exec, g->priv), "group graph launch");
-  count_launch(g->graph_kernels);   // start marker, B packing, GEMMs and the FFT kernels
+  count_launch(g->graph_kernels);   // B packing, GEMMs, FP64-pipe and FFT kernels
   SHTB_TRY_CUDA(cudaEventRecord(g->ev_out, g->priv), "group event");
   SHTB_TRY_CUDA(cudaStreamWaitEvent(st, g->ev_out, 0), "group wait");
   return SHTB_OK;
@@ -613,6 +640,7 @@ extern "C" int shtb_group_latency_ns(const shtb_group* g, uint64_t* ns) {
   unsigned long long t0 = 0;
   SHTB_TRY_CUDA(cudaMemcpy(done.data(), g->d_done, g->n * 8, cudaMemcpyDeviceToHost), "group latency read");
   SHTB_TRY_CUDA(cudaMemcpy(&t0, g->d_t0, 8, cudaMemcpyDeviceToHost), "group latency read");
+  t0 = ~t0;   // kept as the complement
   for (int t = 0; t < g->n; ++t) ns[t] = done[t] > t0 ? (uint64_t)(done[t] - t0) : 0;
   return SHTB_OK;
 }

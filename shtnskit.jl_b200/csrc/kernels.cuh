@@ -67,7 +67,8 @@ int launch_zero_columns64(const shtb_plan* p, double2* a, int nf, int mlim, cuda
 // FP32 FFTs on packed pairs of latitude pairs (fft2.cu) for power-of-two nlon <= 2048 and
 // nlat a multiple of 4: the mixed path's analysis into B tile images, and its synthesis.
 bool fft2_applicable(const shtb_plan* p);
-int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int mlim, double wscale, cudaStream_t st);
+int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int mlim, double wscale, int wtile,
+                    cudaStream_t st);
 int launch_fft2_syn(const shtb_plan* p, const void* W, float* grid, int nf, int mlim, double gscale, cudaStream_t st);
 
 // Floats of one analysis B tile image of the mixed path (hi and lo images back to back).
@@ -76,6 +77,18 @@ size_t fft_btile_floats(const shtb_plan* p, int nf);
 size_t mixed_workspace_bytes(const shtb_plan* p, int op, int nf);
 
 // Grouped (uneven-batch) execution: persistent launches over the tiles of many plans.
+#ifdef __CUDACC__
+__device__ __forceinline__ unsigned long long group_time() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// Records the earliest start of the roundtrip's first kernels as the complement (zeroed memory
+// holds "not yet").
+__device__ __forceinline__ void group_start(unsigned long long* t0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(t0, ~group_time());
+}
+#endif
 int mixed_prepare(const shtb_plan* p, cudaStream_t st);
 size_t mixed_args_bytes();
 void mixed_fill_args(const shtb_plan* p, int mode, const void* in, void* out, int nf, void* host_args);
@@ -85,24 +98,31 @@ unsigned long long mixed_group_tile(const shtb_plan* p, int mode, int im, int t0
 int mixed_group_tile_rows();
 int launch_gemm_group(int mode, const void* targs, const int4* items, const unsigned long long* masks, int nitems,
                       int grid, unsigned long long* done, int* queue, cudaStream_t st);
-int launch_pack_group(const void* targs, const int2* items, int nitems, int grid, int* queue, cudaStream_t st);
+int launch_pack_group(const void* targs, const int2* items, int nitems, int grid, int* queue, unsigned long long* t0,
+                      cudaStream_t st);
 size_t fft_job_bytes_f32();
 void fft_fill_job_f32(const shtb_plan* p, int syn, const void* W, void* grid, int nf, void* host_job);
 size_t fft_group_smem_f32(const shtb_plan* p, int h);
 bool fft_plan_generic(const shtb_plan* p);
 int launch_fft_group_f32(int syn, int h, bool generic, const void* jobs, const int4* items, int nitems, int grid,
                          size_t smem, int* queue, cudaStream_t st);
-// Mixed-precision Legendre synthesis on the FP64 pipes for one or two fields (simt.cu):
-// coefficients (dense or packed LM) -> Fourier buffer.
+// Mixed-precision Legendre stage on the FP64 pipes for one or two fields (simt.cu): coefficients
+// (dense or packed LM) <-> Fourier buffer.
 bool simt_applicable(const shtb_plan* p, int nf);
 int launch_simt_syn(const shtb_plan* p, const void* alm, void* W, int nf, int ltr, int mlim, int packed,
                     cudaStream_t st);
+int launch_simt_ana(const shtb_plan* p, const void* W, void* alm, int nf, int ltr, int mlim, int packed,
+                    cudaStream_t st);
 size_t simt_args_bytes();
-void simt_fill_args(const shtb_plan* p, const void* alm, void* W, int nf, void* host_args);
+// syn: coefficients -> Fourier buffer, else Fourier buffer -> coefficients.
+void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int nf, void* host_args);
+int simt_ana_segment(int nf);   // degrees per item of the grouped analysis
 int simt_syn_pair_blocks(const shtb_plan* p);
 size_t simt_group_syn_smem(const shtb_plan* p);
 int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, size_t smem, int* queue,
-                      cudaStream_t st);
+                      unsigned long long* t0, cudaStream_t st);
+int launch_simt_ana_group(const void* targs, const int4* items, int nitems, int grid, int* queue,
+                          unsigned long long* done, cudaStream_t st);
 // the packed-pair FP32 FFTs of fft2_applicable members (2 HP latitude pairs per item)
 size_t fft2_job_bytes();
 int fft2_group_pairs();

@@ -1165,9 +1165,11 @@ __device__ __forceinline__ void pack_field1(const Args& a, int im, int k) {
 // claimed in list order from the device counter *queue (zero at launch).
 __global__ void __launch_bounds__(kPack1Threads) mixed_pack_group_kernel(const Args* __restrict__ targs,
                                                                        const int2* __restrict__ items, int nitems,
-                                                                       int* __restrict__ queue) {
+                                                                       int* __restrict__ queue,
+                                                                       unsigned long long* __restrict__ t0) {
   __shared__ Args sa;
   __shared__ int s_item, s_order;
+  group_start(t0);
   for (;;) {
     if (threadIdx.x == 0) {
       const int i = atomicAdd(queue, 1);
@@ -1496,6 +1498,15 @@ __global__ void zero_columns_kernel32(PlanDev P, float2* __restrict__ a, long lo
   for (int l = threadIdx.x; l <= P.lmax; l += blockDim.x) col[l] = make_float2(0.f, 0.f);
 }
 
+static int clear_columns(const shtb_plan* p, void* alm, int nf, int mlim, cudaStream_t st) {
+  if (p->mres == 1 && mlim >= p->mmax) return SHTB_OK;
+  prof_begin(st);
+  zero_columns_kernel32<<<dim3(p->mmax + 1, nf), 256, 0, st>>>(p->dev, (float2*)alm,
+                                                               (long long)(p->lmax + 1) * (p->mmax + 1), mlim);
+  SHTB_LAUNCHED("zero fill kernel");
+  return SHTB_OK;
+}
+
 static Args base_args(const shtb_plan* p) {
   Args a{};
   a.P = p->dev;
@@ -1635,12 +1646,17 @@ int mixed_analysis(const shtb_plan* p, const void* f, void* alm, int nf, int ltr
                    int packed) {
   const int mlim = std::min(p->mmax, ltr);
   int rc;
-  if ((rc = ensure_table(p, st))) return rc;
   const long long nlm = lm_count(p->lmax, p->mmax, p->mres);
+  const bool simt = simt_applicable(p, nf);   // one or two fields: recurrence on the FP64 pipes, no table
+  if (!simt && (rc = ensure_table(p, st))) return rc;
   if (packed && ltr < p->lmax)   // degrees above ltr are no tile's output
     SHTB_TRY_CUDA(cudaMemsetAsync(alm, 0, (size_t)nlm * nf * sizeof(float2), st), "packed output clear");
-  if ((rc = launch_fft_ana<float, float>(p, (const float*)f, nullptr, 1, work, nf, mlim, p->ana_scale, 1, 0, st, 1)))
+  if ((rc = launch_fft_ana<float, float>(p, (const float*)f, nullptr, 1, work, nf, mlim, p->ana_scale, 1, 0, st, !simt)))
     return rc;
+  if (simt) {
+    if ((rc = launch_simt_ana(p, work, alm, nf, ltr, mlim, packed, st))) return rc;
+    return packed ? SHTB_OK : clear_columns(p, alm, nf, mlim, st);
+  }
   // analysis tiles: 128 degrees of each parity per tile
   shtb_plan::MxTileList tl;
   if ((rc = gemm_tiles_list(p, 1, ltr, mlim, st, &tl))) return rc;
@@ -1659,13 +1675,7 @@ int mixed_analysis(const shtb_plan* p, const void* f, void* alm, int nf, int ltr
     a.ld_k = nlm;
   }
   if ((rc = dispatch_gemm<1>(p, a, nf, 2 * tl.count, st))) return rc;
-  if (!packed && (p->mres > 1 || mlim < p->mmax)) {
-    dim3 zg(p->mmax + 1, nf);
-    prof_begin(st);
-    zero_columns_kernel32<<<zg, 256, 0, st>>>(p->dev, (float2*)alm, a.ld_k, mlim);
-    SHTB_LAUNCHED("zero fill kernel");
-  }
-  return SHTB_OK;
+  return packed ? SHTB_OK : clear_columns(p, alm, nf, mlim, st);
 }
 
 // ---------------------------------------------------------------- grouped transforms
@@ -1711,9 +1721,10 @@ unsigned long long mixed_group_tile(const shtb_plan* p, int mode, int im, int t0
 
 int mixed_group_tile_rows() { return kM; }
 
-int launch_pack_group(const void* targs, const int2* items, int nitems, int grid, int* queue, cudaStream_t st) {
+int launch_pack_group(const void* targs, const int2* items, int nitems, int grid, int* queue, unsigned long long* t0,
+                      cudaStream_t st) {
   if (nitems <= 0) return SHTB_OK;
-  mixed_pack_group_kernel<<<grid, kPack1Threads, 0, st>>>((const Args*)targs, items, nitems, queue);
+  mixed_pack_group_kernel<<<grid, kPack1Threads, 0, st>>>((const Args*)targs, items, nitems, queue, t0);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "group pack launch");
   return SHTB_OK;

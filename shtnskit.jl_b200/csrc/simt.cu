@@ -1,5 +1,5 @@
 // simt.cu — Legendre stage for one or two fields, with the recurrence regenerated on the fly
-// on the FP64 pipes: synthesis and analysis of the FP64 path, synthesis of the mixed path.
+// on the FP64 pipes: synthesis and analysis of the FP64 and of the mixed path.
 //
 // With one or two fields an MMA tile is mostly padding: the FP64 MMAs take 8 columns for 2 or
 // 4, and the tensor-core GEMM of mixed.cu streams 4 bytes of P table per value for 2 or 4
@@ -13,7 +13,8 @@
 //              the sum over pairs crosses the lanes once, at the end
 // E and O (even and odd l - m) sums in FP64 on both paths. Measured at lmax 1023, one field
 // (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 164 us against the 8-column MMA
-// kernels; the FP64 pipes alone would take about 60 us each.
+// kernels; the FP64 pipes alone would take about 60 us each. Mixed path at lmax 511, one field:
+// the analysis GEMM, which streams 134 MB of P table for 2 columns, 41 us, this kernel 37 us.
 #include <climits>
 #include <cstring>
 #include <type_traits>
@@ -244,6 +245,8 @@ __device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, con
   const int* pl0 = P.l0 + (size_t)im * npair;
   const C* W = (const C*)a.cin + (size_t)im * 2 * npair;
   const size_t wld = (size_t)P.nm * 2 * npair;
+  const double* px = P.x;
+  const int nf = a.nf;
   double2 acc[SG][NF];
 #pragma unroll
   for (int s = 0; s < SG; ++s)
@@ -263,7 +266,7 @@ __device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, con
       const bool ok = p < npair;
       const int pc = ok ? p : 0;
       cp_async<16>(&R.ck[fq][u][lane], ck + pc, ok);
-      cp_async<8>(&R.x[fq][u][lane], P.x + pc, ok);
+      cp_async<8>(&R.x[fq][u][lane], px + pc, ok);
       cp_async<4>(&R.l0[fq][u][lane], pl0 + pc, ok);
 #pragma unroll
       for (int k = 0; k < NF; ++k) {
@@ -365,7 +368,7 @@ __device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, con
     }
   }
   const int l = lseg + lane / NF, k = lane % NF;
-  if (l <= a.lcap && k < a.nf) {
+  if (l <= a.lcap && k < nf) {
     const double f = factor_at(a, poff, l, m);
     C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
     narrow(*dst, make_double2(v[0].x * f, v[0].y * f));
@@ -487,8 +490,10 @@ __device__ __forceinline__ void syn_warp_item(const Args& a, int im, int pb, dou
 
 __global__ void __launch_bounds__(kThreads, 8) syn_group_kernel(const Args* __restrict__ targs,
                                                                 const int4* __restrict__ items, int nitems,
-                                                                int* __restrict__ queue) {
+                                                                int* __restrict__ queue,
+                                                                unsigned long long* __restrict__ t0) {
   extern __shared__ __align__(16) double smem[];
+  group_start(t0);
   double* wsm = smem + (threadIdx.x >> 5) * kGroupWarpDoubles;
   const int lane = threadIdx.x & 31;
   for (;;) {
@@ -502,6 +507,56 @@ __global__ void __launch_bounds__(kThreads, 8) syn_group_kernel(const Args* __re
       syn_warp_item<1>(a, it.y, it.z, wsm);
     else
       syn_warp_item<2>(a, it.y, it.z, wsm);
+  }
+}
+
+// Persistent analysis over the items of many transforms, one item per warp: item = (transform,
+// order, segment of kSeg degrees), list sorted by decreasing work and claimed by each warp from
+// *queue. A segment's sums are those of ana_kernel, so the results are the same bit for bit. The
+// warp of an order's first segment clears the degrees below the order. done[t] receives the
+// largest %globaltimer value at which an item of transform t was stored.
+struct GroupAnaWarp {
+  union {
+    Ring<float2, 1> r1;
+    Ring<float2, 2> r2;
+  };
+  double sal[32];
+};
+
+template <int NF>
+__device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, Ring<float2, NF>& R, double* sal) {
+  const int lane = threadIdx.x & 31, m = im * a.P.mres, lseg = m + kSeg<NF> * seg;
+  __syncwarp();   // the previous item's alpha is read
+  if (lane < kSeg<NF>) sal[lane] = (lseg + lane <= a.lend) ? a.P.alpha[a.P.off[im] + (lseg + lane - m)] : 0.0;
+  __syncwarp();
+  ana_segment<float2, NF>(a, im, lseg, sal, R);
+  if (seg == 0)
+    for (int k = 0; k < a.nf; ++k) {
+      float2* col = (float2*)a.out + (long long)k * a.ld_k + (long long)m * a.ld_m;
+      for (int l = lane; l < m; l += 32) col[l] = make_float2(0.f, 0.f);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) ana_group_kernel(const Args* __restrict__ targs,
+                                                             const int4* __restrict__ items, int nitems,
+                                                             int* __restrict__ queue,
+                                                             unsigned long long* __restrict__ done) {
+  __shared__ __align__(16) GroupAnaWarp sw[kThreads / 32];
+  GroupAnaWarp& w = sw[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    int i = 0;
+    if (lane == 0) i = atomicAdd(queue, 1);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if (i >= nitems) break;
+    const int4 it = items[i];
+    const Args& a = targs[it.x];
+    if (a.nf == 1)
+      ana_warp_item<1>(a, it.y, it.z, w.r1, w.sal);
+    else
+      ana_warp_item<2>(a, it.y, it.z, w.r2, w.sal);
+    __syncwarp();
+    if (lane == 0) atomicMax(done + it.x, group_time());
   }
 }
 
@@ -541,20 +596,39 @@ static int launch_syn(const shtb_plan* p, const sx::Args& a, int nmu, const char
   return SHTB_OK;
 }
 
-static Factors mixed_factors(const shtb_plan* p) {
-  return Factors{p->dev.cfac, p->d_scale, p->d_scale ? 1 : 0, 1.0, 1.0};
+static Factors mixed_factors(const shtb_plan* p, int sc_mode) {
+  return Factors{p->dev.cfac, p->d_scale, p->d_scale ? sc_mode : 0, 1.0, 1.0};
 }
 
 // Coefficients (FP32, dense or packed LM) -> Fourier buffer W (FP32), orders 0..mlim.
 int launch_simt_syn(const shtb_plan* p, const void* alm, void* W, int nf, int ltr, int mlim, int packed,
                     cudaStream_t st) {
-  sx::Args a = simt_args(p, alm, W, mixed_factors(p), nf, ltr);
+  sx::Args a = simt_args(p, alm, W, mixed_factors(p, 1), nf, ltr);
   a.packed = packed ? 2 : 0;
   a.ld_k = packed ? lm_count(p->lmax, p->mmax, p->mres) : (long long)(p->lmax + 1) * (p->mmax + 1);
   a.ld_m = p->lmax + 1;
   const int nmu = mlim / p->mres + 1;
   return nf == 1 ? launch_syn<float2, 1>(p, a, nmu, "simt legendre synthesis kernel", st)
                  : launch_syn<float2, 2>(p, a, nmu, "simt legendre synthesis kernel", st);
+}
+
+// Fourier buffer W (FP32) -> coefficients (FP32, dense or packed LM), degrees up to ltr.
+int launch_simt_ana(const shtb_plan* p, const void* W, void* alm, int nf, int ltr, int mlim, int packed,
+                    cudaStream_t st) {
+  sx::Args a = simt_args(p, W, alm, mixed_factors(p, 2), nf, ltr);
+  a.packed = packed ? 2 : 0;
+  a.ld_k = packed ? lm_count(p->lmax, p->mmax, p->mres) : (long long)(p->lmax + 1) * (p->mmax + 1);
+  a.ld_m = p->lmax + 1;
+  a.mlim = mlim;
+  a.lcap = ltr;
+  a.zero_fill = !packed;
+  prof_begin(st);
+  if (nf == 1)
+    sx::ana_kernel<float2, 1><<<p->dev.natiles, 128, 0, st>>>(a);
+  else
+    sx::ana_kernel<float2, 2><<<dim3(p->dev.natiles, 2), 128, 0, st>>>(a);
+  SHTB_LAUNCHED("simt legendre analysis kernel");
+  return SHTB_OK;
 }
 
 // FP64 coefficients -> Fourier buffer for one or two fields.
@@ -591,25 +665,37 @@ int launch_simt_ana64(const shtb_plan* p, const void* W, int nf, int row_end, in
 // ------------------------------------------------------------- grouped transforms
 size_t simt_args_bytes() { return sizeof(sx::Args); }
 
-void simt_fill_args(const shtb_plan* p, const void* alm, void* W, int nf, void* host_args) {
-  sx::Args a = simt_args(p, alm, W, mixed_factors(p), nf, p->lmax);
+void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int nf, void* host_args) {
+  sx::Args a = simt_args(p, in, out, mixed_factors(p, syn ? 1 : 2), nf, p->lmax);
   a.ld_k = (long long)(p->lmax + 1) * (p->mmax + 1);
   a.ld_m = p->lmax + 1;
+  a.lcap = p->lmax;
   std::memcpy(host_args, &a, sizeof(a));
 }
+
+int simt_ana_segment(int nf) { return nf == 1 ? sx::kSeg<1> : sx::kSeg<2>; }
 
 int simt_syn_pair_blocks(const shtb_plan* p) { return (p->npair + 31) / 32; }   // per-warp items of the group kernel
 
 size_t simt_group_syn_smem(const shtb_plan*) { return (sx::kThreads / 32) * sx::kGroupWarpDoubles * sizeof(double); }
 
 int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, size_t smem, int* queue,
-                      cudaStream_t st) {
+                      unsigned long long* t0, cudaStream_t st) {
   if (nitems <= 0) return SHTB_OK;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(sx::syn_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "simt group smem attr");
-  sx::syn_group_kernel<<<grid, sx::kThreads, smem, st>>>((const sx::Args*)targs, items, nitems, queue);
+  sx::syn_group_kernel<<<grid, sx::kThreads, smem, st>>>((const sx::Args*)targs, items, nitems, queue, t0);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "simt group launch");
+  return SHTB_OK;
+}
+
+int launch_simt_ana_group(const void* targs, const int4* items, int nitems, int grid, int* queue,
+                          unsigned long long* done, cudaStream_t st) {
+  if (nitems <= 0) return SHTB_OK;
+  sx::ana_group_kernel<<<grid, sx::kThreads, 0, st>>>((const sx::Args*)targs, items, nitems, queue, done);
+  count_launch();
+  SHTB_TRY_CUDA(cudaGetLastError(), "simt analysis group launch");
   return SHTB_OK;
 }
 
