@@ -526,16 +526,30 @@ static FFTJob<T> fft_job(const shtb_plan* p, const int* perm, const typename V2<
   return J;
 }
 
-// H latitude pairs per CTA: the largest power of two <= 16 whose shared-memory
-// footprint stays within ~200 KB (one CTA of 512 threads per SM). Two CTAs of 256
-// threads with half the pairs measured slower on B200: their grid segments shrink to
-// 16 bytes and each FFT has half the threads.
-static int fft_pick_h(const FFTDesc& fd, size_t celem, int npair) {
+// Latitude pairs and threads of a CTA. A CTA runs its loads, passes and stores one after the
+// other behind barriers, so an SM needs several CTAs in different phases: the registers
+// allow 512 threads an SM, here as two CTAs of 256 or four of 128 wherever rows are short
+// enough that a CTA still holds 4 or 8 pairs (grid runs of at least 16 bytes) at some 23 points
+// a thread. Measured, synthesis / analysis in us, against one CTA of 512 threads with the most
+// pairs that fit:
+//   FP32 nlon 1080, 64 fields 263 / 252 -> 254 / 242, 13 fields 84 / 78 -> 62 / 60;
+//   FP64 nlon 720, 20 fields 72 / 64 -> 64 / 60; nlon 512, 32 fields 31 / 41 -> 31 / 39;
+//   nlon 2048 keeps 4 pairs and 512 threads (211 / 256; 2 pairs and 256 threads 262 / 281).
+// Pairs are halved, down to 2 (4 for the B tile images, which are written 4 pairs at a time),
+// while the launch fills less than three quarters of the SMs' CTA slots: FP64 nlon 720,
+// 3 fields 23 / 23 -> 17 / 17; FP32 nlon 720, one field 41 / 29 -> 17 / 17.
+struct FFTShape {
+  int h, threads;
+};
+static FFTShape fft_shape(const FFTDesc& fd, size_t celem, int npair, int nfw, int wtile) {
+  constexpr int kSMs = 148;
   const size_t S = (size_t)fft_row_stride(fd.n, fft_padsh(fd, celem));
-  int h = 16;
+  int h = (fd.n <= 760 && !fd.big) ? 8 : 4;
   while (h > 1 && (size_t)h * S * celem * (fd.big ? 2 : 1) + 16 * 8 > 200 * 1024) h >>= 1;
-  while (h > 1 && h / 2 >= npair) h >>= 1;
-  return h;
+  int t = 64;
+  while (t < 512 && (celem == 16 ? 23 : 24) * t < h * fd.n) t <<= 1;
+  while (h > (wtile ? 4 : 2) && 4ll * ((npair + h - 1) / h) * nfw < 3ll * kSMs * (512 / t)) h >>= 1;
+  return FFTShape{h, t};
 }
 
 static size_t fft_smem(const FFTDesc& fd, size_t celem, int h) {
@@ -553,7 +567,7 @@ static bool fft_generic(const shtb_plan* p) {
 
 template <typename T, int H>
 static int launch_syn_h(const shtb_plan* p, const void* W, T* out0, T* out1, int ncomp, int nfw, int mlim,
-                        double gscale, int use_w, int spow, cudaStream_t st) {
+                        double gscale, int use_w, int spow, int threads, cudaStream_t st) {
   using V = typename V2<T>::type;
   const size_t smem = fft_smem(p->fft, sizeof(V), H);
   if (smem > 227 * 1024) return set_error(SHTB_ERR_UNSUPPORTED, "nlon too large for the shared-memory FFT");
@@ -562,14 +576,14 @@ static int launch_syn_h(const shtb_plan* p, const void* W, T* out0, T* out1, int
   dim3 grid((p->npair + H - 1) / H, nfw);
   const FFTJob<T> J = fft_job<T>(p, p->d_rinv, (const V*)W, nullptr, out0, out1, ncomp, mlim, gscale, use_w, spow);
   prof_begin(st);
-  kern<<<grid, 512, smem, st>>>(J);
+  kern<<<grid, threads, smem, st>>>(J);
   SHTB_LAUNCHED("fft synthesis kernel");
   return SHTB_OK;
 }
 
 template <typename T, int H>
 static int launch_ana_h(const shtb_plan* p, const T* in0, const T* in1, int ncomp, void* W, int nfw, int mlim,
-                        double wscale, int use_w, int spow, int wtile, cudaStream_t st) {
+                        double wscale, int use_w, int spow, int wtile, int threads, cudaStream_t st) {
   using V = typename V2<T>::type;
   const size_t smem = fft_smem(p->fft, sizeof(V), H);
   if (smem > 227 * 1024) return set_error(SHTB_ERR_UNSUPPORTED, "nlon too large for the shared-memory FFT");
@@ -580,7 +594,7 @@ static int launch_ana_h(const shtb_plan* p, const T* in0, const T* in1, int ncom
   const FFTJob<T> J = fft_job<T>(p, p->d_rev, nullptr, (V*)W, const_cast<T*>(in0), const_cast<T*>(in1), ncomp, mlim,
                                  wscale, use_w, spow, wtile, nfw);
   prof_begin(st);
-  kern<<<grid, 512, smem, st>>>(J);
+  kern<<<grid, threads, smem, st>>>(J);
   SHTB_LAUNCHED("fft analysis kernel");
   return SHTB_OK;
 }
@@ -593,12 +607,12 @@ int launch_fft_syn(const shtb_plan* p, const void* W, GT* out0, GT* out1, int nc
     if (ncomp == 1 && !use_w && !spow && fft2_applicable(p))
       return launch_fft2_syn(p, W, (float*)out0, nfw, mlim, gscale, st);
   }
-  switch (fft_pick_h(p->fft, sizeof(typename V2<T>::type), p->npair)) {
-    case 16: return launch_syn_h<T, 16>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, st);
-    case 8: return launch_syn_h<T, 8>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, st);
-    case 4: return launch_syn_h<T, 4>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, st);
-    case 2: return launch_syn_h<T, 2>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, st);
-    default: return launch_syn_h<T, 1>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, st);
+  const FFTShape s = fft_shape(p->fft, sizeof(typename V2<T>::type), p->npair, nfw, 0);
+  switch (s.h) {
+    case 8: return launch_syn_h<T, 8>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, s.threads, st);
+    case 4: return launch_syn_h<T, 4>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, s.threads, st);
+    case 2: return launch_syn_h<T, 2>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, s.threads, st);
+    default: return launch_syn_h<T, 1>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, s.threads, st);
   }
 }
 
@@ -610,12 +624,12 @@ int launch_fft_ana(const shtb_plan* p, const GT* in0, const GT* in1, int ncomp, 
     if (ncomp == 1 && use_w && !spow && fft2_applicable(p))
       return launch_fft2_ana(p, (const float*)in0, W, nfw, mlim, wscale, wtile, st);
   }
-  switch (fft_pick_h(p->fft, sizeof(typename V2<T>::type), p->npair)) {
-    case 16: return launch_ana_h<T, 16>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, st);
-    case 8: return launch_ana_h<T, 8>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, st);
-    case 4: return launch_ana_h<T, 4>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, st);
-    case 2: return launch_ana_h<T, 2>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, st);
-    default: return launch_ana_h<T, 1>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, st);
+  const FFTShape s = fft_shape(p->fft, sizeof(typename V2<T>::type), p->npair, nfw, wtile);
+  switch (s.h) {
+    case 8: return launch_ana_h<T, 8>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, s.threads, st);
+    case 4: return launch_ana_h<T, 4>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, s.threads, st);
+    case 2: return launch_ana_h<T, 2>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, s.threads, st);
+    default: return launch_ana_h<T, 1>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, s.threads, st);
   }
 }
 
@@ -772,7 +786,8 @@ static int launch_fft_group_h(int syn, const void* jobs, const int4* items, int 
                               int* queue, cudaStream_t st) {
   auto kern = syn ? fft_group_kernel<float, H, GENERIC, true> : fft_group_kernel<float, H, GENERIC, false>;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "group fft smem attr");
-  kern<<<grid, 512, smem, st>>>((const FFTJob<float>*)jobs, items, nitems, queue);
+  // two CTAs of 256 threads an SM (the launch shapes count such CTAs)
+  kern<<<grid, 256, smem, st>>>((const FFTJob<float>*)jobs, items, nitems, queue);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "group fft launch");
   return SHTB_OK;

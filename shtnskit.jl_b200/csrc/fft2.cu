@@ -15,7 +15,7 @@
 // Scope: power-of-two nlon from 64 to 2048 and nlat a multiple of 4 (every latitude has
 // its mirror, the south rows of two pairs are adjacent, and pair-pairs start on 16-byte
 // boundaries of the Fourier buffer); other sizes use the general kernels.
-// One CTA transforms 2 HP latitude pairs (HP pair-pairs) of one field with 128 HP threads.
+// One CTA transforms 2 HP latitude pairs (HP pair-pairs) of one field with up to 128 HP threads.
 #include <algorithm>
 #include <cstring>
 
@@ -535,10 +535,19 @@ static f2::Job fft2_job(const shtb_plan* p, const int* perm, double scale, int n
   return J;
 }
 
-// Pair-pairs per CTA: 4 (8 latitude pairs, 512 threads, one CTA per SM). Two CTAs of 2
+// Pair-pairs per CTA: 4 (8 latitude pairs). Two CTAs of 2
 // pair-pairs per SM measured slower (0.56 vs 0.51 ms analysis, 0.51 vs 0.43 ms synthesis
 // at nlon 2048, 64 fields).
 constexpr int kFft2HP = 4;
+// Threads of a CTA: 512 at nlon 2048, whose rows fill an SM's shared memory; shorter rows run
+// several smaller CTAs an SM, 16 points a thread, so that their loads, passes and stores
+// overlap (64 fields, synthesis / analysis: nlon 1024 117 / 129 -> 90 / 103 us, nlon 512 39 / 45 ->
+// 29 / 31), as long as the launch still fills the SMs' 512 threads.
+static int fft2_threads(const shtb_plan* p, long long ctas) {
+  int t = std::max(64, std::min(512, p->fft.n * kFft2HP / 16));
+  while (t < 512 && ctas * t < 148ll * 512) t <<= 1;
+  return t;
+}
 
 int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int mlim, double wscale, int wtile,
                     cudaStream_t st) {
@@ -554,7 +563,7 @@ int launch_fft2_ana(const shtb_plan* p, const float* grid, void* W, int nf, int 
   // tile region run together
   dim3 grd(nf, (p->npair + 2 * HP - 1) / (2 * HP));
   prof_begin(st);
-  f2::ana_kernel<HP><<<grd, 128 * HP, smem, st>>>(J);
+  f2::ana_kernel<HP><<<grd, fft2_threads(p, (long long)grd.x * grd.y), smem, st>>>(J);
   SHTB_LAUNCHED("fft analysis kernel");
   return SHTB_OK;
 }
@@ -586,7 +595,7 @@ int launch_fft2_group(int syn, const void* jobs, const int4* items, int nitems, 
   auto kern = syn ? f2::group_kernel<HP, true> : f2::group_kernel<HP, false>;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "group fft2 smem attr");
-  kern<<<grid, 128 * HP, smem, st>>>((const f2::Job*)jobs, items, nitems, queue);
+  kern<<<grid, 64 * HP, smem, st>>>((const f2::Job*)jobs, items, nitems, queue);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "group fft2 launch");
   return SHTB_OK;
@@ -602,7 +611,7 @@ int launch_fft2_syn(const shtb_plan* p, const void* W, float* grid, int nf, int 
   J.grid = grid;
   dim3 grd((p->npair + 2 * HP - 1) / (2 * HP), nf);
   prof_begin(st);
-  f2::syn_kernel<HP><<<grd, 128 * HP, smem, st>>>(J);
+  f2::syn_kernel<HP><<<grd, fft2_threads(p, (long long)grd.x * grd.y), smem, st>>>(J);
   SHTB_LAUNCHED("fft synthesis kernel");
   return SHTB_OK;
 }

@@ -294,7 +294,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
     f2items.swap(sorted);
   }
   g->n_fft2 = (int)f2items.size();
-  g->fft2_ctas = std::max(1, std::min(g->nsm, g->n_fft2));
+  g->fft2_ctas = std::max(1, std::min(2 * g->nsm, g->n_fft2));   // CTAs of 256 threads, two per SM where rows fit
   // GEMM tiles with their live-chunk masks, most live K-steps first
   const int TM = mixed_group_tile_rows();
   std::vector<int4> syn, ana;
