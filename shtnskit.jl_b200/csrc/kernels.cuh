@@ -76,6 +76,27 @@ size_t fft_btile_floats(const shtb_plan* p, int nf);
 // Bytes of the mixed path's workspace for op (SHTB_OP_SYNTHESIS or SHTB_OP_ANALYSIS).
 size_t mixed_workspace_bytes(const shtb_plan* p, int op, int nf);
 
+#ifdef __CUDACC__
+// First latitude pair of the first block of 32 (a multiple of 32) in which some pair starts below
+// degree lim; npair or more if none does. Eight blocks' start degrees load together: one
+// after the other, the blocks near the poles that a high order skips cost a memory latency each.
+__device__ __forceinline__ int first_live_pair(const int* __restrict__ l0, int npair, int lim) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < npair; base += 256) {
+    int v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int p = base + 32 * j + lane;
+      v[j] = p < npair ? l0[p] : lim;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (__any_sync(0xffffffffu, v[j] < lim)) return base + 32 * j;
+  }
+  return npair;
+}
+#endif
+
 // Grouped (uneven-batch) execution: persistent launches over the tiles of many plans.
 #ifdef __CUDACC__
 __device__ __forceinline__ unsigned long long group_time() {

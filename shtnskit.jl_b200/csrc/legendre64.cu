@@ -361,11 +361,7 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
 
   // leading groups of 32 pairs that all start above the tile hold only zeros
   const int nk = (npair + 3) / 4;
-  int k0 = 0;
-  for (; k0 < nk; k0 += 8) {
-    const int p = 4 * k0 + lane;
-    if (__any_sync(0xffffffffu, p < npair && pl0[p] <= tlast)) break;
-  }
+  const int k0 = first_live_pair(pl0, npair, tlast + 1) / 4;
   // operand ring: each lane copies its own operands of the next RG - 1 steps (a checkpoint, x,
   // W of MT fields, E and O) and reads them back itself, so no barrier is needed
   constexpr int RG = kAnaRing, NS = 2 * MT + 1;

@@ -253,11 +253,7 @@ __device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, con
 #pragma unroll
     for (int k = 0; k < NF; ++k) acc[s][k] = make_double2(0.0, 0.0);
   // pairs from the first block with a start below the segment's end
-  int p0 = 0;
-  for (; p0 < npair; p0 += 32) {
-    const int p = p0 + lane;
-    if (__any_sync(0xffffffffu, p < npair && pl0[p] < lseg + SG)) break;
-  }
+  int p0 = first_live_pair(pl0, npair, lseg + SG);
   int fp = p0 + lane, fq = 0;   // next pair and slot to copy
   auto fetch = [&]() {
 #pragma unroll
