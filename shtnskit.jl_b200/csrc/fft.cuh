@@ -171,16 +171,21 @@ __device__ __forceinline__ void dft_small(V* u, int dir, const V* __restrict__ t
 // W_Ns^(j*q) on output q, read from this pass's table twp[(q-1)*span + j].
 // Group indices are split with multiply-high divisions (magic_div_mul), and each
 // thread loads two groups before computing either so their loads overlap.
-template <typename T, typename V, int RADIX>
-__device__ __forceinline__ void dif_group_load(const V* X, int S, int N, int span, unsigned mrow, unsigned mspan,
-                                               int per_row, int r, int b, V* u, int& rowoff, int& base, int& j,
-                                               int sh) {
+__device__ __forceinline__ void dif_group_at(int b, int S, int r, int span, int per_row, unsigned mrow, unsigned mspan,
+                                             int& rowoff, int& base, int& j) {
   const int f = mrow ? (int)__umulhi((unsigned)b, mrow) : b;
   const int t = b - f * per_row;
   const int blk = mspan ? (int)__umulhi((unsigned)t, mspan) : t;
   j = t - blk * span;
   base = blk * span * r + j;
   rowoff = f * S;
+}
+
+template <typename T, typename V, int RADIX>
+__device__ __forceinline__ void dif_group_load(const V* X, int S, int N, int span, unsigned mrow, unsigned mspan,
+                                               int per_row, int r, int b, V* u, int& rowoff, int& base, int& j,
+                                               int sh) {
+  dif_group_at(b, S, r, span, per_row, mrow, mspan, rowoff, base, j);
 #pragma unroll
   for (int q = 0; q < RADIX; ++q)
     if (q < r) u[q] = X[rowoff + fft_pad(base + q * span, sh)];
@@ -242,31 +247,12 @@ __device__ __forceinline__ void dif_pass(V* X, int F, int N, int S, int Ns, int 
 // values of k for GU groups, so that a pair of table values serves GU groups and a pair of
 // elements KU sums (one table load and one shared-memory load for every 8 multiply-adds).
 // FP64, nlon 402 = 2 3 67, 102 pairs x 3 fields: 279 -> 33 us against the dense DFT.
-template <typename T, typename V>
-__device__ __forceinline__ void dif_pass_prime(V* X, V* Y, int F, int N, int S, int Ns, int r, const V* __restrict__ tw,
-                                               const V* __restrict__ twp, unsigned mrow, unsigned mspan, int dir, int sh) {
-  constexpr int KU = 4, GU = 2;
-  const int span = Ns / r, per_row = N / r, total = F * per_row, h = (r - 1) >> 1, tws = N / r;
+template <typename T, typename V, int KU, int GU>
+__device__ __forceinline__ void dif_prime_sums(const V* X, V* Y, int N, int S, int Ns, int r, const V* __restrict__ tw,
+                                               const V* __restrict__ twp, unsigned mrow, unsigned mspan, int dir, int sh,
+                                               int total) {
+  const int span = Ns / r, per_row = N / r, h = (r - 1) >> 1, tws = N / r;
   const int bd = blockDim.x;
-  auto locate = [&](int b, int& rowoff, int& base, int& j) {
-    const int f = mrow ? (int)__umulhi((unsigned)b, mrow) : b;
-    const int t = b - f * per_row;
-    const int blk = mspan ? (int)__umulhi((unsigned)t, mspan) : t;
-    j = t - blk * span;
-    base = blk * span * r + j;
-    rowoff = f * S;
-  };
-  for (int i = threadIdx.x; i < total * h; i += bd) {
-    const int q = i / total + 1;
-    int ro, ba, j;
-    locate(i - (q - 1) * total, ro, ba, j);
-    V* p = X + ro + fft_pad(ba + q * span, sh);
-    V* m = X + ro + fft_pad(ba + (r - q) * span, sh);
-    const V a = *p, b = *m;
-    *p = cadd(a, b);
-    *m = csub(a, b);
-  }
-  __syncthreads();
   const int ngb = (total + GU - 1) / GU, nkb = h / KU + 1;
   for (int i = threadIdx.x; i < ngb * nkb; i += bd) {
     const int kb = i / ngb, gb = i - kb * ngb, k0 = kb * KU;
@@ -274,7 +260,7 @@ __device__ __forceinline__ void dif_pass_prime(V* X, V* Y, int F, int N, int S, 
     V A[GU][KU], B[GU][KU];
 #pragma unroll
     for (int g = 0; g < GU; ++g) {
-      locate(min(gb + g * ngb, total - 1), ro[g], ba[g], jj[g]);
+      dif_group_at(min(gb + g * ngb, total - 1), S, r, span, per_row, mrow, mspan, ro[g], ba[g], jj[g]);
       const V x0 = X[ro[g] + fft_pad(ba[g], sh)];
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
@@ -284,6 +270,7 @@ __device__ __forceinline__ void dif_pass_prime(V* X, V* Y, int F, int N, int S, 
     }
 #pragma unroll
     for (int u = 0; u < KU; ++u) t[u] = 0;
+#pragma unroll 2
     for (int j = 1; j <= h; ++j) {
       V w[KU];
 #pragma unroll
@@ -327,6 +314,29 @@ __device__ __forceinline__ void dif_pass_prime(V* X, V* Y, int F, int N, int S, 
       }
     }
   }
+}
+
+template <typename T, typename V>
+__device__ __forceinline__ void dif_pass_prime(V* X, V* Y, int F, int N, int S, int Ns, int r, const V* __restrict__ tw,
+                                               const V* __restrict__ twp, unsigned mrow, unsigned mspan, int dir, int sh) {
+  const int span = Ns / r, per_row = N / r, total = F * per_row, h = (r - 1) >> 1;
+  const int bd = blockDim.x;
+  for (int i = threadIdx.x; i < total * h; i += bd) {
+    const int q = i / total + 1;
+    int ro, ba, j;
+    dif_group_at(i - (q - 1) * total, S, r, span, per_row, mrow, mspan, ro, ba, j);
+    V* p = X + ro + fft_pad(ba + q * span, sh);
+    V* m = X + ro + fft_pad(ba + (r - q) * span, sh);
+    const V a = *p, b = *m;
+    *p = cadd(a, b);
+    *m = csub(a, b);
+  }
+  __syncthreads();
+  // wide sums while they still give every thread an item
+  if (((total + 1) / 2) * (h / 4 + 1) >= bd)
+    dif_prime_sums<T, V, 4, 2>(X, Y, N, S, Ns, r, tw, twp, mrow, mspan, dir, sh, total);
+  else
+    dif_prime_sums<T, V, 2, 1>(X, Y, N, S, Ns, r, tw, twp, mrow, mspan, dir, sh, total);
   __syncthreads();
 }
 
