@@ -313,12 +313,23 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
         ssyn.push_back(make_int4(t, im, pb, 0));
         cssyn.push_back(p->lmax - im + 1);
       }
+  }
+  long long nsegs = 0;
+  for (int t = 0; t < n; ++t)
+    if (g->simt[t]) nsegs += plans[t]->hoff[plans[t]->nm] / simt_ana_segment(nfields[t]);
+  const int per_item = simt_ana_segments_per_warp(nsegs);
+  for (int t = 0; t < n; ++t) {
+    if (!g->simt[t]) continue;
+    const shtb_plan* p = plans[t];
     const int sg = simt_ana_segment(nfields[t]);
-    for (int im = 0; im <= mlim; ++im)
-      for (int s = 0; im + s * sg <= p->lmax; ++s) {
-        sana.push_back(make_int4(t, im, s, 0));
-        csana.push_back(p->npair * sg * (2 + 2 * nfields[t]));
+    for (int im = 0; im <= std::min(p->mmax, p->lmax); ++im) {
+      const int segs = (p->lmax - im) / sg + 1;
+      for (int s = 0; s < segs; s += per_item) {
+        const int k = std::min(per_item, segs - s);
+        sana.push_back(make_int4(t, im, s, k));
+        csana.push_back(k * p->npair * sg * (2 + 2 * nfields[t]));
       }
+    }
   }
   for (int t = 0; t < n; ++t) {
     const shtb_plan* p = plans[t];

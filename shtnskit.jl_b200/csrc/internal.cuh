@@ -41,8 +41,10 @@ cudaError_t noalloc_scratch_address(void** out);
     if (_rc != SHTB_OK) return _rc;                                 \
   } while (0)
 
-// Degrees of one tile of the few-field FP64 analysis.
-constexpr int kAnaTile = 128;
+// Degrees of one tile of the FP64 analysis GEMM, and the widest checkpoint spacing.
+constexpr int kAnaTile = 64;
+constexpr int kSimtTile = 128;   // of the analysis of one and two fields
+constexpr int kMaxCkStep = 128;
 // Recurrence chains start at multiples of kStartStep degrees from their order.
 constexpr int kStartStep = 8;
 // Largest checkpoint table the plan keeps (bytes); the spacing grows from 8 degrees (the
@@ -66,11 +68,11 @@ struct PlanDev {
   // the state (r_{t-1}, r_{t-2}) before degree t = m + k * ckstep
   const double2* ckpt;
   const int* ckbase;       // [nm]
-  int ckstep;              // 8, 16, 32, 64 or 128 (a divisor of kAnaTile)
-  // FP64 analysis tiles (im, t0, 0, 0) of kAnaTile and of 64 degrees
-  const int4* atiles;
-  const int4* atiles64;
-  int natiles, natiles64;
+  int ckstep;              // 8, 16, 32, 64 or 128
+  // FP64 analysis GEMM tiles of kAnaTile degrees: (im, t0)
+  const int2* atiles;
+  const int2* stiles;      // the same of kSimtTile degrees
+  int natiles, nstiles;
 };
 
 // FFT description for nlon

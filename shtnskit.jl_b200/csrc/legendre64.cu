@@ -319,6 +319,7 @@ int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, v
 constexpr int kAnaThreads = 128;
 constexpr int kAnaSteps = 8;             // degrees per chain; 8 chains per tile
 constexpr int kAnaDeg = 8 * kAnaSteps;   // degrees per tile
+static_assert(kAnaDeg == kAnaTile, "tile list of the plan");
 constexpr int kAnaRing = 4;              // operand ring: steps of four pairs in flight, plus one
 
 template <int MT, int CG>
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
   constexpr int SL = kAnaSteps, KS = 4 / CG;
   __shared__ __align__(16) unsigned char buf[4 * kAnaRing * ((2 * MT + 1) * 512 + 256)];
   static_assert((KS - 1) * CG * SL * 4 * 32 * 8 <= sizeof(buf), "partial sums");
-  const int4 tile = P.atiles64[blockIdx.x];
+  const int2 tile = P.atiles[blockIdx.x];
   const int im = tile.x, t0 = tile.y, m = im * P.mres;
   const int lend = min(row_end, P.lrec);
   if (m > mlim || t0 > lend) return;
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
 template <int MT, int CG>
 static int launch_ana_tile(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                            const Factors& F, int zero_fill, cudaStream_t st) {
-  const dim3 grid(p->dev.natiles64, (nf + 8 * MT * CG - 1) / (8 * MT * CG));
+  const dim3 grid(p->dev.natiles, (nf + 8 * MT * CG - 1) / (8 * MT * CG));
   prof_begin(st);
   leg_ana64_kernel<MT, CG><<<grid, kAnaThreads, 0, st>>>(p->dev, (const double2*)W, nf, row_end, mlim, dst, F, zero_fill);
   SHTB_LAUNCHED("legendre analysis kernel");
@@ -501,6 +502,7 @@ static int launch_ana_tile(const shtb_plan* p, const void* W, int nf, int row_en
 
 int launch_leg_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                      const Factors& F, int zero_fill, cudaStream_t st) {
+  if (p->npair > 8192) return set_error(SHTB_ERR_UNSUPPORTED, "nlat too large for the FP64 analysis kernel");
   if (nf <= 2) return launch_simt_ana64(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
   if (nf > 32) return launch_ana_tile<2, 4>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
   if (nf > 16) return launch_ana_tile<2, 2>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);

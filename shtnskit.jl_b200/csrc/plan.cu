@@ -302,20 +302,19 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
     for (int im = 0; im < nm; ++im) n += (LR - im * mres + cs) / cs;
     return n;
   };
-  while (ckstep < kAnaTile && (size_t)nseg_total(ckstep) * npair * 16 > kCkptBudget) ckstep *= 2;
+  while (ckstep < kMaxCkStep && (size_t)nseg_total(ckstep) * npair * 16 > kCkptBudget) ckstep *= 2;
   std::vector<int> ckbase(nm);
   int nseg = 0;
   for (int im = 0; im < nm; ++im) {
     ckbase[im] = nseg;
     nseg += (LR - im * mres + ckstep) / ckstep;
   }
-  std::vector<int4> atiles, atiles64;
+  std::vector<int2> atiles, stiles;
   for (int im = 0; im < nm; ++im) {
-    const int m = im * mres;
-    for (int t0 = m; t0 <= LR; t0 += kAnaTile) atiles.push_back(make_int4(im, t0, 0, 0));
-    for (int t0 = m; t0 <= LR; t0 += 64) atiles64.push_back(make_int4(im, t0, 0, 0));
+    for (int t0 = im * mres; t0 <= LR; t0 += kAnaTile) atiles.push_back(make_int2(im, t0));
+    for (int t0 = im * mres; t0 <= LR; t0 += kSimtTile) stiles.push_back(make_int2(im, t0));
   }
-  const int natiles = (int)atiles.size(), natiles64 = (int)atiles64.size();
+  const int natiles = (int)atiles.size(), nstiles = (int)stiles.size();
   std::vector<double> alpha(npk, 0.0), cfac(npk, 1.0), dco(npk, 0.0);
   for (int im = 0; im < nm; ++im) {
     const int m = im * mres;
@@ -370,7 +369,7 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   const size_t o_off = take((nm + 1) * 8), o_alpha = take(npk * 8), o_c = take(npk * 8), o_d = take(npk * 8);
   const size_t o_l0 = take((size_t)nm * npair * 4), o_start = take((size_t)nm * npair * 16);
   const size_t o_ck = take((size_t)nseg * npair * 16), o_ckbase = take((size_t)nm * 4);
-  const size_t o_atiles = take((size_t)natiles * 16), o_atiles64 = take((size_t)natiles64 * 16);
+  const size_t o_atiles = take((size_t)natiles * sizeof(int2)), o_stiles = take((size_t)nstiles * sizeof(int2));
   const size_t o_scale = coeff_scale ? take((size_t)(lmax + 1) * (mmax + 1) * 8) : 0;
   const size_t o_tw = take((size_t)nlon * 16), o_tw32 = take((size_t)nlon * 8);
   const size_t o_seed = take((mmax + 2) * 8), o_rev = take((size_t)nlon * 4), o_rinv = take((size_t)nlon * 4);
@@ -395,8 +394,8 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   if (ce == cudaSuccess) ce = up(o_c, cfac.data(), npk * 8);
   if (ce == cudaSuccess) ce = up(o_d, dco.data(), npk * 8);
   if (ce == cudaSuccess) ce = up(o_ckbase, ckbase.data(), (size_t)nm * 4);
-  if (ce == cudaSuccess) ce = up(o_atiles, atiles.data(), (size_t)natiles * 16);
-  if (ce == cudaSuccess) ce = up(o_atiles64, atiles64.data(), (size_t)natiles64 * 16);
+  if (ce == cudaSuccess) ce = up(o_atiles, atiles.data(), (size_t)natiles * sizeof(int2));
+  if (ce == cudaSuccess) ce = up(o_stiles, stiles.data(), (size_t)nstiles * sizeof(int2));
   if (ce == cudaSuccess && coeff_scale) ce = up(o_scale, coeff_scale, (size_t)(lmax + 1) * (mmax + 1) * 8);
   if (ce == cudaSuccess) ce = up(o_tw, tw.data(), (size_t)nlon * 16);
   if (ce == cudaSuccess) ce = up(o_tw32, tw32.data(), (size_t)nlon * 8);
@@ -424,10 +423,10 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   dv.ckpt = (const double2*)(D + o_ck);
   dv.ckbase = (const int*)(D + o_ckbase);
   dv.ckstep = ckstep;
-  dv.atiles = (const int4*)(D + o_atiles);
-  dv.atiles64 = (const int4*)(D + o_atiles64);
+  dv.atiles = (const int2*)(D + o_atiles);
+  dv.stiles = (const int2*)(D + o_stiles);
   dv.natiles = natiles;
-  dv.natiles64 = natiles64;
+  dv.nstiles = nstiles;
   p->d_scale = coeff_scale ? (const double*)(D + o_scale) : nullptr;
   p->d_tw64 = (const double2*)(D + o_tw);
   p->d_tw32 = (const float2*)(D + o_tw32);

@@ -220,12 +220,19 @@ constexpr int kPU = 2 / NF;
 template <int NF>
 constexpr int kRing = NF == 1 ? 3 : 4;
 
+// A warp of the persistent kernel takes up to kMaxSegs consecutive segments: the ring runs on
+// into the next segment's first pairs while the sums of the current one cross the lanes (32
+// uneven transforms 652 -> 623 us). A single transform's warps take one: four made the CTAs
+// uneven (lmax 1023, one field 154 -> 183 us).
+constexpr int kMaxSegs = 4;
+
 template <typename C, int NF>
 struct Ring {   // one warp's slots
   double2 ck[kRing<NF>][kPU<NF>][32];
   C w[kRing<NF>][kPU<NF>][2 * NF][32];
   double x[kRing<NF>][kPU<NF>][32];
   int l0[kRing<NF>][kPU<NF>][32];
+  int p0[kMaxSegs];   // first pair of each segment of the warp
 };
 
 template <int BYTES>
@@ -234,50 +241,71 @@ __device__ __forceinline__ void cp_async(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(BYTES), "r"(n) : "memory");
 }
 
-template <typename C, int NF>
-__device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, const double* sal, Ring<C, NF>& R) {
+template <typename C, int NF, int MAXS>
+__device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, int nsegs, const double* sal0,
+                                             Ring<C, NF>& R) {
+  const int nseg = MAXS == 1 ? 1 : nsegs;
   constexpr int SG = kSeg<NF>, PU = kPU<NF>, RG = kRing<NF>;
   const PlanDev& P = a.P;
   const int lane = threadIdx.x & 31, npair = P.npair, m = im * P.mres;
   const long long poff = P.off[im];
-  const int cs = P.ckstep, ks = (lseg - m) / cs, roll = (lseg - m) - ks * cs;
-  const double2* ck = P.ckpt + (size_t)(P.ckbase[im] + ks) * npair;
+  const int cs = P.ckstep;
+  const double2* ck0 = P.ckpt + (size_t)P.ckbase[im] * npair;
   const int* pl0 = P.l0 + (size_t)im * npair;
   const C* W = (const C*)a.cin + (size_t)im * 2 * npair;
   const size_t wld = (size_t)P.nm * 2 * npair;
   const double* px = P.x;
   const int nf = a.nf;
+  // each segment's pairs start at the first block with a start below the segment's end
+  const int first = first_live_pair(pl0, npair, lseg0 + SG);
+  if constexpr (MAXS > 1) {
+    for (int j = 1; j < nseg; ++j) {
+      const int p = first_live_pair(pl0, npair, lseg0 + SG * (j + 1));
+      if (lane == 0) R.p0[j] = p;
+    }
+    __syncwarp();
+  }
+  int fs = 0, fp = first + lane, fq = 0;   // next segment, pair and slot to copy
+  auto fetch = [&]() {
+    if constexpr (MAXS > 1) {
+      while (fs < nseg && fp - lane >= npair) {
+        ++fs;
+        if (fs < nseg) fp = R.p0[fs] + lane;
+      }
+    }
+    if (MAXS == 1 || fs < nseg) {
+      const double2* ck = ck0 + (size_t)((lseg0 + SG * fs - m) / cs) * npair;
+#pragma unroll
+      for (int u = 0; u < PU; ++u) {
+        const int p = fp + 32 * u;
+        const bool ok = p < npair;
+        const int pc = ok ? p : 0;
+        cp_async<16>(&R.ck[fq][u][lane], ck + pc, ok);
+        cp_async<8>(&R.x[fq][u][lane], px + pc, ok);
+        cp_async<4>(&R.l0[fq][u][lane], pl0 + pc, ok);
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+          cp_async<sizeof(C)>(&R.w[fq][u][2 * k][lane], W + k * wld + pc, ok);
+          cp_async<sizeof(C)>(&R.w[fq][u][2 * k + 1][lane], W + k * wld + npair + pc, ok);
+        }
+      }
+      fp += 32 * PU;
+      fq = fq + 1 == RG ? 0 : fq + 1;
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < RG - 1; ++i) fetch();
+  int q = 0;
+  for (int seg = 0; seg < nseg; ++seg) {
+  const int lseg = lseg0 + SG * seg, roll = (lseg - m) % cs;
+  const double* sal = sal0 + SG * seg;
   double2 acc[SG][NF];
 #pragma unroll
   for (int s = 0; s < SG; ++s)
 #pragma unroll
     for (int k = 0; k < NF; ++k) acc[s][k] = make_double2(0.0, 0.0);
-  // pairs from the first block with a start below the segment's end
-  int p0 = first_live_pair(pl0, npair, lseg + SG);
-  int fp = p0 + lane, fq = 0;   // next pair and slot to copy
-  auto fetch = [&]() {
-#pragma unroll
-    for (int u = 0; u < PU; ++u) {
-      const int p = fp + 32 * u;
-      const bool ok = p < npair;
-      const int pc = ok ? p : 0;
-      cp_async<16>(&R.ck[fq][u][lane], ck + pc, ok);
-      cp_async<8>(&R.x[fq][u][lane], px + pc, ok);
-      cp_async<4>(&R.l0[fq][u][lane], pl0 + pc, ok);
-#pragma unroll
-      for (int k = 0; k < NF; ++k) {
-        cp_async<sizeof(C)>(&R.w[fq][u][2 * k][lane], W + k * wld + pc, ok);
-        cp_async<sizeof(C)>(&R.w[fq][u][2 * k + 1][lane], W + k * wld + npair + pc, ok);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    fp += 32 * PU;
-    fq = fq + 1 == RG ? 0 : fq + 1;
-  };
-#pragma unroll
-  for (int i = 0; i < RG - 1; ++i) fetch();
-  int q = 0;
-  for (; p0 < npair; p0 += 32 * PU) {
+  for (int p0 = seg == 0 ? first : R.p0[seg]; p0 < npair; p0 += 32 * PU) {
     fetch();
     asm volatile("cp.async.wait_group %0;\n" ::"n"(RG - 1) : "memory");
     double x[PU], ra[PU], rb[PU];
@@ -349,7 +377,6 @@ __device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, con
       }
     }
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy in flight past the segment
   // items i = s * NF + k; after the step with lane bit o, a lane keeps the half of its items
   // whose index has that bit as its lane number has
   double2 (&v)[SG * NF] = reinterpret_cast<double2 (&)[SG * NF]>(acc);
@@ -369,24 +396,26 @@ __device__ __forceinline__ void ana_segment(const Args& a, int im, int lseg, con
     C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
     narrow(*dst, make_double2(v[0].x * f, v[0].y * f));
   }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy in flight past the last segment
 }
 
-// CTA = four consecutive segments of one order, a warp each: blockIdx.y of NF parts of a
-// kAnaTile-degree tile.
+// CTA = four consecutive segments of one order, a warp each: blockIdx.y of NF parts of a tile of
+// kSimtTile degrees.
 template <typename C, int NF>
 __global__ void __launch_bounds__(128) ana_kernel(const __grid_constant__ Args a) {
   constexpr int ND = 4 * kSeg<NF>;
   __shared__ double sal[ND];
   __shared__ __align__(16) Ring<C, NF> ring[4];
   const PlanDev& P = a.P;
-  const int4 tile = P.atiles[blockIdx.x];
+  const int2 tile = P.stiles[blockIdx.x];
   const int im = tile.x, t0 = tile.y + ND * blockIdx.y, m = im * P.mres;
   if (m > a.mlim || t0 > a.lend) return;
   const long long poff = P.off[im];
   for (int i = threadIdx.x; i < ND; i += blockDim.x) sal[i] = (t0 + i <= a.lend) ? P.alpha[poff + (t0 + i - m)] : 0.0;
   __syncthreads();
   const int w = threadIdx.x >> 5, lseg = t0 + kSeg<NF> * w;
-  if (lseg <= a.lend) ana_segment<C, NF>(a, im, lseg, sal + kSeg<NF> * w, ring[w]);
+  if (lseg <= a.lend) ana_segments<C, NF, 1>(a, im, lseg, 1, sal + kSeg<NF> * w, ring[w]);
   if (a.zero_fill && t0 == m) {
     const int nrow = m + max(P.lmax - a.lcap, 0);   // rows [0, m) and (lcap, lmax]
     for (int idx = threadIdx.x; idx < nrow * a.nf; idx += blockDim.x) {
@@ -507,7 +536,7 @@ __global__ void __launch_bounds__(kThreads, 8) syn_group_kernel(const Args* __re
 }
 
 // Persistent analysis over the items of many transforms, one item per warp: item = (transform,
-// order, segment of kSeg degrees), list sorted by decreasing work and claimed by each warp from
+// order, first segment of kSeg degrees, segments), list sorted by decreasing work and claimed by each warp from
 // *queue. A segment's sums are those of ana_kernel, so the results are the same bit for bit. The
 // warp of an order's first segment clears the degrees below the order. done[t] receives the
 // largest %globaltimer value at which an item of transform t was stored.
@@ -516,16 +545,18 @@ struct GroupAnaWarp {
     Ring<float2, 1> r1;
     Ring<float2, 2> r2;
   };
-  double sal[32];
+  double sal[kMaxSegs * 32];
 };
 
 template <int NF>
-__device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, Ring<float2, NF>& R, double* sal) {
+__device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, int nseg, Ring<float2, NF>& R,
+                                              double* sal) {
   const int lane = threadIdx.x & 31, m = im * a.P.mres, lseg = m + kSeg<NF> * seg;
   __syncwarp();   // the previous item's alpha is read
-  if (lane < kSeg<NF>) sal[lane] = (lseg + lane <= a.lend) ? a.P.alpha[a.P.off[im] + (lseg + lane - m)] : 0.0;
+  for (int i = lane; i < nseg * kSeg<NF>; i += 32)
+    sal[i] = (lseg + i <= a.lend) ? a.P.alpha[a.P.off[im] + (lseg + i - m)] : 0.0;
   __syncwarp();
-  ana_segment<float2, NF>(a, im, lseg, sal, R);
+  ana_segments<float2, NF, kMaxSegs>(a, im, lseg, nseg, sal, R);
   if (seg == 0)
     for (int k = 0; k < a.nf; ++k) {
       float2* col = (float2*)a.out + (long long)k * a.ld_k + (long long)m * a.ld_m;
@@ -548,9 +579,9 @@ __global__ void __launch_bounds__(kThreads) ana_group_kernel(const Args* __restr
     const int4 it = items[i];
     const Args& a = targs[it.x];
     if (a.nf == 1)
-      ana_warp_item<1>(a, it.y, it.z, w.r1, w.sal);
+      ana_warp_item<1>(a, it.y, it.z, it.w, w.r1, w.sal);
     else
-      ana_warp_item<2>(a, it.y, it.z, w.r2, w.sal);
+      ana_warp_item<2>(a, it.y, it.z, it.w, w.r2, w.sal);
     __syncwarp();
     if (lane == 0) atomicMax(done + it.x, group_time());
   }
@@ -592,6 +623,15 @@ static int launch_syn(const shtb_plan* p, const sx::Args& a, int nmu, const char
   return SHTB_OK;
 }
 
+template <typename C, int NF>
+static int launch_ana(const shtb_plan* p, const sx::Args& a, const char* name, cudaStream_t st) {
+  static_assert(4 * sx::kSeg<NF> * NF == kSimtTile, "tile list of the plan");
+  prof_begin(st);
+  sx::ana_kernel<C, NF><<<dim3(p->dev.nstiles, NF), 128, 0, st>>>(a);
+  SHTB_LAUNCHED(name);
+  return SHTB_OK;
+}
+
 static Factors mixed_factors(const shtb_plan* p, int sc_mode) {
   return Factors{p->dev.cfac, p->d_scale, p->d_scale ? sc_mode : 0, 1.0, 1.0};
 }
@@ -618,13 +658,8 @@ int launch_simt_ana(const shtb_plan* p, const void* W, void* alm, int nf, int lt
   a.mlim = mlim;
   a.lcap = ltr;
   a.zero_fill = !packed;
-  prof_begin(st);
-  if (nf == 1)
-    sx::ana_kernel<float2, 1><<<p->dev.natiles, 128, 0, st>>>(a);
-  else
-    sx::ana_kernel<float2, 2><<<dim3(p->dev.natiles, 2), 128, 0, st>>>(a);
-  SHTB_LAUNCHED("simt legendre analysis kernel");
-  return SHTB_OK;
+  return nf == 1 ? launch_ana<float2, 1>(p, a, "simt legendre analysis kernel", st)
+                 : launch_ana<float2, 2>(p, a, "simt legendre analysis kernel", st);
 }
 
 // FP64 coefficients -> Fourier buffer for one or two fields.
@@ -649,13 +684,8 @@ int launch_simt_ana64(const shtb_plan* p, const void* W, int nf, int row_end, in
   a.mlim = mlim;
   a.lcap = dst.packed == 1 ? a.lend : std::min(a.lend, p->lmax);
   a.zero_fill = zero_fill && !dst.packed;
-  prof_begin(st);
-  if (nf == 1)
-    sx::ana_kernel<double2, 1><<<p->dev.natiles, 128, 0, st>>>(a);
-  else
-    sx::ana_kernel<double2, 2><<<dim3(p->dev.natiles, 2), 128, 0, st>>>(a);
-  SHTB_LAUNCHED("legendre analysis kernel");
-  return SHTB_OK;
+  return nf == 1 ? launch_ana<double2, 1>(p, a, "legendre analysis kernel", st)
+                 : launch_ana<double2, 2>(p, a, "legendre analysis kernel", st);
 }
 
 // ------------------------------------------------------------- grouped transforms
@@ -670,6 +700,11 @@ void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int 
 }
 
 int simt_ana_segment(int nf) { return nf == 1 ? sx::kSeg<1> : sx::kSeg<2>; }
+
+// Several once every warp slot (two per scheduler) has work for three rounds.
+int simt_ana_segments_per_warp(long long segs) {
+  return (int)std::max(1ll, std::min<long long>(sx::kMaxSegs, segs / (3 * 148 * 8)));
+}
 
 int simt_syn_pair_blocks(const shtb_plan* p) { return (p->npair + 31) / 32; }   // per-warp items of the group kernel
 
