@@ -55,7 +55,6 @@ struct shtb_group {
   unsigned char *d_sargs = nullptr, *d_sargs_ana = nullptr;
   int4 *d_items_ssyn = nullptr, *d_items_sana = nullptr;
   int n_ssyn = 0, ssyn_ctas = 148, n_sana = 0, sana_ctas = 148;
-  size_t ssyn_smem = 0;
   size_t argsz = 0, jobsz = 0, job2sz = 0;
   // device memory: [args syn | args ana | jobs syn | jobs ana | done | t0 | gemm items | W]
   unsigned char* dmem = nullptr;
@@ -180,8 +179,8 @@ static int group_synthesis_stage(shtb_group* g, int* q, cudaStream_t st) {
     SHTB_TRY_CUDA(cudaEventRecord(g->ev_fork, st), "group fork");
     SHTB_TRY_CUDA(cudaStreamWaitEvent(g->aux, g->ev_fork, 0), "group fork");
   }
-  if ((rc = launch_simt_group(g->d_sargs, g->d_items_ssyn, g->n_ssyn, g->ssyn_ctas, g->ssyn_smem, q + 7,
-                              g->d_t0, fork ? g->aux : st)))
+  if ((rc = launch_simt_group(g->d_sargs, g->d_items_ssyn, g->n_ssyn, g->ssyn_ctas, q + 7, g->d_t0,
+                              fork ? g->aux : st)))
     return rc;
   if ((rc = launch_pack_group(g->d_args_syn, g->d_items_pack, g->n_pack, std::min(g->n_pack, 24 * g->nsm), q, g->d_t0, st)))
     return rc;
@@ -307,7 +306,6 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
     if (!g->simt[t]) continue;
     const shtb_plan* p = plans[t];
     const int mlim = std::min(p->mmax, p->lmax);
-    g->ssyn_smem = std::max(g->ssyn_smem, simt_group_syn_smem(p));
     for (int im = 0; im <= mlim; ++im)
       for (int pb = 0; pb < simt_syn_pair_blocks(p); ++pb) {
         ssyn.push_back(make_int4(t, im, pb, 0));
@@ -396,7 +394,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   g->gemm_ctas_syn = std::max(1, std::min(2 * g->nsm, g->n_syn));
   g->gemm_ctas_ana = std::max(1, std::min(2 * g->nsm, g->n_ana));
   g->n_ssyn = (int)ssyn.size();
-  g->ssyn_ctas = std::max(1, std::min(8 * g->nsm, g->n_ssyn));   // 128-thread CTAs, several per SM
+  g->ssyn_ctas = std::max(1, std::min(4 * g->nsm, g->n_ssyn));   // 128-thread CTAs, four per SM
   g->n_sana = (int)sana.size();
   g->sana_ctas = std::max(1, std::min(2 * g->nsm, g->n_sana));   // 128-thread CTAs, two per SM
   g->sargsz = simt_args_bytes();

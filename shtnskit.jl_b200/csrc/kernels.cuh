@@ -140,9 +140,8 @@ void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int 
 int simt_ana_segment(int nf);   // degrees per segment of the grouped analysis
 int simt_ana_segments_per_warp(long long segs);   // segments per item, for that many segments in all
 int simt_syn_pair_blocks(const shtb_plan* p);
-size_t simt_group_syn_smem(const shtb_plan* p);
-int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, size_t smem, int* queue,
-                      unsigned long long* t0, cudaStream_t st);
+int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, int* queue, unsigned long long* t0,
+                      cudaStream_t st);
 int launch_simt_ana_group(const void* targs, const int4* items, int nitems, int grid, int* queue,
                           unsigned long long* done, cudaStream_t st);
 // the packed-pair FP32 FFTs of fft2_applicable members (2 HP latitude pairs per item)

@@ -76,19 +76,27 @@ __device__ __forceinline__ long long coef_base(const Args& a, long long poff, in
 template <int NF>
 constexpr int kChunk = 64 / NF;   // two coefficients per lane
 
+template <int NF, int UP>
+struct SynWarp {   // one warp's shared memory
+  double2 c[2][kChunk<NF> * NF];   // coefficients of two chunks
+  double2 s[UP][32];               // start states
+  double al[2][kChunk<NF>];
+};
+
+// Pairs 32 UP pb .. of order im.
 template <typename C, int NF, int UP>
-__global__ void __launch_bounds__(32) syn_kernel(const __grid_constant__ Args a) {
+__device__ __forceinline__ void syn_item(const Args& a, int im, int pb, SynWarp<NF, UP>& sw) {
   constexpr int CH = kChunk<NF>;
-  __shared__ double sAl[2][CH];
-  __shared__ __align__(16) double2 sC[2][CH * NF];
+  auto& sAl = sw.al;
+  auto& sC = sw.c;
+  auto& sS = sw.s;
   const PlanDev& P = a.P;
-  const int im = blockIdx.y, m = im * P.mres;
-  const int lane = threadIdx.x;
+  const int m = im * P.mres;
+  const int lane = threadIdx.x & 31;
   const int npair = P.npair, ndeg = a.lend - m + 1;
   const long long poff = P.off[im];
   const C* cin = (const C*)a.cin + coef_base(a, poff, m) + m;
-  const int pair0 = blockIdx.x * (32 * UP) + lane;
-  __shared__ double2 sS[UP][32];   // start states
+  const int pair0 = pb * (32 * UP) + lane;
   double x[UP], ra[UP], rb[UP];
   int l0[UP];
   int mn = INT_MAX / 2;   // first start of the warp's pairs, relative to m (a multiple of kStartStep)
@@ -198,6 +206,12 @@ __global__ void __launch_bounds__(32) syn_kernel(const __grid_constant__ Args a)
       narrow(w[npair], accO[u][k]);
     }
   }
+}
+
+template <typename C, int NF, int UP>
+__global__ void __launch_bounds__(32) syn_kernel(const __grid_constant__ Args a) {
+  __shared__ __align__(16) SynWarp<NF, UP> sw;
+  syn_item<C, NF, UP>(a, blockIdx.y, blockIdx.x, sw);
 }
 
 // -------------------------------------------------------------------------- analysis
@@ -425,101 +439,24 @@ __global__ void __launch_bounds__(128) ana_kernel(const __grid_constant__ Args a
   }
 }
 
-// Persistent kernel over the items of many transforms (uneven batches), one item per warp:
-// item = (transform, order index, block of 32 latitude pairs), list sorted by decreasing
-// work and claimed by each warp from the device counter *queue (zero at launch). A warp
-// stages its order's recurrence coefficients and FP64 coefficients in its own shared-memory
-// slice, kGroupChunk degrees at a time, so warps never wait for one another (a CTA-wide item
-// ends with a barrier at which the warps nearer the poles, which start at higher degrees,
-// wait for the others). Per latitude pair the arithmetic is that of syn_kernel, so the results
-// are the same bit for bit.
-constexpr int kGroupChunk = 128;
-constexpr size_t kGroupWarpDoubles = kGroupChunk + kGroupChunk * 2 * 2;   // alpha, then [degree][NF <= 2] double2
+// Persistent synthesis over the items of many transforms (uneven batches), one item per warp:
+// item = (transform, order index, block of 32 kGroupUP latitude pairs), list sorted by
+// decreasing work and claimed by each warp from the device counter *queue (zero at launch). An
+// item is one CTA's work of syn_kernel, so the results are the same bit for bit (two pairs per lane and
+// chunks fetched ahead: 32 uneven transforms 631 -> 602 us against one pair and a staging wait).
+constexpr int kGroupUP = 2;
+union GroupSynWarp {
+  SynWarp<1, kGroupUP> s1;
+  SynWarp<2, kGroupUP> s2;
+};
 
-template <int NF>
-__device__ __forceinline__ void syn_warp_item(const Args& a, int im, int pb, double* wsm) {
-  const PlanDev& P = a.P;
-  const int lane = threadIdx.x & 31;
-  const int m = im * P.mres;
-  const int lend = a.lend, ndeg = lend - m + 1;
-  const long long poff = P.off[im];
-  double* sAl = wsm;
-  double2* sC = reinterpret_cast<double2*>(wsm + kGroupChunk);
-  const int npair = P.npair, pair = pb * 32 + lane;
-  int l0 = INT_MAX / 2;
-  double x = 0.0, s0 = 0.0, s1 = 0.0;
-  if (pair < npair) {
-    x = P.x[pair];
-    l0 = P.l0[(size_t)im * npair + pair] - m;
-    const double2 v = P.start[(size_t)im * npair + pair];
-    s0 = v.x;
-    s1 = v.y;
-  }
-  const int dbeg = __reduce_min_sync(0xffffffffu, l0);   // first start, a multiple of kStartStep from m
-  const long long col = coef_base(a, poff, m);
-  double2 accE[NF], accO[NF];
-#pragma unroll
-  for (int k = 0; k < NF; ++k) accE[k] = accO[k] = make_double2(0.0, 0.0);
-  double ra = 0.0, rb = 0.0;
-  for (int d0 = dbeg; d0 < ndeg; d0 += kGroupChunk) {
-    const int nd = min(kGroupChunk, ndeg - d0);
-    __syncwarp();   // the previous chunk's values are read
-    // up to the next multiple of kStartStep, zeros past the order's last degree
-    const int nz = (nd + kStartStep - 1) & ~(kStartStep - 1);
-    for (int d = lane; d < nz; d += 32) sAl[d] = d < nd ? P.alpha[poff + d0 + d] : 0.0;
-    for (int i = lane; i < nz * NF; i += 32) {
-      const int d = i / NF, k = i - d * NF, l = m + d0 + d;
-      double2 v = make_double2(0.0, 0.0);
-      if (d < nd && k < a.nf) {
-        const float2 c = ((const float2*)a.cin)[(long long)k * a.ld_k + col + l];
-        double f = P.cfac[poff + d0 + d];
-        if (a.F.sc_mode) f *= a.F.sc[l + (long long)(P.lmax + 1) * m];
-        v = make_double2(c.x * f, c.y * f);
-      }
-      sC[i] = v;
-    }
-    __syncwarp();
-    auto step = [&](int d, double2 (&acc)[NF]) {
-      const double r = fma(sAl[d] * x, ra, -rb);
-      rb = ra;
-      ra = r;
-#pragma unroll
-      for (int k = 0; k < NF; ++k) {
-        const double2 c = sC[d * NF + k];
-        acc[k].x = fma(r, c.x, acc[k].x);
-        acc[k].y = fma(r, c.y, acc[k].y);
-      }
-    };
-    for (int g = 0; g < nd; g += kStartStep) {
-      if (l0 == d0 + g) {
-        ra = s0;
-        rb = s1;
-      }
-#pragma unroll
-      for (int d = 0; d < kStartStep; d += 2) {
-        step(g + d, accE);
-        step(g + d + 1, accO);
-      }
-    }
-  }
-  if (pair < npair) {
-#pragma unroll
-    for (int k = 0; k < NF; ++k) {
-      if (k >= a.nf) break;
-      float2* w = (float2*)a.out + (((size_t)k * P.nm + im) * 2) * npair + pair;
-      w[0] = make_float2((float)accE[k].x, (float)accE[k].y);
-      w[npair] = make_float2((float)accO[k].x, (float)accO[k].y);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kThreads, 8) syn_group_kernel(const Args* __restrict__ targs,
+__global__ void __launch_bounds__(kThreads, 4) syn_group_kernel(const Args* __restrict__ targs,
                                                                 const int4* __restrict__ items, int nitems,
                                                                 int* __restrict__ queue,
                                                                 unsigned long long* __restrict__ t0) {
-  extern __shared__ __align__(16) double smem[];
+  __shared__ __align__(16) GroupSynWarp sw[kThreads / 32];
   group_start(t0);
-  double* wsm = smem + (threadIdx.x >> 5) * kGroupWarpDoubles;
+  GroupSynWarp& w = sw[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   for (;;) {
     int i = 0;
@@ -528,10 +465,11 @@ __global__ void __launch_bounds__(kThreads, 8) syn_group_kernel(const Args* __re
     if (i >= nitems) break;
     const int4 it = items[i];
     const Args& a = targs[it.x];
+    __syncwarp();   // the previous item's shared memory is read
     if (a.nf == 1)
-      syn_warp_item<1>(a, it.y, it.z, wsm);
+      syn_item<float2, 1, kGroupUP>(a, it.y, it.z, w.s1);
     else
-      syn_warp_item<2>(a, it.y, it.z, wsm);
+      syn_item<float2, 2, kGroupUP>(a, it.y, it.z, w.s2);
   }
 }
 
@@ -706,16 +644,14 @@ int simt_ana_segments_per_warp(long long segs) {
   return (int)std::max(1ll, std::min<long long>(sx::kMaxSegs, segs / (3 * 148 * 8)));
 }
 
-int simt_syn_pair_blocks(const shtb_plan* p) { return (p->npair + 31) / 32; }   // per-warp items of the group kernel
+int simt_syn_pair_blocks(const shtb_plan* p) {   // per-warp items of the group kernel
+  return (p->npair + 32 * sx::kGroupUP - 1) / (32 * sx::kGroupUP);
+}
 
-size_t simt_group_syn_smem(const shtb_plan*) { return (sx::kThreads / 32) * sx::kGroupWarpDoubles * sizeof(double); }
-
-int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, size_t smem, int* queue,
-                      unsigned long long* t0, cudaStream_t st) {
+int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, int* queue, unsigned long long* t0,
+                      cudaStream_t st) {
   if (nitems <= 0) return SHTB_OK;
-  SHTB_TRY_CUDA(cudaFuncSetAttribute(sx::syn_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "simt group smem attr");
-  sx::syn_group_kernel<<<grid, sx::kThreads, smem, st>>>((const sx::Args*)targs, items, nitems, queue, t0);
+  sx::syn_group_kernel<<<grid, sx::kThreads, 0, st>>>((const sx::Args*)targs, items, nitems, queue, t0);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "simt group launch");
   return SHTB_OK;
