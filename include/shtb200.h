@@ -254,9 +254,9 @@ int shtb_synthesis_noalloc(const shtb_plan* plan, const void* alm, void* f, int 
  * Legendre stage) scalar transforms, each with its own plan (its own lmax, Gauss grid
  * and nlon) and 1..8 fields. No single counterpart in the reference, whose transforms
  * run one configuration per call (src/core_transforms.jl, src/batch_transforms.jl):
- * a group runs every member's tiles in one persistent launch per stage (B packing and
- * order-GEMM synthesis for members of three or more fields, the FP64-pipe synthesis for
- * one- or two-field members, FFT synthesis, FFT analysis, order-GEMM analysis), work items
+ * a group runs every member's tiles in one persistent launch per stage (B packing and the
+ * order GEMMs for members of three or more fields, the FP64-pipe synthesis and analysis for
+ * one- or two-field members, FFT synthesis, FFT analysis), work items
  * sorted by cost and claimed by the CTAs (or warps) from a device work counter, the stage
  * launches captured once in a CUDA graph and replayed.
  * Members must use lcap = lmax and mres = 1. Buffers (device pointers, per member):

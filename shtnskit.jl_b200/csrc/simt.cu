@@ -12,7 +12,7 @@
 //   analysis   lane = latitude pair, warp = a segment of degrees with their sums in registers;
 //              the sum over pairs crosses the lanes once, at the end
 // E and O (even and odd l - m) sums in FP64 on both paths. Measured at lmax 1023, one field
-// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 164 us against the 8-column MMA
+// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 154 us against the 8-column MMA
 // kernels; the FP64 pipes alone would take about 60 us each. Mixed path at lmax 511, one field:
 // the analysis GEMM, which streams 134 MB of P table for 2 columns, 41 us, this kernel 37 us.
 #include <climits>
@@ -236,7 +236,7 @@ constexpr int kRing = NF == 1 ? 3 : 4;
 
 // A warp of the persistent kernel takes up to kMaxSegs consecutive segments: the ring runs on
 // into the next segment's first pairs while the sums of the current one cross the lanes (32
-// uneven transforms 652 -> 623 us). A single transform's warps take one: four made the CTAs
+// uneven transforms 652 -> 631 us). A single transform's warps take one: four made the CTAs
 // uneven (lmax 1023, one field 154 -> 183 us).
 constexpr int kMaxSegs = 4;
 
@@ -312,104 +312,104 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
   for (int i = 0; i < RG - 1; ++i) fetch();
   int q = 0;
   for (int seg = 0; seg < nseg; ++seg) {
-  const int lseg = lseg0 + SG * seg, roll = (lseg - m) % cs;
-  const double* sal = sal0 + SG * seg;
-  double2 acc[SG][NF];
+    const int lseg = lseg0 + SG * seg, roll = (lseg - m) % cs;
+    const double* sal = sal0 + SG * seg;
+    double2 acc[SG][NF];
 #pragma unroll
-  for (int s = 0; s < SG; ++s)
+    for (int s = 0; s < SG; ++s)
 #pragma unroll
-    for (int k = 0; k < NF; ++k) acc[s][k] = make_double2(0.0, 0.0);
-  for (int p0 = seg == 0 ? first : R.p0[seg]; p0 < npair; p0 += 32 * PU) {
-    fetch();
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(RG - 1) : "memory");
-    double x[PU], ra[PU], rb[PU];
-    int l0[PU];
-    double2 E[PU][NF], O[PU][NF];
-    bool st = false;
-#pragma unroll
-    for (int u = 0; u < PU; ++u) {
-      x[u] = R.x[q][u][lane];
-      const double2 v = R.ck[q][u][lane];
-      ra[u] = v.x;
-      rb[u] = v.y;
-      l0[u] = R.l0[q][u][lane];   // 0 for pairs past the end: no start to look for
-      st |= l0[u] > lseg && l0[u] < lseg + SG;
-#pragma unroll
-      for (int k = 0; k < NF; ++k) {
-        E[u][k] = wide(R.w[q][u][2 * k][lane]);
-        O[u][k] = wide(R.w[q][u][2 * k + 1][lane]);
-      }
-    }
-    q = q + 1 == RG ? 0 : q + 1;
-    auto step = [&](int s, double al) {
+      for (int k = 0; k < NF; ++k) acc[s][k] = make_double2(0.0, 0.0);
+    for (int p0 = seg == 0 ? first : R.p0[seg]; p0 < npair; p0 += 32 * PU) {
+      fetch();
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(RG - 1) : "memory");
+      double x[PU], ra[PU], rb[PU];
+      int l0[PU];
+      double2 E[PU][NF], O[PU][NF];
+      bool st = false;
 #pragma unroll
       for (int u = 0; u < PU; ++u) {
-        const double r = fma(al * x[u], ra[u], -rb[u]);
-        rb[u] = ra[u];
-        ra[u] = r;
+        x[u] = R.x[q][u][lane];
+        const double2 v = R.ck[q][u][lane];
+        ra[u] = v.x;
+        rb[u] = v.y;
+        l0[u] = R.l0[q][u][lane];   // 0 for pairs past the end: no start to look for
+        st |= l0[u] > lseg && l0[u] < lseg + SG;
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
-          const double2 w = (s & 1) ? O[u][k] : E[u][k];
-          acc[s][k].x = fma(r, w.x, acc[s][k].x);
-          acc[s][k].y = fma(r, w.y, acc[s][k].y);
+          E[u][k] = wide(R.w[q][u][2 * k][lane]);
+          O[u][k] = wide(R.w[q][u][2 * k + 1][lane]);
         }
       }
-    };
-    if (!roll && !__any_sync(0xffffffffu, st)) {
-#pragma unroll
-      for (int s = 0; s < SG; ++s) step(s, sal[s]);
-    } else {
-      // a pair of the warp starts inside the segment, or the checkpoint lies below it
-      double2 v[PU];
-#pragma unroll
-      for (int u = 0; u < PU; ++u) {
-        const int p = p0 + 32 * u + lane;
-        v[u] = p < npair ? P.start[(size_t)im * npair + p] : make_double2(0.0, 0.0);
-      }
-      auto begin = [&](int l) {
-#pragma unroll
-        for (int u = 0; u < PU; ++u)
-          if (l == l0[u]) {
-            ra[u] = v[u].x;
-            rb[u] = v[u].y;
-          }
-      };
-      for (int l = lseg - roll; l < lseg; ++l) {
-        begin(l);
-        const double al = P.alpha[poff + (l - m)];
+      q = q + 1 == RG ? 0 : q + 1;
+      auto step = [&](int s, double al) {
 #pragma unroll
         for (int u = 0; u < PU; ++u) {
           const double r = fma(al * x[u], ra[u], -rb[u]);
           rb[u] = ra[u];
           ra[u] = r;
+#pragma unroll
+          for (int k = 0; k < NF; ++k) {
+            const double2 w = (s & 1) ? O[u][k] : E[u][k];
+            acc[s][k].x = fma(r, w.x, acc[s][k].x);
+            acc[s][k].y = fma(r, w.y, acc[s][k].y);
+          }
+        }
+      };
+      if (!roll && !__any_sync(0xffffffffu, st)) {
+#pragma unroll
+        for (int s = 0; s < SG; ++s) step(s, sal[s]);
+      } else {
+        // a pair of the warp starts inside the segment, or the checkpoint lies below it
+        double2 v[PU];
+#pragma unroll
+        for (int u = 0; u < PU; ++u) {
+          const int p = p0 + 32 * u + lane;
+          v[u] = p < npair ? P.start[(size_t)im * npair + p] : make_double2(0.0, 0.0);
+        }
+        auto begin = [&](int l) {
+#pragma unroll
+          for (int u = 0; u < PU; ++u)
+            if (l == l0[u]) {
+              ra[u] = v[u].x;
+              rb[u] = v[u].y;
+            }
+        };
+        for (int l = lseg - roll; l < lseg; ++l) {
+          begin(l);
+          const double al = P.alpha[poff + (l - m)];
+#pragma unroll
+          for (int u = 0; u < PU; ++u) {
+            const double r = fma(al * x[u], ra[u], -rb[u]);
+            rb[u] = ra[u];
+            ra[u] = r;
+          }
+        }
+#pragma unroll
+        for (int s = 0; s < SG; ++s) {
+          if (s % kStartStep == 0) begin(lseg + s);
+          step(s, sal[s]);
         }
       }
+    }
+    // items i = s * NF + k; after the step with lane bit o, a lane keeps the half of its items
+    // whose index has that bit as its lane number has
+    double2 (&v)[SG * NF] = reinterpret_cast<double2 (&)[SG * NF]>(acc);
 #pragma unroll
-      for (int s = 0; s < SG; ++s) {
-        if (s % kStartStep == 0) begin(lseg + s);
-        step(s, sal[s]);
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const double2 send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+        v[i].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, o);
+        v[i].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, o);
       }
     }
-  }
-  // items i = s * NF + k; after the step with lane bit o, a lane keeps the half of its items
-  // whose index has that bit as its lane number has
-  double2 (&v)[SG * NF] = reinterpret_cast<double2 (&)[SG * NF]>(acc);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < o; ++i) {
-      const double2 send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
-      v[i].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, o);
-      v[i].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, o);
+    const int l = lseg + lane / NF, k = lane % NF;
+    if (l <= a.lcap && k < nf) {
+      const double f = factor_at(a, poff, l, m);
+      C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
+      narrow(*dst, make_double2(v[0].x * f, v[0].y * f));
     }
-  }
-  const int l = lseg + lane / NF, k = lane % NF;
-  if (l <= a.lcap && k < nf) {
-    const double f = factor_at(a, poff, l, m);
-    C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
-    narrow(*dst, make_double2(v[0].x * f, v[0].y * f));
-  }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy in flight past the last segment
 }
@@ -442,8 +442,9 @@ __global__ void __launch_bounds__(128) ana_kernel(const __grid_constant__ Args a
 // Persistent synthesis over the items of many transforms (uneven batches), one item per warp:
 // item = (transform, order index, block of 32 kGroupUP latitude pairs), list sorted by
 // decreasing work and claimed by each warp from the device counter *queue (zero at launch). An
-// item is one CTA's work of syn_kernel, so the results are the same bit for bit (two pairs per lane and
-// chunks fetched ahead: 32 uneven transforms 631 -> 602 us against one pair and a staging wait).
+// item is one CTA's work of syn_kernel, so the results are the same bit for bit (two pairs per
+// lane and chunks fetched ahead: 32 uneven transforms 631 -> 602 us against one pair per lane
+// and a wait for each chunk).
 constexpr int kGroupUP = 2;
 union GroupSynWarp {
   SynWarp<1, kGroupUP> s1;
@@ -474,8 +475,8 @@ __global__ void __launch_bounds__(kThreads, 4) syn_group_kernel(const Args* __re
 }
 
 // Persistent analysis over the items of many transforms, one item per warp: item = (transform,
-// order, first segment of kSeg degrees, segments), list sorted by decreasing work and claimed by each warp from
-// *queue. A segment's sums are those of ana_kernel, so the results are the same bit for bit. The
+// order, first segment of kSeg degrees, segments), list sorted by decreasing work and claimed by
+// each warp from *queue. A segment's sums are those of ana_kernel, so the results are the same bit for bit. The
 // warp of an order's first segment clears the degrees below the order. done[t] receives the
 // largest %globaltimer value at which an item of transform t was stored.
 struct GroupAnaWarp {
