@@ -12,7 +12,7 @@
 //   analysis   lane = latitude pair, warp = a segment of degrees with their sums in registers;
 //              the sum over pairs crosses the lanes once, at the end
 // E and O (even and odd l - m) sums in FP64 on both paths. Measured at lmax 1023, one field
-// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 154 us against the 8-column MMA
+// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 152 us against the 8-column MMA
 // kernels; the FP64 pipes alone would take about 60 us each. Mixed path at lmax 511, one field:
 // the analysis GEMM, which streams 134 MB of P table for 2 columns, 41 us, this kernel 37 us.
 #include <climits>
@@ -215,30 +215,38 @@ __global__ void __launch_bounds__(32) syn_kernel(const __grid_constant__ Args a)
 }
 
 // -------------------------------------------------------------------------- analysis
-// a_l = sum over pairs of P_l(x_pair) W[pair]: a warp owns kSeg<NF> = 32 / NF consecutive degrees
-// of one order and holds their sums for every lane (kSeg x NF complex doubles = 128 registers);
-// lane = latitude pair, the warp walks the pairs 32 at a time. Per pair and segment the chain
+// a_l = sum over pairs of P_l(x_pair) W[pair]: kLanes lanes own a segment of kSeg<NF> = 32 / NF
+// consecutive degrees of one order and hold their sums in every lane (kSeg x NF complex doubles
+// = 128 registers); lane = latitude pair, a warp's kSplit consecutive segments (a span) walk the
+// pairs together, kLanes at a time, and share the lines they read. Per pair and segment the chain
 // starts from the plan's checkpoint and the pair's Fourier values stay in registers, so P
 // costs 2 FP64 operations and each field 2 more, with one broadcast load of alpha per degree.
 // The lanes' sums meet once, at the end, in a butterfly that halves the values each lane keeps
-// per step (62 adds for 64 sums) and leaves lane i with item i = (degree i / NF, field i % NF).
-// Pair blocks whose every pair starts above the segment are skipped while they lead.
+// per step and leaves lane j of a segment with items kSplit j .. (item i = degree i / NF, field
+// i % NF): 30 exchanges for two segments, 31 for one where a segment has all 32 lanes (32 uneven
+// transforms 602 -> 575 us, lmax 1023 and one field 156 -> 152 us).
+// Pair blocks whose every pair starts above the span are skipped while they lead.
 // Every lane copies its own operands of the next pairs into its slots of a shared-memory
 // ring (cp.async; only the lane itself reads them, so no barrier): the registers left beside
 // the sums allow two warps per scheduler, too few to cover the loads. A slot holds kPU<NF>
-// blocks of 32 pairs, summed together: one alpha load serves both, and their chains overlap.
+// blocks of kLanes pairs, summed together: one alpha load serves both, and their chains overlap.
 template <int NF>
 constexpr int kSeg = 32 / NF;
+constexpr int kLanes = 16, kSplit = 32 / kLanes;
+template <int NF>
+constexpr int kSpan = kSplit * kSeg<NF>;
+template <int NF>
+constexpr int kAlLd = kSeg<NF> + 1;   // stride of a segment's alpha in shared memory: segments of a warp in other banks
 template <int NF>
 constexpr int kPU = 2 / NF;
 template <int NF>
 constexpr int kRing = NF == 1 ? 3 : 4;
 
-// A warp of the persistent kernel takes up to kMaxSegs consecutive segments: the ring runs on
-// into the next segment's first pairs while the sums of the current one cross the lanes (32
+// A warp of the persistent kernel takes up to kMaxSegs consecutive spans: the ring runs on
+// into the next span's first pairs while the sums of the current one cross the lanes (32
 // uneven transforms 652 -> 631 us). A single transform's warps take one: four made the CTAs
-// uneven (lmax 1023, one field 154 -> 183 us).
-constexpr int kMaxSegs = 4;
+// uneven (lmax 1023, one field 154 -> 183 us, with 32 lanes a segment).
+constexpr int kMaxSegs = 2;
 
 template <typename C, int NF>
 struct Ring {   // one warp's slots
@@ -246,7 +254,7 @@ struct Ring {   // one warp's slots
   C w[kRing<NF>][kPU<NF>][2 * NF][32];
   double x[kRing<NF>][kPU<NF>][32];
   int l0[kRing<NF>][kPU<NF>][32];
-  int p0[kMaxSegs];   // first pair of each segment of the warp
+  int p0[kMaxSegs];   // first pair of each span of the warp
 };
 
 template <int BYTES>
@@ -259,9 +267,9 @@ template <typename C, int NF, int MAXS>
 __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, int nsegs, const double* sal0,
                                              Ring<C, NF>& R) {
   const int nseg = MAXS == 1 ? 1 : nsegs;
-  constexpr int SG = kSeg<NF>, PU = kPU<NF>, RG = kRing<NF>;
+  constexpr int SG = kSeg<NF>, SP = kSpan<NF>, PU = kPU<NF>, RG = kRing<NF>;
   const PlanDev& P = a.P;
-  const int lane = threadIdx.x & 31, npair = P.npair, m = im * P.mres;
+  const int lane = threadIdx.x & 31, h = lane / kLanes, j = lane % kLanes, npair = P.npair, m = im * P.mres;
   const long long poff = P.off[im];
   const int cs = P.ckstep;
   const double2* ck0 = P.ckpt + (size_t)P.ckbase[im] * npair;
@@ -270,29 +278,31 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
   const size_t wld = (size_t)P.nm * 2 * npair;
   const double* px = P.x;
   const int nf = a.nf;
-  // each segment's pairs start at the first block with a start below the segment's end
-  const int first = first_live_pair(pl0, npair, lseg0 + SG);
+  // each span's pairs start at the first block with a start below the span's end
+  const int first = first_live_pair(pl0, npair, lseg0 + SP);
   if constexpr (MAXS > 1) {
-    for (int j = 1; j < nseg; ++j) {
-      const int p = first_live_pair(pl0, npair, lseg0 + SG * (j + 1));
-      if (lane == 0) R.p0[j] = p;
+    for (int i = 1; i < nseg; ++i) {
+      const int p = first_live_pair(pl0, npair, lseg0 + SP * (i + 1));
+      if (lane == 0) R.p0[i] = p;
     }
     __syncwarp();
   }
-  int fs = 0, fp = first + lane, fq = 0;   // next segment, pair and slot to copy
+  int fs = 0, fp = first + j, fq = 0;   // next span, pair and slot to copy
   auto fetch = [&]() {
     if constexpr (MAXS > 1) {
-      while (fs < nseg && fp - lane >= npair) {
+      while (fs < nseg && fp - j >= npair) {
         ++fs;
-        if (fs < nseg) fp = R.p0[fs] + lane;
+        if (fs < nseg) fp = R.p0[fs] + j;
       }
     }
     if (MAXS == 1 || fs < nseg) {
-      const double2* ck = ck0 + (size_t)((lseg0 + SG * fs - m) / cs) * npair;
+      const int lf = lseg0 + SP * fs + SG * h;
+      const bool live = lf <= a.lend;   // the last span may hold one segment only
+      const double2* ck = live ? ck0 + (size_t)((lf - m) / cs) * npair : ck0;
 #pragma unroll
       for (int u = 0; u < PU; ++u) {
-        const int p = fp + 32 * u;
-        const bool ok = p < npair;
+        const int p = fp + kLanes * u;
+        const bool ok = live && p < npair;
         const int pc = ok ? p : 0;
         cp_async<16>(&R.ck[fq][u][lane], ck + pc, ok);
         cp_async<8>(&R.x[fq][u][lane], px + pc, ok);
@@ -303,7 +313,7 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
           cp_async<sizeof(C)>(&R.w[fq][u][2 * k + 1][lane], W + k * wld + npair + pc, ok);
         }
       }
-      fp += 32 * PU;
+      fp += kLanes * PU;
       fq = fq + 1 == RG ? 0 : fq + 1;
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -312,14 +322,14 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
   for (int i = 0; i < RG - 1; ++i) fetch();
   int q = 0;
   for (int seg = 0; seg < nseg; ++seg) {
-    const int lseg = lseg0 + SG * seg, roll = (lseg - m) % cs;
-    const double* sal = sal0 + SG * seg;
+    const int lseg = lseg0 + SP * seg + SG * h, roll = lseg <= a.lend ? (lseg - m) % cs : 0;
+    const double* sal = sal0 + kAlLd<NF> * (kSplit * seg + h);
     double2 acc[SG][NF];
 #pragma unroll
     for (int s = 0; s < SG; ++s)
 #pragma unroll
       for (int k = 0; k < NF; ++k) acc[s][k] = make_double2(0.0, 0.0);
-    for (int p0 = seg == 0 ? first : R.p0[seg]; p0 < npair; p0 += 32 * PU) {
+    for (int p0 = seg == 0 ? first : R.p0[seg]; p0 < npair; p0 += kLanes * PU) {
       fetch();
       asm volatile("cp.async.wait_group %0;\n" ::"n"(RG - 1) : "memory");
       double x[PU], ra[PU], rb[PU];
@@ -332,7 +342,7 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
         const double2 v = R.ck[q][u][lane];
         ra[u] = v.x;
         rb[u] = v.y;
-        l0[u] = R.l0[q][u][lane];   // 0 for pairs past the end: no start to look for
+        l0[u] = R.l0[q][u][lane];   // 0 for pairs past the end and dead segments: no start to look for
         st |= l0[u] > lseg && l0[u] < lseg + SG;
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
@@ -355,7 +365,7 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
           }
         }
       };
-      if (!roll && !__any_sync(0xffffffffu, st)) {
+      if (!__any_sync(0xffffffffu, st || roll)) {
 #pragma unroll
         for (int s = 0; s < SG; ++s) step(s, sal[s]);
       } else {
@@ -363,7 +373,7 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
         double2 v[PU];
 #pragma unroll
         for (int u = 0; u < PU; ++u) {
-          const int p = p0 + 32 * u + lane;
+          const int p = p0 + kLanes * u + j;
           v[u] = p < npair ? P.start[(size_t)im * npair + p] : make_double2(0.0, 0.0);
         }
         auto begin = [&](int l) {
@@ -392,44 +402,49 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
       }
     }
     // items i = s * NF + k; after the step with lane bit o, a lane keeps the half of its items
-    // whose index has that bit as its lane number has
+    // whose index has bit o * kSplit as its lane number has bit o
     double2 (&v)[SG * NF] = reinterpret_cast<double2 (&)[SG * NF]>(acc);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const bool up = lane & o;
+    for (int o = kLanes / 2; o > 0; o >>= 1) {
+      const bool up = j & o;
 #pragma unroll
-      for (int i = 0; i < o; ++i) {
-        const double2 send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      for (int i = 0; i < o * kSplit; ++i) {
+        const double2 send = up ? v[i] : v[i + o * kSplit], keep = up ? v[i + o * kSplit] : v[i];
         v[i].x = keep.x + __shfl_xor_sync(0xffffffffu, send.x, o);
         v[i].y = keep.y + __shfl_xor_sync(0xffffffffu, send.y, o);
       }
     }
-    const int l = lseg + lane / NF, k = lane % NF;
-    if (l <= a.lcap && k < nf) {
-      const double f = factor_at(a, poff, l, m);
-      C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
-      narrow(*dst, make_double2(v[0].x * f, v[0].y * f));
+#pragma unroll
+    for (int i = 0; i < kSplit; ++i) {
+      const int l = lseg + (j * kSplit + i) / NF, k = (j * kSplit + i) % NF;
+      if (l <= a.lcap && k < nf) {
+        const double f = factor_at(a, poff, l, m);
+        C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
+        narrow(*dst, make_double2(v[i].x * f, v[i].y * f));
+      }
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy in flight past the last segment
 }
 
-// CTA = four consecutive segments of one order, a warp each: blockIdx.y of NF parts of a tile of
-// kSimtTile degrees.
+// CTA = kAnaWarps consecutive spans of one order, a warp each: blockIdx.y of NF parts of a tile
+// of kSimtTile degrees.
+constexpr int kAnaWarps = 2;
 template <typename C, int NF>
-__global__ void __launch_bounds__(128) ana_kernel(const __grid_constant__ Args a) {
-  constexpr int ND = 4 * kSeg<NF>;
-  __shared__ double sal[ND];
-  __shared__ __align__(16) Ring<C, NF> ring[4];
+__global__ void __launch_bounds__(32 * kAnaWarps) ana_kernel(const __grid_constant__ Args a) {
+  constexpr int ND = kAnaWarps * kSpan<NF>, SG = kSeg<NF>;
+  __shared__ double sal[ND / SG * kAlLd<NF>];
+  __shared__ __align__(16) Ring<C, NF> ring[kAnaWarps];
   const PlanDev& P = a.P;
   const int2 tile = P.stiles[blockIdx.x];
   const int im = tile.x, t0 = tile.y + ND * blockIdx.y, m = im * P.mres;
   if (m > a.mlim || t0 > a.lend) return;
   const long long poff = P.off[im];
-  for (int i = threadIdx.x; i < ND; i += blockDim.x) sal[i] = (t0 + i <= a.lend) ? P.alpha[poff + (t0 + i - m)] : 0.0;
+  for (int i = threadIdx.x; i < ND; i += blockDim.x)
+    sal[i / SG * kAlLd<NF> + i % SG] = (t0 + i <= a.lend) ? P.alpha[poff + (t0 + i - m)] : 0.0;
   __syncthreads();
-  const int w = threadIdx.x >> 5, lseg = t0 + kSeg<NF> * w;
-  if (lseg <= a.lend) ana_segments<C, NF, 1>(a, im, lseg, 1, sal + kSeg<NF> * w, ring[w]);
+  const int w = threadIdx.x >> 5, lseg = t0 + kSpan<NF> * w;
+  if (lseg <= a.lend) ana_segments<C, NF, 1>(a, im, lseg, 1, sal + kAlLd<NF> * kSplit * w, ring[w]);
   if (a.zero_fill && t0 == m) {
     const int nrow = m + max(P.lmax - a.lcap, 0);   // rows [0, m) and (lcap, lmax]
     for (int idx = threadIdx.x; idx < nrow * a.nf; idx += blockDim.x) {
@@ -475,25 +490,25 @@ __global__ void __launch_bounds__(kThreads, 4) syn_group_kernel(const Args* __re
 }
 
 // Persistent analysis over the items of many transforms, one item per warp: item = (transform,
-// order, first segment of kSeg degrees, segments), list sorted by decreasing work and claimed by
-// each warp from *queue. A segment's sums are those of ana_kernel, so the results are the same bit for bit. The
-// warp of an order's first segment clears the degrees below the order. done[t] receives the
+// order, first span, spans), list sorted by decreasing work and claimed by
+// each warp from *queue. A span's sums are those of ana_kernel, so the results are the same bit for bit. The
+// warp of an order's first span clears the degrees below the order. done[t] receives the
 // largest %globaltimer value at which an item of transform t was stored.
 struct GroupAnaWarp {
   union {
     Ring<float2, 1> r1;
     Ring<float2, 2> r2;
   };
-  double sal[kMaxSegs * 32];
+  double sal[kMaxSegs * kSplit * kAlLd<1>];
 };
 
 template <int NF>
 __device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, int nseg, Ring<float2, NF>& R,
                                               double* sal) {
-  const int lane = threadIdx.x & 31, m = im * a.P.mres, lseg = m + kSeg<NF> * seg;
+  const int lane = threadIdx.x & 31, m = im * a.P.mres, lseg = m + kSpan<NF> * seg;
   __syncwarp();   // the previous item's alpha is read
-  for (int i = lane; i < nseg * kSeg<NF>; i += 32)
-    sal[i] = (lseg + i <= a.lend) ? a.P.alpha[a.P.off[im] + (lseg + i - m)] : 0.0;
+  for (int i = lane; i < nseg * kSpan<NF>; i += 32)
+    sal[i / kSeg<NF> * kAlLd<NF> + i % kSeg<NF>] = (lseg + i <= a.lend) ? a.P.alpha[a.P.off[im] + (lseg + i - m)] : 0.0;
   __syncwarp();
   ana_segments<float2, NF, kMaxSegs>(a, im, lseg, nseg, sal, R);
   if (seg == 0)
@@ -564,9 +579,9 @@ static int launch_syn(const shtb_plan* p, const sx::Args& a, int nmu, const char
 
 template <typename C, int NF>
 static int launch_ana(const shtb_plan* p, const sx::Args& a, const char* name, cudaStream_t st) {
-  static_assert(4 * sx::kSeg<NF> * NF == kSimtTile, "tile list of the plan");
+  static_assert(sx::kAnaWarps * sx::kSpan<NF> * NF == kSimtTile, "tile list of the plan");
   prof_begin(st);
-  sx::ana_kernel<C, NF><<<dim3(p->dev.nstiles, NF), 128, 0, st>>>(a);
+  sx::ana_kernel<C, NF><<<dim3(p->dev.nstiles, NF), 32 * sx::kAnaWarps, 0, st>>>(a);
   SHTB_LAUNCHED(name);
   return SHTB_OK;
 }
@@ -638,7 +653,7 @@ void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int 
   std::memcpy(host_args, &a, sizeof(a));
 }
 
-int simt_ana_segment(int nf) { return nf == 1 ? sx::kSeg<1> : sx::kSeg<2>; }
+int simt_ana_segment(int nf) { return nf == 1 ? sx::kSpan<1> : sx::kSpan<2>; }
 
 // Several once every warp slot (two per scheduler) has work for three rounds.
 int simt_ana_segments_per_warp(long long segs) {
