@@ -77,6 +77,13 @@ def is_julia_dense(t: torch.Tensor) -> bool:
     return True
 
 
+def _kernel_ready(t: torch.Tensor) -> bool:
+    """Whether a kernel may use ``t``'s memory as it lies: column-major, and the values themselves.
+    ``conj()`` of a complex tensor, and ``.imag`` of that, are views of unchanged memory with a
+    conjugate or negative bit that only torch's own operations apply."""
+    return is_julia_dense(t) and not t.is_conj() and not t.is_neg()
+
+
 _cuda_devices: dict = {}
 _no_guard = contextlib.nullcontext()
 
@@ -109,7 +116,7 @@ def to_device(x, dtype, device_index: int) -> torch.Tensor:
         x = torch.from_numpy(np.asfortranarray(x))
     if not isinstance(x, torch.Tensor):
         raise ArgumentError(f"unsupported operand type {type(x)}")
-    if x.device != dev or x.dtype != dtype or not is_julia_dense(x):
+    if x.device != dev or x.dtype != dtype or not _kernel_ready(x):
         out = julia_empty(x.shape, dtype, dev)
         out.copy_(x.to(dev) if x.dtype == dtype else x.to(dev).to(dtype))
         x = out
@@ -426,7 +433,7 @@ def _synthesis_impl(cfg, alm, batched, real_output, use_rfft, fft_scratch, lcap,
     if prec == _lib.SHTB_PREC_FP64 and a.requires_grad and torch.is_grad_enabled() and out is None:
         f = _Synthesis.apply(a if batched else a.unsqueeze(2), cfg, ltr)
         return f if batched else f[:, :, 0]
-    if out is None or out.dtype != rt or not is_julia_dense(out) or out.device != a.device:
+    if out is None or out.dtype != rt or not _kernel_ready(out) or out.device != a.device:
         f = julia_empty(_fields_shape(cfg.nlat, cfg.nlon, a), rt, a.device)
         synthesis_device(cfg, a, f, ltr, prec)
         if out is None:
@@ -721,21 +728,22 @@ def _spectral_op(name, op, cfg, src, out):
         raise ArgumentError(f"{name}: complex64 or complex128 coefficients expected")
     dev = _device_index(src) if out is None else _device_index(src, out)
     a = to_device(a, a.dtype, dev)
-    if out is None:
-        o = julia_empty(tuple(a.shape), a.dtype, a.device)
-    else:
-        o = out
-        if not isinstance(o, torch.Tensor) or not o.is_cuda or tuple(o.shape) != tuple(a.shape):
+    if out is not None:
+        if not isinstance(out, torch.Tensor) or not out.is_cuda or tuple(out.shape) != tuple(a.shape):
             raise DimensionMismatch(f"{name}: output dims")
-        if o.dtype != a.dtype or not is_julia_dense(o):
+        if out.dtype != a.dtype or not is_julia_dense(out):
             raise ArgumentError(f"{name}: output must be a column-major {a.dtype} device array")
+    o = out if out is not None and _kernel_ready(out) else julia_empty(tuple(a.shape), a.dtype, a.device)
     nf = a.shape[2] if a.dim() == 3 else 1
     plan = cfg.plan(dev)
     dcode = _lib.SHTB_F64 if a.dtype == torch.complex128 else _lib.SHTB_F32
     with _device_guard(dev):
         rc = _lib.load().shtb_spectral_op(plan.handle, op, _ptr(a), _ptr(o), nf, dcode, _stream(dev))
     _lib.check(rc, name)
-    return o
+    if out is None or o is out:
+        return o
+    out.copy_(o)
+    return out
 
 
 def divergence_from_spheroidal(cfg: SHTConfig, Slm):
