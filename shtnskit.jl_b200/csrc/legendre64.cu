@@ -50,6 +50,11 @@ __device__ __forceinline__ void cp8(void* smem, const void* gmem, unsigned src_b
                "l"(gmem), "r"(src_bytes)
                : "memory");
 }
+__device__ __forceinline__ void cp4(void* smem, const void* gmem, unsigned src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+               "l"(gmem), "r"(src_bytes)
+               : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait_group() {
@@ -315,21 +320,49 @@ int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, v
 // the B operand of step s as it comes, for MT tiles of 8 fields: no P panel, no shared memory
 // and no barrier in the loop. Each step has its own accumulators (8 steps x MT x 4 doubles).
 // Four pairs take 8 chain steps (2 FP64 operations a lane) and 8 MT MMAs; the operands of
-// the next four (MT x 32 bytes of W, a checkpoint, x, the pair's first degree) load meanwhile.
+// the next four (MT x 32 bytes of W, a checkpoint, x) load meanwhile.
+// Where the checkpoint table does not fit its budget at 8 degrees, the checkpoints are farther
+// apart than these chains, and rolling each chain forward from the checkpoint below it costs
+// up to ckstep - 8 steps for the 8 that count (analysis of 64 fields: lmax 1799, ckstep 16, 26.4 ms; lmax
+// 2047, ckstep 32, 62.3 ms). So
+//   ckstep 16    chains have 16 steps (SL = 16, MT = 1: as many accumulators as SL = 8, MT = 2) and
+//                tiles 128 degrees; a pair may start in the middle of a chain. 13.2 ms.
+//   ckstep >= 32 (SPARSE) a lane rolls one chain from a checkpoint through all the tile's degrees up
+//                to the next one, for one of bg = 4 groups of four pairs, and leaves
+//                the states at every 8th degree in the ring slots of the bg steps to come: ckstep - 8
+//                roll steps per 32 chain steps of a lane. lmax 2047, 64 fields 22.3 ms, 3 fields 11.1 -> 3.4 ms.
 constexpr int kAnaThreads = 128;
 constexpr int kAnaSteps = 8;             // degrees per chain; 8 chains per tile
-constexpr int kAnaDeg = 8 * kAnaSteps;   // degrees per tile
-static_assert(kAnaDeg == kAnaTile, "tile list of the plan");
+static_assert(8 * kAnaSteps == kAnaTile && 16 * kAnaSteps == kSimtTile, "tile lists of the plan");
 constexpr int kAnaRing = 4;              // operand ring: steps of four pairs in flight, plus one
 
-template <int MT, int CG>
-__global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
+// Loads that stay where they are written, ahead of the step's MMAs.
+__device__ __forceinline__ double2 ld_here(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_here(const double* p) {
+  double v;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int ld_here(const int* p) {
+  int v;
+  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+template <int MT, int CG, int SL, bool SPARSE>
+__global__ void __launch_bounds__(kAnaThreads, MT * SL == 16 ? 2 : 3)
     leg_ana64_kernel(PlanDev P, const double2* __restrict__ W, int nf, int row_end, int mlim, CoefSink dst, Factors F,
                      int zero_fill) {
-  constexpr int SL = kAnaSteps, KS = 4 / CG;
+  constexpr int KS = 4 / CG, DEG = 8 * SL;
+  static_assert(SL == kAnaSteps || (SL == 2 * kAnaSteps && MT == 1 && !SPARSE), "chains");
   __shared__ __align__(16) unsigned char buf[4 * kAnaRing * ((2 * MT + 1) * 512 + 256)];
-  static_assert((KS - 1) * CG * SL * 4 * 32 * 8 <= sizeof(buf), "partial sums");
-  const int2 tile = P.atiles[blockIdx.x];
+  __shared__ int sl0[SL > kStartStep ? 4 * kAnaRing * 32 : 1];   // start degrees, long chains only
+  static_assert((KS - 1) * CG * kAnaSteps * 4 * 32 * 8 <= sizeof(buf), "partial sums");
+  const int2 tile = (SL == kAnaSteps ? P.atiles : P.stiles)[blockIdx.x];
   const int im = tile.x, t0 = tile.y, m = im * P.mres;
   const int lend = min(row_end, P.lrec);
   if (m > mlim || t0 > lend) return;
@@ -340,11 +373,13 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
   const int kb = blockIdx.y * (8 * MT * CG);            // the CTA's first field
   const int kf0 = kb + 8 * MT * cg + g;                 // this lane's field of tile 0
   const int lg = t0 + SL * g;                           // first degree of this lane's chain
-  const int tlast = min(t0 + kAnaDeg - 1, lend);
-  // this lane's chain: checkpoint, degrees from it to lg, alpha of its steps
-  const int cs = P.ckstep;
-  const int ks = (min(lg, P.lrec) - m) / cs, nroll = lg <= P.lrec ? lg - m - ks * cs : 0;
-  const int mroll = __reduce_max_sync(0xffffffffu, nroll);
+  const int tlast = min(t0 + DEG - 1, lend);
+  // this lane's chain: its checkpoint, or (SPARSE) that of the chain it rolls from degree lk for
+  // the degrees lr .. lr + seg - 1, for group rg of bg groups of pairs; alpha of its steps
+  const int cs = SPARSE ? P.ckstep : SL;
+  const int bg = SPARSE ? kAnaRing : 1, rg = g & (bg - 1), seg = min(cs, DEG);
+  const int lr = SPARSE ? t0 + seg * (g / bg) : lg;
+  const int ks = (min(lr, P.lrec) - m) / cs, lk = lr <= P.lrec ? m + ks * cs : lr;
   const double2* ck = P.ckpt + (size_t)(P.ckbase[im] + ks) * npair;
   const int* pl0 = P.l0 + (size_t)im * npair;
   double al[SL];
@@ -378,8 +413,9 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
     const unsigned n = p < npair ? 16u : 0u;
     const int pc = p < npair ? p : 0;
     double2* r = ring + st * (NS * 32);
-    cp16(r, ck + pc, n);
+    if constexpr (!SPARSE) cp16(r, ck + pc, n);
     cp8(xring + st * 32, P.x + pc, n >> 1);
+    if constexpr (SL > kStartStep) cp4(sl0 + (warp * RG + st) * 32 + lane, pl0 + pc, n >> 2);
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
       cp16(r + (1 + 2 * i) * 32, Wi[i] + pc, n);
@@ -392,9 +428,49 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
     cp_commit();
   }
   int st = 0;
+  // SPARSE: checkpoint, x and start degree of the next chain to roll; zeros past the last pair and degree
+  double2 rc = make_double2(0.0, 0.0);
+  double rx = 0.0;
+  int rl0 = INT_MAX, rp = 0;
+  auto roll_fetch = [&](int k) {
+    rp = 4 * (k + rg * KS) + t;
+    rc = make_double2(0.0, 0.0);
+    rx = 0.0;
+    rl0 = INT_MAX;
+    if (rp < npair && lr <= P.lrec) {
+      rc = ld_here(ck + rp);
+      rx = ld_here(P.x + rp);
+      rl0 = ld_here(pl0 + rp);
+    }
+  };
+  if constexpr (SPARSE) roll_fetch(k0 + kw);   // ckstep >= 8 kAnaRing
   for (int k = k0 + kw; k < nk; k += KS) {
     fetch(k + (RG - 1) * KS, st == 0 ? RG - 1 : st - 1);
     cp_commit();
+    if constexpr (SPARSE) {
+      if (st == 0) {
+        // the states of the next bg steps, into their ring slots
+        double2* slot = ring - lane + rg * (NS * 32) + t;
+        __syncwarp();   // the slots are read
+        for (int l = lk;;) {
+          if (l == rl0) rc = P.start[(size_t)im * npair + rp];   // starts lie multiples of 8 degrees from m
+          if (l >= lr && lr < t0 + DEG) slot[(l - t0) / SL * 4] = rc;
+          if (l + SL >= lr + seg) break;
+          double a[SL];
+#pragma unroll
+          for (int s = 0; s < SL; ++s) a[s] = l + s <= P.lrec ? P.alpha[poff + (l + s - m)] : 0.0;
+#pragma unroll
+          for (int s = 0; s < SL; ++s) {
+            const double q = fma(a[s] * rx, rc.x, -rc.y);
+            rc.y = rc.x;
+            rc.x = q;
+          }
+          l += SL;
+        }
+        __syncwarp();
+        roll_fetch(k + bg * KS);
+      }
+    }
     cp_wait_group<RG - 1>();
     const double2* r = ring + st * (NS * 32);
     const double x = xring[st * 32];
@@ -405,30 +481,15 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
       e[i] = r[(1 + 2 * i) * 32];
       o[i] = r[(2 + 2 * i) * 32];
     }
+    const int l0 = SL > kStartStep ? sl0[(warp * RG + st) * 32 + lane] : 0;   // 0 past the last pair
     st = st == RG - 1 ? 0 : st + 1;
-    if (mroll) {
-      // checkpoints sparser than the chains: roll forward, past the pair's start if it lies between
-      double2 s0 = make_double2(0.0, 0.0);
-      int l0 = INT_MAX;
-      if (4 * k + t < npair) {
-        s0 = P.start[(size_t)im * npair + 4 * k + t];
-        l0 = pl0[4 * k + t];
-      }
-      for (int i = 0; i <= mroll; ++i) {
-        const int l = lg - nroll + i;
-        if (i > nroll) continue;
-        if (l == l0) {
-          ra = s0.x;
-          rb = s0.y;
-        }
-        if (i == nroll) continue;   // the state before lg
-        const double q = fma(P.alpha[poff + (l - m)] * x, ra, -rb);
-        rb = ra;
-        ra = q;
-      }
-    }
 #pragma unroll
     for (int s = 0; s < SL; ++s) {
+      if (SL > kStartStep && s == kStartStep && l0 == lg + s) {   // the pair starts inside the chain
+        const double2 v = P.start[(size_t)im * npair + 4 * k + t];
+        ra = v.x;
+        rb = v.y;
+      }
       const double q = fma(al[s] * x, ra, -rb);
       rb = ra;
       ra = q;
@@ -442,23 +503,24 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
     double* part = reinterpret_cast<double*>(buf);
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-      if (i > 0) __syncthreads();
+    for (int c = 0; c < MT * SL / kAnaSteps; ++c) {   // eight steps of one row tile at a time
+      const int i = c % MT, s0 = c / MT * kAnaSteps;
+      if (c > 0) __syncthreads();
       if (kw > 0) {
-        double* d = part + ((kw - 1) * CG + cg) * SL * 4 * 32 + lane;
+        double* d = part + ((kw - 1) * CG + cg) * kAnaSteps * 4 * 32 + lane;
 #pragma unroll
-        for (int s = 0; s < SL; ++s)
+        for (int s = 0; s < kAnaSteps; ++s)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) d[(s * 4 + q) * 32] = acc[s][i][q];
+          for (int q = 0; q < 4; ++q) d[(s * 4 + q) * 32] = acc[s0 + s][i][q];
       }
       __syncthreads();
       if (kw == 0)
         for (int w = 0; w < KS - 1; ++w) {
-          const double* d = part + (w * CG + cg) * SL * 4 * 32 + lane;
+          const double* d = part + (w * CG + cg) * kAnaSteps * 4 * 32 + lane;
 #pragma unroll
-          for (int s = 0; s < SL; ++s)
+          for (int s = 0; s < kAnaSteps; ++s)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[s][i][q] += d[(s * 4 + q) * 32];
+            for (int q = 0; q < 4; ++q) acc[s0 + s][i][q] += d[(s * 4 + q) * 32];
         }
     }
   }
@@ -490,24 +552,38 @@ __global__ void __launch_bounds__(kAnaThreads, MT == 2 ? 2 : 3)
   }
 }
 
-template <int MT, int CG>
+template <int MT, int CG, int SL, bool SPARSE>
 static int launch_ana_tile(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                            const Factors& F, int zero_fill, cudaStream_t st) {
-  const dim3 grid(p->dev.natiles, (nf + 8 * MT * CG - 1) / (8 * MT * CG));
+  const dim3 grid(SL == kAnaSteps ? p->dev.natiles : p->dev.nstiles, (nf + 8 * MT * CG - 1) / (8 * MT * CG));
   prof_begin(st);
-  leg_ana64_kernel<MT, CG><<<grid, kAnaThreads, 0, st>>>(p->dev, (const double2*)W, nf, row_end, mlim, dst, F, zero_fill);
+  leg_ana64_kernel<MT, CG, SL, SPARSE>
+      <<<grid, kAnaThreads, 0, st>>>(p->dev, (const double2*)W, nf, row_end, mlim, dst, F, zero_fill);
   SHTB_LAUNCHED("legendre analysis kernel");
   return SHTB_OK;
+}
+
+template <bool SPARSE>
+static int launch_ana_short(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
+                            const Factors& F, int zero_fill, cudaStream_t st) {
+  constexpr int SL = kAnaSteps;
+  if (nf > 32) return launch_ana_tile<2, 4, SL, SPARSE>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (nf > 16) return launch_ana_tile<2, 2, SL, SPARSE>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (nf > 8) return launch_ana_tile<2, 1, SL, SPARSE>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  return launch_ana_tile<1, 1, SL, SPARSE>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
 }
 
 int launch_leg_ana64(const shtb_plan* p, const void* W, int nf, int row_end, int mlim, const CoefSink& dst,
                      const Factors& F, int zero_fill, cudaStream_t st) {
   if (p->npair > 8192) return set_error(SHTB_ERR_UNSUPPORTED, "nlat too large for the FP64 analysis kernel");
   if (nf <= 2) return launch_simt_ana64(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 32) return launch_ana_tile<2, 4>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 16) return launch_ana_tile<2, 2>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  if (nf > 8) return launch_ana_tile<2, 1>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
-  return launch_ana_tile<1, 1>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  // chains as long as the checkpoints are apart, up to 16 degrees; beyond, chains of 8 that roll
+  if (p->dev.ckstep == kAnaSteps) return launch_ana_short<false>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (p->dev.ckstep > 2 * kAnaSteps) return launch_ana_short<true>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  constexpr int SL = 2 * kAnaSteps;
+  if (nf > 16) return launch_ana_tile<1, 4, SL, false>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  if (nf > 8) return launch_ana_tile<1, 2, SL, false>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
+  return launch_ana_tile<1, 1, SL, false>(p, W, nf, row_end, mlim, dst, F, zero_fill, st);
 }
 
 }  // namespace shtb

@@ -7,6 +7,7 @@ quarters), 32 (segments, lanes) and 64 (tiles, chunks). Bounds: the paths' own 1
 """
 import numpy as np
 import pytest
+import torch
 
 import shtb200 as sht
 from oracle import sht_oracle as so
@@ -75,12 +76,28 @@ def test_late_starts_and_two_row_tiles():
     assert rel_l2(sht.to_host(sht.analysis(cfg, one[0])), a[:, :, 0]) <= 1e-12
 
 
-@pytest.mark.parametrize("nf", [1, 3])
-def test_sparse_checkpoints(nf):
-    """lmax 2047: the checkpoint table exceeds its budget at 8 degrees, so chains roll forward
-    from sparser checkpoints. Roundtrip error grows with the number of degrees (7e-14 at 1023)."""
-    cfg = sht.create_gauss_config(2047, 2048, nlon=4096)
-    a = rand_alm(2047, 2047, nf, seed=5)
-    back = sht.to_host(sht.analysis_batch(cfg, sht.synthesis_batch(cfg, a)))
-    for k in range(nf):
-        assert rel_l2(back[:, :, k], a[:, :, k]) <= 1e-12
+@pytest.mark.parametrize("lmax", [1799, 2047, 2999, 3599], ids=["step16", "step32", "step64", "step128"])
+def test_sparse_checkpoints(lmax):
+    """Sizes at which the checkpoint table exceeds its budget (2 GiB) at 8 degrees, so that chains
+    are rolled forward from checkpoints 16, 32, 64 and 128 degrees apart: analyses of three or more
+    fields (every tile width), of two fields (segments of 16 degrees) from 32 on and of one field
+    (32 degrees) from 64 on. Roundtrip error grows with the number of degrees (7e-14 at 1023)."""
+    step = 8
+    while step < 128 and sum((lmax + 1 - m + step) // step for m in range(lmax + 1)) * ((lmax + 2) // 2) * 16 > 2 ** 31:
+        step *= 2
+    assert step == {1799: 16, 2047: 32, 2999: 64, 3599: 128}[lmax]
+    cfg = sht.create_gauss_config(lmax, lmax + 1, nlon=2 * lmax + 2)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    l = torch.arange(lmax + 1, device="cuda")
+    keep = (l[:, None] >= l[None, :]) / (l[:, None] + 1.0)
+    for nf in (1, 2, 3, 9, 17, 33):
+        a = sht.julia_empty((lmax + 1, lmax + 1, nf), torch.complex128, "cuda")
+        for k in range(nf):
+            z = torch.randn((lmax + 1, lmax + 1, 2), dtype=torch.float64, device="cuda", generator=g)
+            z[:, 0, 1] = 0
+            a[:, :, k] = torch.view_as_complex(z) * keep
+        back = sht.analysis_batch(cfg, sht.synthesis_batch(cfg, a))
+        for k in range(nf):
+            assert float((back[:, :, k] - a[:, :, k]).norm() / a[:, :, k].norm()) <= 1e-12, (nf, k)
+        del a, back, z
+    cfg.clear_plans()
