@@ -526,34 +526,59 @@ static FFTJob<T> fft_job(const shtb_plan* p, const int* perm, const typename V2<
   return J;
 }
 
+static size_t fft_smem(const FFTDesc& fd, size_t celem, int h) {
+  return (size_t)h * fft_row_stride(fd.n, fft_padsh(fd, celem)) * celem * (fd.big ? 2 : 1) + (size_t)h * 8 + 16;
+}
+
 // Latitude pairs and threads of a CTA. A CTA runs its loads, passes and stores one after the
-// other behind barriers, so an SM needs several CTAs in different phases: the registers
-// allow 512 threads an SM, here as two CTAs of 256 or four of 128 wherever rows are short
-// enough that a CTA still holds 4 or 8 pairs (grid runs of at least 16 bytes) at some 23 points
-// a thread. Measured, synthesis / analysis in us, against one CTA of 512 threads with the most
-// pairs that fit:
-//   FP32 nlon 1080, 64 fields 263 / 252 -> 254 / 242, 13 fields 84 / 78 -> 62 / 60;
-//   FP64 nlon 720, 20 fields 72 / 64 -> 64 / 60; nlon 512, 32 fields 31 / 41 -> 31 / 39;
-//   nlon 2048 keeps 4 pairs and 512 threads (211 / 256; 2 pairs and 256 threads 262 / 281).
-// Pairs are halved, down to 2 (4 for the B tile images, which are written 4 pairs at a time),
-// while the launch fills less than three quarters of the SMs' CTA slots: FP64 nlon 720,
-// 3 fields 23 / 23 -> 17 / 17; FP32 nlon 720, one field 41 / 29 -> 17 / 17.
+// other behind barriers, and the kernels' registers allow 512 threads an SM: one CTA of 512
+// threads with the most pairs whose rows fit (200 KB), or, so that phases overlap, two CTAs of
+// 256 threads with half the pairs each. Half the pairs also halve the runs in which the grid is
+// read and written, so two CTAs are taken where these keep 32 bytes, and for FP32 rows below 2048
+// points at 16 bytes too. Two CTAs against one, synthesis / analysis in us:
+//   FP32, 64 fields: nlon 360 52 / 47 -> 45 / 46, 1024 152 / 189 -> 138 / 170, 1080 344 / 326 -> 272 / 267,
+//     1620 (16 bytes) 875 / 697 -> 805 / 669, 2000 (16 bytes) 772 / 752 -> 718 / 714;
+//     at 16 bytes and 2048 points 586 / 713 -> 551 / 742, 2304 points 842 / 825 -> 859 / 858: one CTA;
+//   FP64: nlon 512, 64 fields 56 / 72 -> 53 / 68; 1080, 64 fields 461 / 422 -> 406 / 397;
+//     at 16 bytes and 1536 points, 24 fields 297 / 281 -> 315 / 287, 2048 points 316 / 381 -> 436 / 419: one CTA.
+// CTAs of 2048 points or fewer run with 128 threads, four an SM (FP64 nlon 256, 64 fields, 8 pairs:
+// 17 / 25 -> 15 / 21; 360 points 49 / 49 -> 51 / 58).
+// A small batch is split finer, down to 2 pairs (4 for runs of 16 bytes in FP32 rows of 1500 points or
+// more, and for the B tile images, which are written 4 pairs at a time): as long as all CTAs of an SM's
+// share still run at once (FP32 nlon 1080, one field 66 / 50 -> 24 / 19; FP64 nlon 720, 3 fields 23 / 25 ->
+// 17 / 19; FP64 nlon 1024, 3 fields, whose CTAs of 2 pairs would not, 29 / 33 against 19 / 27), and where
+// one CTA fills an SM, when it shortens the waves by a quarter (FP32 nlon 2700, 3 fields 88 / 84 -> 80 / 78).
+// CTAs that then have an SM each get 512 threads (FP32 nlon 2000, one field 27 / 29 -> 25 / 25).
+// Rows with a prime radix above 13 take up to 4 pairs and a thread for 23 or 24 points, so that its
+// pass keeps its wide sums (nlon 1018, 3 fields, FP64 146 us; 512 threads 189).
 struct FFTShape {
   int h, threads;
 };
 static FFTShape fft_shape(const FFTDesc& fd, size_t celem, int npair, int nfw, int wtile) {
   constexpr int kSMs = 148;
-  const size_t S = (size_t)fft_row_stride(fd.n, fft_padsh(fd, celem));
-  int h = (fd.n <= 760 && !fd.big) ? 8 : 4;
-  while (h > 1 && (size_t)h * S * celem * (fd.big ? 2 : 1) + 16 * 8 > 200 * 1024) h >>= 1;
-  int t = 64;
-  while (t < 512 && (celem == 16 ? 23 : 24) * t < h * fd.n) t <<= 1;
-  while (h > (wtile ? 4 : 2) && 4ll * ((npair + h - 1) / h) * nfw < 3ll * kSMs * (512 / t)) h >>= 1;
+  const bool f32 = celem == sizeof(float2);
+  int h = fd.big ? 4 : 16, t = 512, hmin = wtile ? 4 : 2;
+  while (h > 1 && fft_smem(fd, celem, h) > 200 * 1024) h >>= 1;
+  auto ctas = [&](int hh) { return ((npair + hh - 1ll) / hh) * nfw; };
+  if (fd.big) {
+    for (t = 64; t < 512 && (f32 ? 24 : 23) * t < h * fd.n;) t <<= 1;
+    while (h > hmin && 4 * ctas(h) < 3ll * kSMs * (512 / t)) h >>= 1;
+    return FFTShape{h, t};
+  }
+  const int run = h / 2 * (int)(celem / 2);   // bytes, with two CTAs
+  if (run >= 32 || (f32 && run == 16 && fd.n < 2048)) {
+    h >>= 1;
+    t = h * fd.n <= 2048 ? 128 : 256;
+    if (run == 16) hmin = 4;
+  }
+  // waves of CTAs of hh pairs: as many an SM as its threads and shared memory (1 KB more a CTA) hold
+  auto waves = [&](int hh) {
+    const long long slots = kSMs * std::min<long long>(512 / t, 227 * 1024 / (fft_smem(fd, celem, hh) + 1024));
+    return (ctas(hh) + slots - 1) / slots;
+  };
+  while (h > hmin && (t < 512 ? waves(h / 2) == 1 : 4 * waves(h / 2) <= 6 * waves(h))) h >>= 1;
+  if (t == 256 && ctas(h) <= kSMs) t = 512;
   return FFTShape{h, t};
-}
-
-static size_t fft_smem(const FFTDesc& fd, size_t celem, int h) {
-  return (size_t)h * fft_row_stride(fd.n, fft_padsh(fd, celem)) * celem * (fd.big ? 2 : 1) + (size_t)h * 8 + 16;
 }
 
 static bool fft_generic(const shtb_plan* p) {
