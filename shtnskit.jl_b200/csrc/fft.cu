@@ -811,8 +811,7 @@ static int launch_fft_group_h(int syn, const void* jobs, const int4* items, int 
                               int* queue, cudaStream_t st) {
   auto kern = syn ? fft_group_kernel<float, H, GENERIC, true> : fft_group_kernel<float, H, GENERIC, false>;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "group fft smem attr");
-  // two CTAs of 256 threads an SM (the launch shapes count such CTAs)
-  kern<<<grid, 256, smem, st>>>((const FFTJob<float>*)jobs, items, nitems, queue);
+  kern<<<grid, fft_group_threads(smem), smem, st>>>((const FFTJob<float>*)jobs, items, nitems, queue);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "group fft launch");
   return SHTB_OK;

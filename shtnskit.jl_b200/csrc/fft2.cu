@@ -595,7 +595,7 @@ int launch_fft2_group(int syn, const void* jobs, const int4* items, int nitems, 
   auto kern = syn ? f2::group_kernel<HP, true> : f2::group_kernel<HP, false>;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                 "group fft2 smem attr");
-  kern<<<grid, 64 * HP, smem, st>>>((const f2::Job*)jobs, items, nitems, queue);
+  kern<<<grid, fft_group_threads(smem), smem, st>>>((const f2::Job*)jobs, items, nitems, queue);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "group fft2 launch");
   return SHTB_OK;

@@ -293,7 +293,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
     f2items.swap(sorted);
   }
   g->n_fft2 = (int)f2items.size();
-  g->fft2_ctas = std::max(1, std::min(2 * g->nsm, g->n_fft2));   // CTAs of 256 threads, two per SM where rows fit
+  g->fft2_ctas = std::max(1, std::min(g->nsm * fft_group_ctas_per_sm(g->fft2_smem), g->n_fft2));
   // GEMM tiles with their live-chunk masks, most live K-steps first
   const int TM = mixed_group_tile_rows();
   std::vector<int4> syn, ana;
@@ -460,10 +460,14 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->ev_join, cudaEventDisableTiming);
   if (e != cudaSuccess) return fail(set_error(SHTB_ERR_CUDA, std::string("group setup: ") + cudaGetErrorString(e)));
-  // default FFT shape: the most latitude pairs per CTA that fit in ~200 KB
+  // default FFT shape: the most latitude pairs whose rows fit twice in an SM, if these are 8 or
+  // more (runs of 32 bytes), else the most that fit once in ~200 KB; as many CTAs as an SM holds
+  // (32 members of 2 fields 1030 us with 16 pairs and one CTA an SM, 989 with 8 and two)
   int h = 16;
-  while (h > 2 && group_fft_smem(g, h) > 200 * 1024) h >>= 1;
-  int rc = set_fft_shape(g, h, g->nsm);
+  while (h >= 8 && fft_group_ctas_per_sm(group_fft_smem(g, h)) < 2) h >>= 1;
+  if (h < 8)
+    for (h = 16; h > 2 && group_fft_smem(g, h) > 200 * 1024;) h >>= 1;
+  int rc = set_fft_shape(g, h, g->nsm * fft_group_ctas_per_sm(group_fft_smem(g, h)));
   if (rc) return fail(rc);
   *out = g;
   return SHTB_OK;

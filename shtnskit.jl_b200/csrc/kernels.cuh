@@ -110,6 +110,12 @@ __device__ __forceinline__ void group_start(unsigned long long* t0) {
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(t0, ~group_time());
 }
 #endif
+// CTAs an SM of the grouped FFT kernels: two of 256 threads where the rows of two fit its shared
+// memory (228 KB, less 1 KB and some static memory a CTA), else one of 512. The kernels' registers
+// allow 512 threads an SM; one CTA of 256 left half of them out (rows of 2048 points, 32 fields:
+// synthesis / analysis 226 / 236 us with 256 threads, 201 / 211 with 512).
+inline int fft_group_ctas_per_sm(size_t smem) { return 2 * (smem + 2048) <= 228 * 1024 ? 2 : 1; }
+inline int fft_group_threads(size_t smem) { return 512 / fft_group_ctas_per_sm(smem); }
 int mixed_prepare(const shtb_plan* p, cudaStream_t st);
 size_t mixed_args_bytes();
 void mixed_fill_args(const shtb_plan* p, int mode, const void* in, void* out, int nf, void* host_args);

@@ -111,6 +111,20 @@ def test_group_autotune_keeps_results():
     assert_same(b, grids, alms)
 
 
+@pytest.mark.parametrize("lmaxes,nfs", [([1023, 255], [1, 3]), ([2047, 100], [1, 3]), ([40, 30], [1, 4])],
+                         ids=["packed-2048", "general-4096", "short"])
+def test_group_row_lengths(lmaxes, nfs):
+    """The longest row decides the threads of a group's FFT kernels: two CTAs of 256 threads an SM
+    where their rows fit, else one of 512 (packed pairs of 2048 points, general rows of 4096)."""
+    cfgs, nfs = members(lmaxes, nfs)
+    b = UnevenBatch(cfgs, nfs)
+    fill(b, 400)
+    b.roundtrip()
+    torch.cuda.synchronize()
+    b.status()
+    assert_same(b, *per_member(b))
+
+
 def test_uneven_workload_sample():
     """32 members drawn like the uneven-batching workload (lmax uniform in 31..511, seed 7)."""
     rng = np.random.default_rng(7)
