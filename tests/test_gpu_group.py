@@ -24,9 +24,9 @@ def packed_pair_fft(cfg):
     return 64 <= n <= 2048 and (n & (n - 1)) == 0 and cfg.nlat % 4 == 0
 
 
-def fp64_pipe_synthesis(nf):
-    """The library's rule for the FP64-pipe Legendre synthesis of the mixed path (one or two
-    fields); other members run the packing and the tensor-core synthesis GEMM."""
+def fp64_pipes(nf):
+    """The library's rule for the FP64-pipe Legendre stage of the mixed path (one or two
+    fields); other members run the packing and the tensor-core GEMMs."""
     return nf <= 2
 
 
@@ -61,20 +61,27 @@ def assert_same(batch, grids, alms):
         assert torch.equal(batch.alm_out[t], alms[t]), f"coefficients of member {t} differ"
 
 
+def launches(cfgs, nfs):
+    """Kernels of one roundtrip: FP64-pipe synthesis and analysis (one- and two-field members),
+    packing and the two GEMMs (the others), one FFT kernel per direction and FFT kind."""
+    pipes = {fp64_pipes(k) for k in nfs}
+    return 2 * (True in pipes) + 3 * (False in pipes) + 2 * len({packed_pair_fft(c) for c in cfgs})
+
+
+def count_launches(run):
+    before = _lib.load().shtb_launch_count(0)
+    run()
+    torch.cuda.synchronize()
+    return _lib.load().shtb_launch_count(0) - before
+
+
 def test_group_matches_per_member_bitwise():
     lmaxes = [15, 31, 100, 47, 63, 127, 20, 255, 7, 80]
     cfgs, nfs = members(lmaxes, [1, 2, 1, 3, 1, 1, 2, 1, 1, 8])
     b = UnevenBatch(cfgs, nfs)
     host = fill(b, 100)
-    launches0 = _lib.load().shtb_launch_count(0)
-    b.roundtrip()
-    torch.cuda.synchronize()
-    # start marker; FP64-pipe synthesis (one- and two-field members); packing and synthesis
-    # GEMM (the others); one FFT kernel per direction and FFT kind; analysis GEMM (all)
-    kinds = len({packed_pair_fft(c) for c in cfgs})
-    synth = {fp64_pipe_synthesis(k) for k in nfs}
-    assert kinds == 2 and synth == {True, False}
-    assert _lib.load().shtb_launch_count(0) - launches0 == 1 + 1 + 2 + 2 * kinds + 1
+    assert launches(cfgs, nfs) == 9
+    assert count_launches(b.roundtrip) == 9
     b.status()
     grids, alms = per_member(b)
     assert_same(b, grids, alms)
@@ -95,6 +102,31 @@ def test_group_matches_per_member_bitwise():
     assert_same(b, grids, alms)
     lat = b.latencies_ns()
     assert np.all(lat > 0)
+
+
+@pytest.mark.parametrize("lmaxes,nfs", [([31, 63], [1, 2]), ([40, 47], [1, 2]), ([31, 63], [3, 8]), ([40, 47], [3, 8])],
+                         ids=["pipes-packed", "pipes-general", "gemm-packed", "gemm-general"])
+def test_group_launches_per_stage(lmaxes, nfs):
+    """Groups that lack one of the Legendre stages, or one of the FFT kinds."""
+    cfgs, nfs = members(lmaxes, nfs)
+    b = UnevenBatch(cfgs, nfs)
+    fill(b, 500)
+    assert count_launches(b.roundtrip) == launches(cfgs, nfs)
+    b.status()
+    assert_same(b, *per_member(b))
+
+
+def test_two_field_members_with_several_spans_per_warp():
+    """Enough spans of degrees (32 of two fields) that a warp of the grouped analysis takes two."""
+    lmaxes = [511, 500, 333]
+    assert sum((l + 1) * (l + 2) // 2 // 32 for l in lmaxes) >= 2 * 3 * 148 * 8
+    cfgs, nfs = members(lmaxes, [2, 2, 2])
+    b = UnevenBatch(cfgs, nfs)
+    fill(b, 600)
+    b.roundtrip()
+    torch.cuda.synchronize()
+    b.status()
+    assert_same(b, *per_member(b))
 
 
 def test_group_autotune_keeps_results():
