@@ -554,15 +554,16 @@ static size_t fft_smem(const FFTDesc& fd, size_t celem, int h) {
 struct FFTShape {
   int h, threads;
 };
-static FFTShape fft_shape(const FFTDesc& fd, size_t celem, int npair, int nfw, int wtile) {
-  constexpr int kSMs = 148;
+static FFTShape fft_shape(const shtb_plan* p, size_t celem, int nfw, int wtile) {
+  const FFTDesc& fd = p->fft;
+  const int npair = p->npair;
   const bool f32 = celem == sizeof(float2);
   int h = fd.big ? 4 : 16, t = 512, hmin = wtile ? 4 : 2;
   while (h > 1 && fft_smem(fd, celem, h) > 200 * 1024) h >>= 1;
   auto ctas = [&](int hh) { return ((npair + hh - 1ll) / hh) * nfw; };
   if (fd.big) {
     for (t = 64; t < 512 && (f32 ? 24 : 23) * t < h * fd.n;) t <<= 1;
-    while (h > hmin && 4 * ctas(h) < 3ll * kSMs * (512 / t)) h >>= 1;
+    while (h > hmin && 4 * ctas(h) < 3ll * p->nsm * (512 / t)) h >>= 1;
     return FFTShape{h, t};
   }
   const int run = h / 2 * (int)(celem / 2);   // bytes, with two CTAs
@@ -573,11 +574,11 @@ static FFTShape fft_shape(const FFTDesc& fd, size_t celem, int npair, int nfw, i
   }
   // waves of CTAs of hh pairs: as many an SM as its threads and shared memory (1 KB more a CTA) hold
   auto waves = [&](int hh) {
-    const long long slots = kSMs * std::min<long long>(512 / t, 227 * 1024 / (fft_smem(fd, celem, hh) + 1024));
+    const long long slots = p->nsm * std::min<long long>(512 / t, 227 * 1024 / (fft_smem(fd, celem, hh) + 1024));
     return (ctas(hh) + slots - 1) / slots;
   };
   while (h > hmin && (t < 512 ? waves(h / 2) == 1 : 4 * waves(h / 2) <= 6 * waves(h))) h >>= 1;
-  if (t == 256 && ctas(h) <= kSMs) t = 512;
+  if (t == 256 && ctas(h) <= p->nsm) t = 512;
   return FFTShape{h, t};
 }
 
@@ -632,7 +633,7 @@ int launch_fft_syn(const shtb_plan* p, const void* W, GT* out0, GT* out1, int nc
     if (ncomp == 1 && !use_w && !spow && fft2_applicable(p))
       return launch_fft2_syn(p, W, (float*)out0, nfw, mlim, gscale, st);
   }
-  const FFTShape s = fft_shape(p->fft, sizeof(typename V2<T>::type), p->npair, nfw, 0);
+  const FFTShape s = fft_shape(p, sizeof(typename V2<T>::type), nfw, 0);
   switch (s.h) {
     case 8: return launch_syn_h<T, 8>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, s.threads, st);
     case 4: return launch_syn_h<T, 4>(p, W, out0, out1, ncomp, nfw, mlim, gscale, use_w, spow, s.threads, st);
@@ -649,7 +650,7 @@ int launch_fft_ana(const shtb_plan* p, const GT* in0, const GT* in1, int ncomp, 
     if (ncomp == 1 && use_w && !spow && fft2_applicable(p))
       return launch_fft2_ana(p, (const float*)in0, W, nfw, mlim, wscale, wtile, st);
   }
-  const FFTShape s = fft_shape(p->fft, sizeof(typename V2<T>::type), p->npair, nfw, wtile);
+  const FFTShape s = fft_shape(p, sizeof(typename V2<T>::type), nfw, wtile);
   switch (s.h) {
     case 8: return launch_ana_h<T, 8>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, s.threads, st);
     case 4: return launch_ana_h<T, 4>(p, in0, in1, ncomp, W, nfw, mlim, wscale, use_w, spow, wtile, s.threads, st);

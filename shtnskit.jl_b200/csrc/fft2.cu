@@ -545,7 +545,7 @@ constexpr int kFft2HP = 4;
 // 29 / 31), as long as the launch still fills the SMs' 512 threads.
 static int fft2_threads(const shtb_plan* p, long long ctas) {
   int t = std::max(64, std::min(512, p->fft.n * kFft2HP / 16));
-  while (t < 512 && ctas * t < 148ll * 512) t <<= 1;
+  while (t < 512 && ctas * t < 512ll * p->nsm) t <<= 1;
   return t;
 }
 

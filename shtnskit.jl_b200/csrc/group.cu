@@ -315,7 +315,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   long long nsegs = 0;
   for (int t = 0; t < n; ++t)
     if (g->simt[t]) nsegs += plans[t]->hoff[plans[t]->nm] / simt_ana_segment(nfields[t]);
-  const int per_item = simt_ana_segments_per_warp(nsegs);
+  const int per_item = simt_ana_segments_per_warp(nsegs, g->nsm);
   for (int t = 0; t < n; ++t) {
     if (!g->simt[t]) continue;
     const shtb_plan* p = plans[t];

@@ -123,6 +123,7 @@ struct shtb_plan {
   int lmax, mmax, mres, nlat, nlon, nm, npair, lrec;
   int robert;
   int device;
+  int nsm = 148;                          // SMs of the device; launch shapes are chosen by it
   double phi_inv_scale, ana_scale;
   bool canonical;
   std::vector<double> hx, hw, hsint;

@@ -144,7 +144,7 @@ size_t simt_args_bytes();
 // syn: coefficients -> Fourier buffer, else Fourier buffer -> coefficients.
 void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int nf, void* host_args);
 int simt_ana_segment(int nf);   // degrees per segment of the grouped analysis
-int simt_ana_segments_per_warp(long long segs);   // segments per item, for that many segments in all
+int simt_ana_segments_per_warp(long long segs, int nsm);   // segments per item, for that many segments in all
 int simt_syn_pair_blocks(const shtb_plan* p);
 int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, int* queue, unsigned long long* t0,
                       cudaStream_t st);

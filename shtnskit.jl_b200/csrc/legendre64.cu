@@ -299,9 +299,9 @@ int launch_leg_syn64(const shtb_plan* p, const CoefSrc& src, const Factors& F, v
   // 32 columns a warp leave registers for four CTAs an SM, 64 for three: 2424 against 2536 us at
   // lmax 1023 x 64 fields, 57 against 62 at lmax 255 x 32 fields plus a wind field
   if (nf > 8) return launch_syn_tile<4, 1>(p, src, F, W, nf, row_end, mlim, st);
-  // narrower tiles: two row tiles per warp share each B fragment where that still leaves CTAs
-  // for every SM
-  const bool two = (long long)((p->npair + 127) / 128) * (mlim / p->mres + 1) >= 592;
+  // narrower tiles: two row tiles per warp share each B fragment where that still leaves four
+  // CTAs for every SM
+  const bool two = (long long)((p->npair + 127) / 128) * (mlim / p->mres + 1) >= 4ll * p->nsm;
   if (nf > 4)
     return two ? launch_syn_tile<2, 2>(p, src, F, W, nf, row_end, mlim, st)
                : launch_syn_tile<2, 1>(p, src, F, W, nf, row_end, mlim, st);

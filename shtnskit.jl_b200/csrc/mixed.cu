@@ -1459,13 +1459,6 @@ static int ensure_table(const shtb_plan* cp, cudaStream_t st) {
   return SHTB_OK;
 }
 
-static int sm_count() {
-  int dev = 0, n = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n;
-}
-
 // ntiles tiles per block of N/2 fields; persistent CTAs, at most the resident number.
 template <int MODE, int N>
 static int launch_gemm(const shtb_plan* p, const Args& a, int ntiles, int nz, cudaStream_t st) {
@@ -1473,7 +1466,7 @@ static int launch_gemm(const shtb_plan* p, const Args& a, int ntiles, int nz, cu
   const int smem = Smem<N>::kBytes;
   SHTB_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "mixed smem attr");
   const int total = ntiles * nz;
-  const int grid = std::max(1, std::min(total, sm_count() * kCtasPerSm<N>));
+  const int grid = std::max(1, std::min(total, p->nsm * kCtasPerSm<N>));
   prof_begin(st);
   kern<<<grid, kThreads<N>, smem, st>>>(a, total, nz);
   SHTB_LAUNCHED(MODE == 0 ? "tc gemm synthesis kernel" : "tc gemm analysis kernel");

@@ -284,6 +284,7 @@ extern "C" int shtb_plan_create(shtb_plan** out, int lmax, int mmax, int mres, i
   p->canonical = (coeff_scale == nullptr);
   if (coeff_scale) p->hscale.assign(coeff_scale, coeff_scale + (size_t)(lmax + 1) * (mmax + 1));
   cudaGetDevice(&p->device);
+  cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, p->device);
   factor_fft(nlon, p->fft);
 
   const int nm = p->nm, npair = p->npair, LR = p->lrec;

@@ -561,7 +561,7 @@ static sx::Args simt_args(const shtb_plan* p, const void* in, void* out, const F
 // SM a dozen warps, else one.
 static int syn_pairs_per_thread(const shtb_plan* p, int nmu) {
   const long long per32 = (long long)((p->npair + 31) / 32) * nmu;
-  return per32 / 2 >= 1776 ? 2 : 1;
+  return per32 / 2 >= 12ll * p->nsm ? 2 : 1;
 }
 
 template <typename C, int NF>
@@ -656,8 +656,8 @@ void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int 
 int simt_ana_segment(int nf) { return nf == 1 ? sx::kSpan<1> : sx::kSpan<2>; }
 
 // Several once every warp slot (two per scheduler) has work for three rounds.
-int simt_ana_segments_per_warp(long long segs) {
-  return (int)std::max(1ll, std::min<long long>(sx::kMaxSegs, segs / (3 * 148 * 8)));
+int simt_ana_segments_per_warp(long long segs, int nsm) {
+  return (int)std::max(1ll, std::min<long long>(sx::kMaxSegs, segs / (3ll * nsm * 8)));
 }
 
 int simt_syn_pair_blocks(const shtb_plan* p) {   // per-warp items of the group kernel
