@@ -396,7 +396,7 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
   g->n_ssyn = (int)ssyn.size();
   g->ssyn_ctas = std::max(1, std::min(4 * g->nsm, g->n_ssyn));   // 128-thread CTAs, four per SM
   g->n_sana = (int)sana.size();
-  g->sana_ctas = std::max(1, std::min(2 * g->nsm, g->n_sana));   // 128-thread CTAs, two per SM
+  g->sana_ctas = std::max(1, std::min(4 * g->nsm, g->n_sana));   // 64-thread CTAs, four per SM
   g->sargsz = simt_args_bytes();
   // one device allocation
   g->argsz = mixed_args_bytes();

@@ -9,12 +9,14 @@
 // start from the plan's start records (zeros below the start degree, a multiple of kStartStep
 // degrees from m, so starts are looked for once every kStartStep degrees).
 //   synthesis  lane = latitude pair; the sum over degrees stays in the lane
-//   analysis   lane = latitude pair, warp = a segment of degrees with their sums in registers;
-//              the sum over pairs crosses the lanes once, at the end
+//   analysis   lane = latitude pair, 16 lanes = a segment of degrees with their sums in registers,
+//              two segments a warp; the sum over pairs crosses the lanes once, at the end
 // E and O (even and odd l - m) sums in FP64 on both paths. Measured at lmax 1023, one field
-// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 152 us against the 8-column MMA
-// kernels; the FP64 pipes alone would take about 60 us each. Mixed path at lmax 511, one field:
-// the analysis GEMM, which streams 134 MB of P table for 2 columns, 41 us, this kernel 37 us.
+// (B200): FP64 synthesis 1236 -> 94 us, analysis 566 -> 135 us against the 8-column MMA
+// kernels; the FP64 pipes alone would take about 60 us each. Mixed path, against the analysis GEMM,
+// which streams 4 bytes a value of P (134 MB at lmax 511) for 2 or 4 columns and sums in FP32: lmax 511
+// one field 41 -> 31 us, two fields 37 -> 46; lmax 1023 160 -> 135 and 164 -> 222. Two fields keep
+// this kernel all the same: no P table, and FP64 sums (1.5e-7 from 64 bits at lmax 511, the GEMM 2.3e-7).
 #include <climits>
 #include <cstring>
 #include <type_traits>
@@ -228,8 +230,12 @@ __global__ void __launch_bounds__(32) syn_kernel(const __grid_constant__ Args a)
 // Pair blocks whose every pair starts above the span are skipped while they lead.
 // Every lane copies its own operands of the next pairs into its slots of a shared-memory
 // ring (cp.async; only the lane itself reads them, so no barrier): the registers left beside
-// the sums allow two warps per scheduler, too few to cover the loads. A slot holds kPU<NF>
-// blocks of kLanes pairs, summed together: one alpha load serves both, and their chains overlap.
+// the sums allow two warps per scheduler, too few to cover the loads. A slot holds kPU
+// blocks of kLanes pairs, summed together: one alpha load serves both, and their chains overlap
+// (two fields at lmax 1023 297 -> 247 us against one block). The addresses were most of the other
+// instructions (12 integer ones a copy): blocks that lie inside the rows are copied from pointers that
+// advance with them, and only the last block of a row, or a span that ends early, checks each
+// lane's pair (247 -> 222 us; one field 150 -> 135).
 template <int NF>
 constexpr int kSeg = 32 / NF;
 constexpr int kLanes = 16, kSplit = 32 / kLanes;
@@ -237,10 +243,8 @@ template <int NF>
 constexpr int kSpan = kSplit * kSeg<NF>;
 template <int NF>
 constexpr int kAlLd = kSeg<NF> + 1;   // stride of a segment's alpha in shared memory: segments of a warp in other banks
-template <int NF>
-constexpr int kPU = 2 / NF;
-template <int NF>
-constexpr int kRing = NF == 1 ? 3 : 4;
+constexpr int kPU = 2;
+constexpr int kRing = 3;
 
 // A warp of the persistent kernel takes up to kMaxSegs consecutive spans: the ring runs on
 // into the next span's first pairs while the sums of the current one cross the lanes (32
@@ -250,15 +254,23 @@ constexpr int kMaxSegs = 2;
 
 template <typename C, int NF>
 struct Ring {   // one warp's slots
-  double2 ck[kRing<NF>][kPU<NF>][32];
-  C w[kRing<NF>][kPU<NF>][2 * NF][32];
-  double x[kRing<NF>][kPU<NF>][32];
-  int l0[kRing<NF>][kPU<NF>][32];
+  struct Slot {
+    double2 ck[kPU][32];
+    C w[kPU][2 * NF][32];
+    double x[kPU][32];
+    int l0[kPU][32];
+  } s[kRing];
   int p0[kMaxSegs];   // first pair of each span of the warp
 };
 
 template <int BYTES>
-__device__ __forceinline__ void cp_async(void* dst, const void* src, bool ok) {
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+// Zeros unless ok; src is readable either way.
+template <int BYTES>
+__device__ __forceinline__ void cp_async_if(void* dst, const void* src, bool ok) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst), n = ok ? BYTES : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(BYTES), "r"(n) : "memory");
 }
@@ -267,7 +279,7 @@ template <typename C, int NF, int MAXS>
 __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, int nsegs, const double* sal0,
                                              Ring<C, NF>& R) {
   const int nseg = MAXS == 1 ? 1 : nsegs;
-  constexpr int SG = kSeg<NF>, SP = kSpan<NF>, PU = kPU<NF>, RG = kRing<NF>;
+  constexpr int SG = kSeg<NF>, SP = kSpan<NF>, PU = kPU, RG = kRing;
   const PlanDev& P = a.P;
   const int lane = threadIdx.x & 31, h = lane / kLanes, j = lane % kLanes, npair = P.npair, m = im * P.mres;
   const long long poff = P.off[im];
@@ -287,33 +299,61 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
     }
     __syncwarp();
   }
-  int fs = 0, fp = first + j, fq = 0;   // next span, pair and slot to copy
+  // next span, first pair of the next blocks and slot to copy; this lane's pointers into every row
+  int fs = 0, fb = first, fq = 0;
+  bool live = false, full = false;   // this lane's segment, every lane's segment holds degrees
+  const double2* gck;
+  const double* gx;
+  const int* gl;
+  const C* gw[2 * NF];
+  auto seek = [&](int span, int pair) {
+    const int lf = lseg0 + SP * span + SG * h;
+    live = lf <= a.lend;   // the last span may hold fewer segments
+    full = lseg0 + SP * span + SG * (kSplit - 1) <= a.lend;
+    fb = pair;
+    gck = (live ? ck0 + (size_t)((lf - m) / cs) * npair : ck0) + pair + j;
+    gx = px + pair + j;
+    gl = pl0 + pair + j;
+#pragma unroll
+    for (int r = 0; r < 2 * NF; ++r) gw[r] = W + (r >> 1) * wld + (r & 1) * npair + pair + j;
+  };
+  seek(0, first);
   auto fetch = [&]() {
     if constexpr (MAXS > 1) {
-      while (fs < nseg && fp - j >= npair) {
+      while (fs < nseg && fb >= npair) {
         ++fs;
-        if (fs < nseg) fp = R.p0[fs] + j;
+        if (fs < nseg) seek(fs, R.p0[fs]);
       }
     }
     if (MAXS == 1 || fs < nseg) {
-      const int lf = lseg0 + SP * fs + SG * h;
-      const bool live = lf <= a.lend;   // the last span may hold one segment only
-      const double2* ck = live ? ck0 + (size_t)((lf - m) / cs) * npair : ck0;
+      auto& S = R.s[fq];
+      if (full && fb + kLanes * PU <= npair) {
 #pragma unroll
-      for (int u = 0; u < PU; ++u) {
-        const int p = fp + kLanes * u;
-        const bool ok = live && p < npair;
-        const int pc = ok ? p : 0;
-        cp_async<16>(&R.ck[fq][u][lane], ck + pc, ok);
-        cp_async<8>(&R.x[fq][u][lane], px + pc, ok);
-        cp_async<4>(&R.l0[fq][u][lane], pl0 + pc, ok);
+        for (int u = 0; u < PU; ++u) {
+          cp_async<16>(&S.ck[u][lane], gck + kLanes * u);
+          cp_async<8>(&S.x[u][lane], gx + kLanes * u);
+          cp_async<4>(&S.l0[u][lane], gl + kLanes * u);
 #pragma unroll
-        for (int k = 0; k < NF; ++k) {
-          cp_async<sizeof(C)>(&R.w[fq][u][2 * k][lane], W + k * wld + pc, ok);
-          cp_async<sizeof(C)>(&R.w[fq][u][2 * k + 1][lane], W + k * wld + npair + pc, ok);
+          for (int r = 0; r < 2 * NF; ++r) cp_async<sizeof(C)>(&S.w[u][r][lane], gw[r] + kLanes * u);
+        }
+      } else if (fb < npair) {
+#pragma unroll
+        for (int u = 0; u < PU; ++u) {
+          const bool ok = live && fb + j + kLanes * u < npair;
+          const int d = ok ? kLanes * u : -(fb + j);   // else each row's first entry
+          cp_async_if<16>(&S.ck[u][lane], gck + d, ok);
+          cp_async_if<8>(&S.x[u][lane], gx + d, ok);
+          cp_async_if<4>(&S.l0[u][lane], gl + d, ok);
+#pragma unroll
+          for (int r = 0; r < 2 * NF; ++r) cp_async_if<sizeof(C)>(&S.w[u][r][lane], gw[r] + d, ok);
         }
       }
-      fp += kLanes * PU;
+      fb += kLanes * PU;
+      gck += kLanes * PU;
+      gx += kLanes * PU;
+      gl += kLanes * PU;
+#pragma unroll
+      for (int r = 0; r < 2 * NF; ++r) gw[r] += kLanes * PU;
       fq = fq + 1 == RG ? 0 : fq + 1;
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -336,18 +376,19 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
       int l0[PU];
       double2 E[PU][NF], O[PU][NF];
       bool st = false;
+      const auto& S = R.s[q];
 #pragma unroll
       for (int u = 0; u < PU; ++u) {
-        x[u] = R.x[q][u][lane];
-        const double2 v = R.ck[q][u][lane];
+        x[u] = S.x[u][lane];
+        const double2 v = S.ck[u][lane];
         ra[u] = v.x;
         rb[u] = v.y;
-        l0[u] = R.l0[q][u][lane];   // 0 for pairs past the end and dead segments: no start to look for
+        l0[u] = S.l0[u][lane];   // 0 for pairs past the end and dead segments: no start to look for
         st |= l0[u] > lseg && l0[u] < lseg + SG;
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
-          E[u][k] = wide(R.w[q][u][2 * k][lane]);
-          O[u][k] = wide(R.w[q][u][2 * k + 1][lane]);
+          E[u][k] = wide(S.w[u][2 * k][lane]);
+          O[u][k] = wide(S.w[u][2 * k + 1][lane]);
         }
       }
       q = q + 1 == RG ? 0 : q + 1;
@@ -518,11 +559,11 @@ __device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, in
     }
 }
 
-__global__ void __launch_bounds__(kThreads) ana_group_kernel(const Args* __restrict__ targs,
+__global__ void __launch_bounds__(32 * kAnaWarps) ana_group_kernel(const Args* __restrict__ targs,
                                                              const int4* __restrict__ items, int nitems,
                                                              int* __restrict__ queue,
                                                              unsigned long long* __restrict__ done) {
-  __shared__ __align__(16) GroupAnaWarp sw[kThreads / 32];
+  __shared__ __align__(16) GroupAnaWarp sw[kAnaWarps];
   GroupAnaWarp& w = sw[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   for (;;) {
@@ -676,7 +717,7 @@ int launch_simt_group(const void* targs, const int4* items, int nitems, int grid
 int launch_simt_ana_group(const void* targs, const int4* items, int nitems, int grid, int* queue,
                           unsigned long long* done, cudaStream_t st) {
   if (nitems <= 0) return SHTB_OK;
-  sx::ana_group_kernel<<<grid, sx::kThreads, 0, st>>>((const sx::Args*)targs, items, nitems, queue, done);
+  sx::ana_group_kernel<<<grid, 32 * sx::kAnaWarps, 0, st>>>((const sx::Args*)targs, items, nitems, queue, done);
   count_launch();
   SHTB_TRY_CUDA(cudaGetLastError(), "simt analysis group launch");
   return SHTB_OK;
