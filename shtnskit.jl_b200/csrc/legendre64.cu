@@ -124,6 +124,12 @@ __global__ void __launch_bounds__(kSynThreads, NT == 4 ? 4 : 1)
     const int p = blockIdx.x * (64 * MT) + i;
     s_start[i] = p < npair ? P.start[(size_t)im * npair + p] : make_double2(0.0, 0.0);
   }
+#pragma unroll 4
+  for (int i = tid; i < ndeg + SM::kPad; i += kSynThreads) {
+    const bool in = i < ndeg;
+    sAl[i] = in ? P.alpha[poff + i] : 0.0;
+    sFa[i] = in ? factor_at(P, F, poff, m + i, m) : 0.0;
+  }
   __syncthreads();
   mn = __reduce_min_sync(0xffffffffu, mn);
   if (lane == 0) atomicMin(&s_lmin, mn);
@@ -152,13 +158,6 @@ __global__ void __launch_bounds__(kSynThreads, NT == 4 ? 4 : 1)
     if (c < nch) stage(c, c);
     cp_commit();
   }
-#pragma unroll 4
-  for (int i = tid; i < ndeg + SM::kPad; i += kSynThreads) {
-    const bool in = i < ndeg;
-    sAl[i] = in ? P.alpha[poff + i] : 0.0;
-    sFa[i] = in ? factor_at(P, F, poff, m + i, m) : 0.0;
-  }
-  __syncthreads();
   // state before degree lq: the checkpoint at or below it, rolled forward
   {
     const int cs = P.ckstep;
@@ -360,6 +359,7 @@ __global__ void __launch_bounds__(kAnaThreads, MT * SL == 16 ? 2 : 3)
   constexpr int KS = 4 / CG, DEG = 8 * SL;
   static_assert(SL == kAnaSteps || (SL == 2 * kAnaSteps && MT == 1 && !SPARSE), "chains");
   __shared__ __align__(16) unsigned char buf[4 * kAnaRing * ((2 * MT + 1) * 512 + 256)];
+  __shared__ double s_fac[DEG];   // factors of the tile's degrees, loaded while the sums run
   __shared__ int sl0[SL > kStartStep ? 4 * kAnaRing * 32 : 1];   // start degrees, long chains only
   static_assert((KS - 1) * CG * kAnaSteps * 4 * 32 * 8 <= sizeof(buf), "partial sums");
   const int2 tile = (SL == kAnaSteps ? P.atiles : P.stiles)[blockIdx.x];
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kAnaThreads, MT * SL == 16 ? 2 : 3)
 
   // leading groups of 32 pairs that all start above the tile hold only zeros
   const int nk = (npair + 3) / 4;
-  const int k0 = first_live_pair(pl0, npair, tlast + 1) / 4;
+  const int k0 = npair <= 32 ? 0 : first_live_pair(pl0, npair, tlast + 1) / 4;
   // operand ring: each lane copies its own operands of the next RG - 1 steps (a checkpoint, x,
   // W of MT fields, E and O) and reads them back itself, so no barrier is needed
   constexpr int RG = kAnaRing, NS = 2 * MT + 1;
@@ -427,6 +427,9 @@ __global__ void __launch_bounds__(kAnaThreads, MT * SL == 16 ? 2 : 3)
     fetch(k0 + kw + i * KS, i);
     cp_commit();
   }
+  const int lcap = dst.packed == 1 ? lend : min(lend, P.lmax);
+  if (tid < DEG && t0 + tid <= lcap) s_fac[tid] = factor_at(P, F, poff, t0 + tid, m);
+  __syncthreads();
   int st = 0;
   // SPARSE: checkpoint, x and start degree of the next chain to roll; zeros past the last pair and degree
   double2 rc = make_double2(0.0, 0.0);
@@ -524,7 +527,6 @@ __global__ void __launch_bounds__(kAnaThreads, MT * SL == 16 ? 2 : 3)
         }
     }
   }
-  const int lcap = dst.packed == 1 ? lend : min(lend, P.lmax);
   if (kw == 0) {
     const long long dbase = dst.packed == 1 ? (poff - m)
                             : dst.packed == 2 ? lm_base(P.lmax, P.mres, m) : (long long)m * dst.ld_m;
@@ -535,7 +537,7 @@ __global__ void __launch_bounds__(kAnaThreads, MT * SL == 16 ? 2 : 3)
       for (int s = 0; s < SL; ++s) {
         const int l = t0 + SL * (2 * t + c) + s;
         if (l > lcap) continue;
-        const double f = factor_at(P, F, poff, l, m);
+        const double f = s_fac[l - t0];
 #pragma unroll
         for (int i = 0; i < MT; ++i)
           if (kf0 + 8 * i < nf)

@@ -291,7 +291,7 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
   const double* px = P.x;
   const int nf = a.nf;
   // each span's pairs start at the first block with a start below the span's end
-  const int first = first_live_pair(pl0, npair, lseg0 + SP);
+  const int first = npair <= 32 ? 0 : first_live_pair(pl0, npair, lseg0 + SP);
   if constexpr (MAXS > 1) {
     for (int i = 1; i < nseg; ++i) {
       const int p = first_live_pair(pl0, npair, lseg0 + SP * (i + 1));
