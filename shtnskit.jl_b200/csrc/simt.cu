@@ -263,6 +263,13 @@ struct Ring {   // one warp's slots
   int p0[kMaxSegs];   // first pair of each span of the warp
 };
 
+// Alpha and factors of a warp's spans: they load while its first operands do.
+template <int NF, int MAXS>
+struct SegTables {
+  double al[MAXS * kSplit * kAlLd<NF>];
+  double fac[MAXS * kSpan<NF>];
+};
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -276,7 +283,7 @@ __device__ __forceinline__ void cp_async_if(void* dst, const void* src, bool ok)
 }
 
 template <typename C, int NF, int MAXS>
-__device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, int nsegs, const double* sal0,
+__device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, int nsegs, SegTables<NF, MAXS>& T,
                                              Ring<C, NF>& R) {
   const int nseg = MAXS == 1 ? 1 : nsegs;
   constexpr int SG = kSeg<NF>, SP = kSpan<NF>, PU = kPU, RG = kRing;
@@ -360,10 +367,16 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
   };
 #pragma unroll
   for (int i = 0; i < RG - 1; ++i) fetch();
+  for (int i = lane; i < nseg * SP; i += 32) {
+    const int l = lseg0 + i;
+    T.al[i / SG * kAlLd<NF> + i % SG] = l <= a.lend ? P.alpha[poff + (l - m)] : 0.0;
+    if (l <= a.lcap) T.fac[i] = factor_at(a, poff, l, m);
+  }
+  __syncwarp();
   int q = 0;
   for (int seg = 0; seg < nseg; ++seg) {
     const int lseg = lseg0 + SP * seg + SG * h, roll = lseg <= a.lend ? (lseg - m) % cs : 0;
-    const double* sal = sal0 + kAlLd<NF> * (kSplit * seg + h);
+    const double* sal = T.al + kAlLd<NF> * (kSplit * seg + h);
     double2 acc[SG][NF];
 #pragma unroll
     for (int s = 0; s < SG; ++s)
@@ -459,7 +472,7 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
     for (int i = 0; i < kSplit; ++i) {
       const int l = lseg + (j * kSplit + i) / NF, k = (j * kSplit + i) % NF;
       if (l <= a.lcap && k < nf) {
-        const double f = factor_at(a, poff, l, m);
+        const double f = T.fac[l - lseg0];
         C* dst = (C*)a.out + (long long)k * a.ld_k + coef_base(a, poff, m) + l;
         narrow(*dst, make_double2(v[i].x * f, v[i].y * f));
       }
@@ -473,19 +486,15 @@ __device__ __forceinline__ void ana_segments(const Args& a, int im, int lseg0, i
 constexpr int kAnaWarps = 2;
 template <typename C, int NF>
 __global__ void __launch_bounds__(32 * kAnaWarps) ana_kernel(const __grid_constant__ Args a) {
-  constexpr int ND = kAnaWarps * kSpan<NF>, SG = kSeg<NF>;
-  __shared__ double sal[ND / SG * kAlLd<NF>];
+  constexpr int ND = kAnaWarps * kSpan<NF>;
+  __shared__ SegTables<NF, 1> tab[kAnaWarps];
   __shared__ __align__(16) Ring<C, NF> ring[kAnaWarps];
   const PlanDev& P = a.P;
   const int2 tile = P.stiles[blockIdx.x];
   const int im = tile.x, t0 = tile.y + ND * blockIdx.y, m = im * P.mres;
   if (m > a.mlim || t0 > a.lend) return;
-  const long long poff = P.off[im];
-  for (int i = threadIdx.x; i < ND; i += blockDim.x)
-    sal[i / SG * kAlLd<NF> + i % SG] = (t0 + i <= a.lend) ? P.alpha[poff + (t0 + i - m)] : 0.0;
-  __syncthreads();
   const int w = threadIdx.x >> 5, lseg = t0 + kSpan<NF> * w;
-  if (lseg <= a.lend) ana_segments<C, NF, 1>(a, im, lseg, 1, sal + kAlLd<NF> * kSplit * w, ring[w]);
+  if (lseg <= a.lend) ana_segments<C, NF, 1>(a, im, lseg, 1, tab[w], ring[w]);
   if (a.zero_fill && t0 == m) {
     const int nrow = m + max(P.lmax - a.lcap, 0);   // rows [0, m) and (lcap, lmax]
     for (int idx = threadIdx.x; idx < nrow * a.nf; idx += blockDim.x) {
@@ -540,18 +549,18 @@ struct GroupAnaWarp {
     Ring<float2, 1> r1;
     Ring<float2, 2> r2;
   };
-  double sal[kMaxSegs * kSplit * kAlLd<1>];
+  union {
+    SegTables<1, kMaxSegs> t1;
+    SegTables<2, kMaxSegs> t2;
+  };
 };
 
 template <int NF>
 __device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, int nseg, Ring<float2, NF>& R,
-                                              double* sal) {
+                                              SegTables<NF, kMaxSegs>& T) {
   const int lane = threadIdx.x & 31, m = im * a.P.mres, lseg = m + kSpan<NF> * seg;
-  __syncwarp();   // the previous item's alpha is read
-  for (int i = lane; i < nseg * kSpan<NF>; i += 32)
-    sal[i / kSeg<NF> * kAlLd<NF> + i % kSeg<NF>] = (lseg + i <= a.lend) ? a.P.alpha[a.P.off[im] + (lseg + i - m)] : 0.0;
-  __syncwarp();
-  ana_segments<float2, NF, kMaxSegs>(a, im, lseg, nseg, sal, R);
+  __syncwarp();   // the previous item's tables are read
+  ana_segments<float2, NF, kMaxSegs>(a, im, lseg, nseg, T, R);
   if (seg == 0)
     for (int k = 0; k < a.nf; ++k) {
       float2* col = (float2*)a.out + (long long)k * a.ld_k + (long long)m * a.ld_m;
@@ -574,9 +583,9 @@ __global__ void __launch_bounds__(32 * kAnaWarps) ana_group_kernel(const Args* _
     const int4 it = items[i];
     const Args& a = targs[it.x];
     if (a.nf == 1)
-      ana_warp_item<1>(a, it.y, it.z, it.w, w.r1, w.sal);
+      ana_warp_item<1>(a, it.y, it.z, it.w, w.r1, w.t1);
     else
-      ana_warp_item<2>(a, it.y, it.z, it.w, w.r2, w.sal);
+      ana_warp_item<2>(a, it.y, it.z, it.w, w.r2, w.t2);
     __syncwarp();
     if (lane == 0) atomicMax(done + it.x, group_time());
   }
