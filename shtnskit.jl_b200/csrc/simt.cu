@@ -70,25 +70,26 @@ __device__ __forceinline__ long long coef_base(const Args& a, long long poff, in
 // 32 lanes' registers (24 bytes a degree with alpha: 6 cycles of the SM's 128-byte path at one
 // field) while a pair's 4 FP64 operations take 2 cycles of its 64 units, so one pair per lane
 // is bound by those loads and four per lane by the FP64 units. The order's alpha and
-// coefficients (times the factors, in FP64) are staged kChunk<NF> degrees at a time in two
+// coefficients (times the factors, in FP64) are staged kChunk degrees at a time in two
 // buffers; the next chunk's values are in registers while the current one is summed. Warps
 // share nothing: the warps nearer the poles start at higher degrees, and in CTAs of four
 // warps the barrier of the shared staging made them wait for the others (148 us, 44 % of
 // the issue slots, at lmax 1023 and one field).
-template <int NF>
-constexpr int kChunk = 64 / NF;   // two coefficients per lane
+// 64 degrees at any field count: with 32 for two fields the next chunk's loads outlast the sums of
+// the current one (synthesis of two fields from cold caches, lmax 255 20.5 -> 16.4 us, 511 38.9 -> 32.8).
+constexpr int kChunk = 64;   // two degrees per lane
 
 template <int NF, int UP>
 struct SynWarp {   // one warp's shared memory
-  double2 c[2][kChunk<NF> * NF];   // coefficients of two chunks
+  double2 c[2][kChunk * NF];       // coefficients of two chunks
   double2 s[UP][32];               // start states
-  double al[2][kChunk<NF>];
+  double al[2][kChunk];
 };
 
 // Pairs 32 UP pb .. of order im.
 template <typename C, int NF, int UP>
 __device__ __forceinline__ void syn_item(const Args& a, int im, int pb, SynWarp<NF, UP>& sw) {
-  constexpr int CH = kChunk<NF>;
+  constexpr int CH = kChunk;
   auto& sAl = sw.al;
   auto& sC = sw.c;
   auto& sS = sw.s;
@@ -119,19 +120,20 @@ __device__ __forceinline__ void syn_item(const Args& a, int im, int pb, SynWarp<
 #pragma unroll
     for (int k = 0; k < NF; ++k) accE[u][k] = accO[u][k] = make_double2(0.0, 0.0);
 
-  // chunk stager: lane stages degrees sd0, sd0 + 32 / NF of field sk
-  const int sk = lane / (32 / NF), sd0 = lane % (32 / NF);
+  // chunk stager: lane stages degrees lane and lane + 32 of every field
   double al[2], cf[2];
-  C cv[2];
+  C cv[2][NF];
   auto fetch = [&](int d0) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const int d = d0 + sd0 + q * (32 / NF);
+      const int d = d0 + lane + 32 * q;
       al[q] = cf[q] = 0.0;
-      cv[q].x = cv[q].y = 0;
+#pragma unroll
+      for (int k = 0; k < NF; ++k) cv[q][k].x = cv[q][k].y = 0;
       if (d < ndeg) {
-        if (sk == 0) al[q] = P.alpha[poff + d];
-        cv[q] = cin[(long long)sk * a.ld_k + d];
+        al[q] = P.alpha[poff + d];
+#pragma unroll
+        for (int k = 0; k < NF; ++k) cv[q][k] = cin[(long long)k * a.ld_k + d];
         cf[q] = factor_at(a, poff, m + d, m);
       }
     }
@@ -139,10 +141,13 @@ __device__ __forceinline__ void syn_item(const Args& a, int im, int pb, SynWarp<
   auto put = [&](int b) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const int sd = sd0 + q * (32 / NF);
-      if (sk == 0) sAl[b][sd] = al[q];
-      const double2 c = wide(cv[q]);
-      sC[b][sd * NF + sk] = make_double2(c.x * cf[q], c.y * cf[q]);
+      const int sd = lane + 32 * q;
+      sAl[b][sd] = al[q];
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        const double2 c = wide(cv[q][k]);
+        sC[b][sd * NF + k] = make_double2(c.x * cf[q], c.y * cf[q]);
+      }
     }
   };
   int buf = 0;
