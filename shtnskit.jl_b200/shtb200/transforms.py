@@ -133,8 +133,15 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
+# the current stream's handle without building a torch.cuda.Stream object for it;
+# the function is private to torch and may be absent
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(device_index: int) -> int:
-    return torch._C._cuda_getCurrentRawStream(device_index)
+    if _raw_stream is not None:
+        return _raw_stream(device_index)
+    return torch.cuda.current_stream(device_index).cuda_stream
 
 
 def _workspace(plan, op, nf, dtype_code, prec, device_index) -> tuple[torch.Tensor, int]:

@@ -68,3 +68,13 @@ def test_transform_arguments_rejected_before_device():
         sht.synthesis(cfg, np.zeros((16, 16, 2), np.complex64), precision="mixed")
     with pytest.raises(sht.ArgumentError, match="precision"):
         sht.analysis_batch(cfg, np.zeros((16, 32, 2), np.float32), precision="tf32")
+
+
+def test_stream_handle_without_torch_private_function(monkeypatch):
+    class Stream:
+        cuda_stream = 77
+
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(T, "_raw_stream", None, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index: Stream() if index == 3 else None)
+    assert T._stream(3) == 77
