@@ -546,8 +546,10 @@ static size_t fft_smem(const FFTDesc& fd, size_t celem, int h) {
 // A small batch is split finer, down to 2 pairs (4 for runs of 16 bytes in FP32 rows of 1500 points or
 // more, and for the B tile images, which are written 4 pairs at a time): as long as all CTAs of an SM's
 // share still run at once (FP32 nlon 1080, one field 66 / 50 -> 24 / 19; FP64 nlon 720, 3 fields 23 / 25 ->
-// 17 / 19; FP64 nlon 1024, 3 fields, whose CTAs of 2 pairs would not, 29 / 33 against 19 / 27), and where
-// one CTA fills an SM, when it shortens the waves by a quarter (FP32 nlon 2700, 3 fields 88 / 84 -> 80 / 78).
+// 17 / 19; FP64 nlon 1024, 3 fields, whose CTAs of 2 pairs would not, 29 / 33 against 19 / 27), and, where
+// one CTA fills an SM or FP32 rows have 700 points, when it shortens the waves by a quarter (FP32 nlon
+// 2700, 3 fields 88 / 84 -> 80 / 78; nlon 1080, 13 fields 80 / 72 -> 66 / 62; with shorter rows the halved runs cost
+// more, FP32 nlon 512, 24 fields 29 / 35 -> 31 / 39, FP64 nlon 720, 8 fields 33 / 37 -> 39 / 37).
 // CTAs that then have an SM each get 512 threads (FP32 nlon 2000, one field 27 / 29 -> 25 / 25).
 // Rows with a prime radix above 13 take up to 4 pairs and a thread for 23 or 24 points, so that its
 // pass keeps its wide sums (nlon 1018, 3 fields, FP64 146 us; 512 threads 189).
@@ -577,7 +579,8 @@ static FFTShape fft_shape(const shtb_plan* p, size_t celem, int nfw, int wtile) 
     const long long slots = p->nsm * std::min<long long>(512 / t, 227 * 1024 / (fft_smem(fd, celem, hh) + 1024));
     return (ctas(hh) + slots - 1) / slots;
   };
-  while (h > hmin && (t < 512 ? waves(h / 2) == 1 : 4 * waves(h / 2) <= 6 * waves(h))) h >>= 1;
+  const bool quarter = t == 512 || (f32 && fd.n >= 700);
+  while (h > hmin && (waves(h / 2) == 1 || (quarter && 2 * waves(h / 2) <= 3 * waves(h)))) h >>= 1;
   if (t == 256 && ctas(h) <= p->nsm) t = 512;
   return FFTShape{h, t};
 }

@@ -16,9 +16,9 @@ from _util import rand_alm, rel_l2
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("precision,nlon", [("mixed", n) for n in (1350, 1440, 1500, 2046, 2048, 2880, 3000)]
+@pytest.mark.parametrize("precision,nlon", [("mixed", n) for n in (690, 720, 1350, 1440, 1500, 2046, 2048, 2880, 3000)]
                          + [("fp64", n) for n in (640, 720, 1350, 1440, 2700, 3000)])
-@pytest.mark.parametrize("nlat,nf", [(33, 1), (33, 3), (301, 24)])
+@pytest.mark.parametrize("nlat,nf", [(33, 1), (33, 3), (301, 13), (301, 24)])
 def test_launch_shapes(precision, nlon, nlat, nf):
     lmax, tol = 20, 1e-12 if precision == "fp64" else 1e-6
     cfg, ocfg = sht.create_gauss_config(lmax, nlat, nlon=nlon), so.create_gauss_config(lmax, nlat, nlon=nlon)
