@@ -116,7 +116,7 @@ def to_device(x, dtype, device_index: int) -> torch.Tensor:
         x = torch.from_numpy(np.asfortranarray(x))
     if not isinstance(x, torch.Tensor):
         raise ArgumentError(f"unsupported operand type {type(x)}")
-    if x.device != dev or x.dtype != dtype or not _kernel_ready(x):
+    if x.dtype != dtype or x.is_conj() or x.is_neg() or x.device != dev or not is_julia_dense(x):
         out = julia_empty(x.shape, dtype, dev)
         out.copy_(x.to(dev) if x.dtype == dtype else x.to(dev).to(dtype))
         x = out
@@ -133,15 +133,17 @@ def _ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 
 
-# the current stream's handle without building a torch.cuda.Stream object for it;
-# the function is private to torch and may be absent
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-
-
-def _stream(device_index: int) -> int:
-    if _raw_stream is not None:
-        return _raw_stream(device_index)
+def _public_stream(device_index: int) -> int:
     return torch.cuda.current_stream(device_index).cuda_stream
+
+
+def _stream_reader(torch_c):
+    """The function that reads the current stream's handle: torch's private one, which builds no
+    torch.cuda.Stream object, or the public call where torch lacks it."""
+    return getattr(torch_c, "_cuda_getCurrentRawStream", _public_stream)
+
+
+_stream = _stream_reader(torch._C)
 
 
 def _workspace(plan, op, nf, dtype_code, prec, device_index) -> tuple[torch.Tensor, int]:

@@ -74,7 +74,6 @@ def test_stream_handle_without_torch_private_function(monkeypatch):
     class Stream:
         cuda_stream = 77
 
-    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
-    monkeypatch.setattr(T, "_raw_stream", None, raising=False)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda index: Stream() if index == 3 else None)
-    assert T._stream(3) == 77
+    assert T._stream_reader(object())(3) == 77
+    assert T._stream is T._stream_reader(torch._C)
