@@ -2,13 +2,13 @@
 // with its own plan (lmax, Gauss grid, nlon) and 1..8 fields, run as persistent stage
 // launches: B packing and order-GEMM synthesis for members with three or more fields, the
 // FP64-pipe synthesis (simt.cu) for members with one or two, FFT synthesis, FFT analysis, and
-// the order-GEMM or FP64-pipe analysis.
+// the order-GEMM or FP64-pipe analysis of the same members.
 //
 // Every stage owns a list of work items over all members — GEMM tiles (member, order,
 // first latitude pair or degree, parity, with the tile's live-chunk mask: chunks whose P
-// image is all zero are skipped), FP64-pipe items (member, order, block of 32 latitude
-// pairs or segment of degrees, one per warp) and FFT tiles (member, first latitude pair, field) — sorted by
-// decreasing cost, and a device work counter (zeroed by a memset at the start of every
+// image is all zero are skipped), FP64-pipe items (member, order, block of latitude
+// pairs or up to two spans of degrees, one item per warp) and FFT tiles (member, first latitude
+// pair, field) — sorted by decreasing cost, and a device work counter (zeroed by a memset at the start of every
 // roundtrip). A stage launches min(items, SMs x CTAs per SM) persistent CTAs; each claims
 // the next item with an atomicAdd on the counter whenever it has room for one, so the
 // longest tiles start first and the short ones fill in behind whichever CTA frees up first,
@@ -312,18 +312,18 @@ extern "C" int shtb_group_create(shtb_group** out, const shtb_plan* const* plans
         cssyn.push_back(p->lmax - im + 1);
       }
   }
-  long long nsegs = 0;
+  long long nspans = 0;
   for (int t = 0; t < n; ++t)
-    if (g->simt[t]) nsegs += plans[t]->hoff[plans[t]->nm] / simt_ana_segment(nfields[t]);
-  const int per_item = simt_ana_segments_per_warp(nsegs, g->nsm);
+    if (g->simt[t]) nspans += plans[t]->hoff[plans[t]->nm] / simt_ana_span(nfields[t]);
+  const int per_item = simt_ana_spans_per_warp(nspans, g->nsm);
   for (int t = 0; t < n; ++t) {
     if (!g->simt[t]) continue;
     const shtb_plan* p = plans[t];
-    const int sg = simt_ana_segment(nfields[t]);
+    const int sg = simt_ana_span(nfields[t]);
     for (int im = 0; im <= std::min(p->mmax, p->lmax); ++im) {
-      const int segs = (p->lmax - im) / sg + 1;
-      for (int s = 0; s < segs; s += per_item) {
-        const int k = std::min(per_item, segs - s);
+      const int spans = (p->lmax - im) / sg + 1;
+      for (int s = 0; s < spans; s += per_item) {
+        const int k = std::min(per_item, spans - s);
         sana.push_back(make_int4(t, im, s, k));
         csana.push_back(k * p->npair * sg * (2 + 2 * nfields[t]));
       }

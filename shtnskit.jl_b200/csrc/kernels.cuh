@@ -143,8 +143,8 @@ int launch_simt_ana(const shtb_plan* p, const void* W, void* alm, int nf, int lt
 size_t simt_args_bytes();
 // syn: coefficients -> Fourier buffer, else Fourier buffer -> coefficients.
 void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int nf, void* host_args);
-int simt_ana_segment(int nf);   // degrees per segment of the grouped analysis
-int simt_ana_segments_per_warp(long long segs, int nsm);   // segments per item, for that many segments in all
+int simt_ana_span(int nf);   // degrees that a warp of the analysis sums at a time
+int simt_ana_spans_per_warp(long long spans, int nsm);   // spans per item, for that many spans in all
 int simt_syn_pair_blocks(const shtb_plan* p);
 int launch_simt_group(const void* targs, const int4* items, int nitems, int grid, int* queue, unsigned long long* t0,
                       cudaStream_t st);

@@ -251,11 +251,11 @@ constexpr int kAlLd = kSeg<NF> + 1;   // stride of a segment's alpha in shared m
 constexpr int kPU = 2;
 constexpr int kRing = 3;
 
-// A warp of the persistent kernel takes up to kMaxSegs consecutive spans: the ring runs on
+// A warp of the persistent kernel takes up to kMaxSpans consecutive spans: the ring runs on
 // into the next span's first pairs while the sums of the current one cross the lanes (32
 // uneven transforms 652 -> 631 us). A single transform's warps take one: four made the CTAs
 // uneven (lmax 1023, one field 154 -> 183 us, with 32 lanes a segment).
-constexpr int kMaxSegs = 2;
+constexpr int kMaxSpans = 2;
 
 template <typename C, int NF>
 struct Ring {   // one warp's slots
@@ -265,7 +265,7 @@ struct Ring {   // one warp's slots
     double x[kPU][32];
     int l0[kPU][32];
   } s[kRing];
-  int p0[kMaxSegs];   // first pair of each span of the warp
+  int p0[kMaxSpans];   // first pair of each span of the warp
 };
 
 // Alpha and factors of a warp's spans: they load while its first operands do.
@@ -555,17 +555,17 @@ struct GroupAnaWarp {
     Ring<float2, 2> r2;
   };
   union {
-    SegTables<1, kMaxSegs> t1;
-    SegTables<2, kMaxSegs> t2;
+    SegTables<1, kMaxSpans> t1;
+    SegTables<2, kMaxSpans> t2;
   };
 };
 
 template <int NF>
 __device__ __forceinline__ void ana_warp_item(const Args& a, int im, int seg, int nseg, Ring<float2, NF>& R,
-                                              SegTables<NF, kMaxSegs>& T) {
+                                              SegTables<NF, kMaxSpans>& T) {
   const int lane = threadIdx.x & 31, m = im * a.P.mres, lseg = m + kSpan<NF> * seg;
   __syncwarp();   // the previous item's tables are read
-  ana_segments<float2, NF, kMaxSegs>(a, im, lseg, nseg, T, R);
+  ana_segments<float2, NF, kMaxSpans>(a, im, lseg, nseg, T, R);
   if (seg == 0)
     for (int k = 0; k < a.nf; ++k) {
       float2* col = (float2*)a.out + (long long)k * a.ld_k + (long long)m * a.ld_m;
@@ -708,11 +708,11 @@ void simt_fill_args(const shtb_plan* p, int syn, const void* in, void* out, int 
   std::memcpy(host_args, &a, sizeof(a));
 }
 
-int simt_ana_segment(int nf) { return nf == 1 ? sx::kSpan<1> : sx::kSpan<2>; }
+int simt_ana_span(int nf) { return nf == 1 ? sx::kSpan<1> : sx::kSpan<2>; }
 
 // Several once every warp slot (two per scheduler) has work for three rounds.
-int simt_ana_segments_per_warp(long long segs, int nsm) {
-  return (int)std::max(1ll, std::min<long long>(sx::kMaxSegs, segs / (3ll * nsm * 8)));
+int simt_ana_spans_per_warp(long long spans, int nsm) {
+  return (int)std::max(1ll, std::min<long long>(sx::kMaxSpans, spans / (3ll * nsm * 8)));
 }
 
 int simt_syn_pair_blocks(const shtb_plan* p) {   // per-warp items of the group kernel
